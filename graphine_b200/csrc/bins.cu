@@ -16,8 +16,8 @@
 // log2 n, log2 m), so graphs of the same shape - the batches of a run, replicas - tune once.
 //
 // GRE_TUNE=0 in the environment turns the measurement off (the default schedule is used), and
-// graphs with fewer than 2^22 arcs always use the default: their supersteps are too short to
-// time apart from launch overhead.  GRE_ROW_SCHEDULE=lane_arcs,cta_min,hub_chunk,seg_window
+// graphs with fewer than 2^22 arcs always use a fixed one of short chains: their supersteps are
+// too short to time apart from launch overhead.  GRE_ROW_SCHEDULE=lane_arcs,cta_min,hub_chunk,seg_window
 // imposes a schedule (tests use it to reach every kernel on small graphs).
 #include <cub/cub.cuh>
 
@@ -34,6 +34,7 @@ namespace gre {
 namespace {
 
 constexpr uint64_t kTuneMinArcs = 1ull << 22;
+constexpr uint64_t kShortChainMinArcs = 1ull << 16;
 constexpr int kHistBuckets = 40;
 
 __global__ void k_bin_of(uint64_t n, const uint64_t* __restrict__ off, uint8_t* __restrict__ bin, uint32_t lane_arcs,
@@ -407,6 +408,15 @@ int ensure_bins(gre_graph g, bool in) {
   const uint32_t* col = in ? g->rcol : g->col;
   const bool sorted = in && !g->symmetric() ? true : g->csr_sorted;  // the CSC is built sorted
   RowSchedule sched;  // default
+  // Below the tuner's range a superstep is bound by the longest chain of dependent loads, not by
+  // bandwidth: a CTA from 512 arcs (PageRank-20 on directed RMAT-16, all bins in one launch: 4 /
+  // 4096 314 us, 4 / 1024 231, 4 / 512 215, 8 / 512 196, 2 / 512 198, 4 / 256 214).  Larger graphs
+  // lose by it (RMAT-24: 31.9 -> 34.6 ms); the smallest have no row that long and gain nothing
+  // (RMAT-11, 45K arcs: 148 us either way; RMAT-12, 97K: 189 -> 148 us).
+  if (g->m >= kShortChainMinArcs && g->m < kTuneMinArcs) {
+    sched.lane_arcs = 8;
+    sched.cta_min = 512;
+  }
   if (const char* e = getenv("GRE_ROW_SCHEDULE")) {  // "lane_arcs,cta_min,hub_chunk,seg_window": a fixed schedule
     unsigned long long a = 0, c = 0, h = 0, w = 0;
     if (sscanf(e, "%llu,%llu,%llu,%llu", &a, &c, &h, &w) != 4 || a < 1 || a > 64 || c < 16 * a || h < c || h == 0) {

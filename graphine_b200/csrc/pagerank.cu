@@ -154,7 +154,7 @@ struct PprFinish {
   }
 };
 
-// rows of bins 0..4 (degree <= 64): one warp per row
+// rows of up to kPprChunk arcs, whatever their bin: one warp per row
 __global__ void __launch_bounds__(256) k_ppr_rows(const uint32_t* __restrict__ rows, uint64_t count, PprRow R, PprFinish F) {
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -495,22 +495,11 @@ int gre_pagerank(gre_graph g, int variant, double d, uint32_t iters, double* pr,
     FinishPR fin{dpr, refresh ? b : nullptr, g->outdeg, tele, d};
     return rows::reduce_rows(g->bins_in, g->roff, GatherContrib{g->rcol, a}, fin, partial, g->stream);
   };
-  // supersteps repeat with period 2 (the contribution buffers swap), 1 for the reference
-  // variant: that period is recorded once as a CUDA graph and replayed
-  const uint32_t period = refresh ? 2 : 1;
-  uint32_t done = 0;
-  if (iters >= 2 * period) {
-    Recorded rec;
-    GRE_CHECK(rec.record(g->stream, [&]() {
-      int e = superstep(c0, c1);
-      if (!e && refresh) e = superstep(c1, c0);
-      return e;
-    }));
-    for (; done + period <= iters; done += period) GRE_CHECK(rec.replay(g->stream));
-  }
-  for (double *cur = c0, *nxt = c1; done < iters; ++done) {
-    GRE_CHECK(superstep(cur, nxt));
-    if (refresh) std::swap(cur, nxt);
+  // one or two launches a superstep: launched as they come (recording and instantiating a CUDA
+  // graph each call cost more than the launches it saved)
+  for (uint32_t done = 0; done < iters; ++done) {
+    GRE_CHECK(superstep(c0, c1));
+    if (refresh) std::swap(c0, c1);
   }
   GRE_CHECK(perm_out_end(g, dpr, dout, 1, 8));
   GRE_CHECK(finish_output(g, pr, dout, n));
@@ -570,7 +559,7 @@ int gre_ppr(gre_graph g, const uint32_t* seeds, uint32_t k, double d, uint32_t i
     GRE_CHECK(ws_array(g, WS_E, kCols, &dseeds));
     const DegreeBins& B = g->bins_in;
     uint64_t short_rows = 0;
-    for (int b = 0; b < 6; ++b) short_rows += B.count[b];  // rows longer than kPprChunk are skipped
+    for (int b = 0; b < DegreeBins::NB; ++b) short_rows += B.count[b];  // rows longer than kPprChunk are skipped
     std::unique_ptr<Recorded> rec;
     uint32_t rec_kk = 0;
     for (uint32_t j0 = 0; j0 < k; j0 += kCols) {

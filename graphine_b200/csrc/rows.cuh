@@ -1,15 +1,14 @@
 // Degree-binned row reductions over a CSR or CSC: the pull form of the superstep's
 // scatter+combine for sums (PageRank, weighted PageRank, its adjoint).
 //
-// Rows are grouped once per graph by degree (DegreeBins, schedule chosen by the autotuner in
-// bins.cu): bins 0..5 give a row 1, 2, 4, 8, 16 or 32 lanes (by default degree 1-4, 5-8, 9-16,
-// 17-32, 33-64, 65-4096: about four arcs per lane per pass); bin 6 gives a row one CTA (by
-// default 4097-65536); bin 7 splits a row into chunks of hub_chunk arcs (65536), one CTA each,
-// whose partial sums are added in chunk order by a second kernel.  Lane j of a group adds arcs
-// j, j+L, j+2L, ... (four independent loads per pass) and the group reduces with xor shuffles,
-// so every row's sum has a fixed association order for a given schedule: results are
-// deterministic run to run.  Column indices of one group are contiguous (coalesced); the
-// gathered value is the only random access.
+// Rows are grouped once per graph by degree (DegreeBins, schedule chosen in bins.cu): bins 0..5
+// give a row 1, 2, 4, 8, 16 or 32 lanes (4 arcs per lane and a warp up to 4096 arcs: degree 1-4,
+// 5-8, 9-16, 17-32, 33-64, 65-4096); bin 6 gives a row one CTA (4097-65536 there); bin 7 splits a
+// row into chunks of hub_chunk arcs (65536), one CTA each, whose partial sums are added in chunk
+// order by a second kernel.  Lane j of a group adds arcs j, j+L, j+2L, ... (four independent loads
+// per pass) and the group reduces with xor shuffles, so every row's sum has a fixed association
+// order for a given schedule: results are deterministic run to run.  Column indices of one group
+// are contiguous (coalesced); the gathered value is the only random access.
 //
 //   Gather: __device__ double operator()(uint32_t row, uint64_t arc) const   value of one arc
 //   Finish: __device__ void operator()(uint32_t row, double sum)
@@ -47,17 +46,16 @@ __device__ __forceinline__ double strided_sum(Gather& gat, uint32_t v, uint64_t 
   return acc;
 }
 
+// The rows of one bin, L lanes each: block `part` of `nparts` takes every nparts-th group of
+// 256 / L rows.
 template <int L, class Gather, class Finish>
-__global__ void __launch_bounds__(256) k_rows_lanes(const uint32_t* __restrict__ rows, uint64_t count,
-                                                     const uint64_t* __restrict__ off, Gather gat, Finish fin) {
-  constexpr int G = 32 / L;  // groups per warp
-  const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t lig = lane % L;
-  const uint64_t warp = tid >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t base = warp * G; base < count; base += nwarps * G) {
-    const uint64_t i = base + lane / L;
+__device__ __forceinline__ void rows_lanes(const uint32_t* __restrict__ rows, uint32_t count, uint32_t part, uint32_t nparts,
+                                           const uint64_t* __restrict__ off, Gather& gat, Finish& fin) {
+  const uint32_t lig = threadIdx.x % L;
+  const uint64_t step = (uint64_t)nparts * (kCta / L);
+  // the warp stays together for the shuffles: its first row decides
+  for (uint64_t base = (uint64_t)part * (kCta / L) + (threadIdx.x & ~31u) / L; base < count; base += step) {
+    const uint64_t i = base + (threadIdx.x & 31u) / L;
     const bool valid = i < count;
     double acc = 0.0;
     uint32_t v = 0;
@@ -69,7 +67,6 @@ __global__ void __launch_bounds__(256) k_rows_lanes(const uint32_t* __restrict__
     for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (valid && lig == 0) fin(v, acc);
   }
-  finish_end(fin, 0);
 }
 
 __device__ __forceinline__ double block_sum(double x, double* smem) {
@@ -86,60 +83,80 @@ __device__ __forceinline__ double block_sum(double x, double* smem) {
   return t;  // valid in thread 0
 }
 
+// What one block of k_rows_all works on.  Segment 0: chunks of the multi-CTA rows (window chunks
+// when the schedule splits rows by source window); 1: a CTA per row; 2..7: 32, 16, 8, 4, 2, 1
+// lanes per row.  Segment s owns blocks [block[s], block[s + 1]).
+struct RowPlan {
+  uint32_t block[9];
+  uint32_t count[8];        // chunks or rows
+  uint32_t row0[8];         // first entry of the segment in `rows`
+  const uint32_t* rows;     // DegreeBins::rows
+  const uint64_t* chunk_row;
+  const uint64_t* chunk_begin;
+  uint64_t chunk;           // arcs per chunk
+  const uint32_t* seg_row;  // window chunks: null when not split
+  const uint64_t* seg_begin;
+  const uint64_t* seg_end;
+  const uint64_t* seg_slot;
+};
+
+// Every bin of a superstep in one launch.  Latency and tails bound a superstep of a small graph
+// when its bins run one after the other (RMAT-16, seven bins: 40 us a superstep, each bin 7-20 us
+// alone); side by side they take as long as the slowest.  The blocks of the longest rows come
+// first, so that the short ones fill the gaps at the end (PageRank-20: RMAT-16
+// directed 820 -> 314 us, RMAT-24 36.1 -> 31.9 ms; weighted solves at RMAT-20 147 -> 60 ms).  The sums are
+// those of a launch per bin: a row's association order depends on its bin alone.
 template <class Gather, class Finish>
-__global__ void __launch_bounds__(kCta) k_rows_cta(const uint32_t* __restrict__ rows, uint64_t count,
-                                                    const uint64_t* __restrict__ off, Gather gat, Finish fin) {
+__global__ void __launch_bounds__(kCta) k_rows_all(const __grid_constant__ RowPlan P, const uint64_t* __restrict__ off, Gather gat,
+                                                   Finish fin, double* __restrict__ partial) {
   __shared__ double smem[kCta / 32];
-  for (uint64_t i = blockIdx.x; i < count; i += gridDim.x) {
-    const uint32_t v = rows[i];
-    double acc = strided_sum<kCta>(gat, v, off[v], off[v + 1], threadIdx.x);
-    acc = block_sum(acc, smem);
-    if (threadIdx.x == 0) fin(v, acc);
+  uint32_t s = 0;
+  while (blockIdx.x >= P.block[s + 1]) ++s;
+  const uint32_t part = blockIdx.x - P.block[s], nparts = P.block[s + 1] - P.block[s], count = P.count[s];
+  const uint32_t* rows = P.rows + P.row0[s];
+  if (s == 0) {
+    for (uint64_t c = part; c < count; c += nparts) {
+      uint32_t v;
+      uint64_t a0, a1, slot = c;
+      if (P.seg_row) {
+        v = P.seg_row[c];
+        a0 = P.seg_begin[c];
+        a1 = P.seg_end[c];
+        slot = P.seg_slot[c];
+      } else {
+        v = rows[P.chunk_row[c]];
+        a0 = P.chunk_begin[c];
+        const uint64_t end = off[v + 1];
+        a1 = (a0 + P.chunk < end) ? a0 + P.chunk : end;
+      }
+      const double acc = block_sum(strided_sum<kCta>(gat, v, a0, a1, threadIdx.x), smem);
+      if (threadIdx.x == 0) partial[slot] = acc;
+    }
+    return;
+  }
+  if (s == 1) {
+    for (uint64_t i = part; i < count; i += nparts) {
+      const uint32_t v = rows[i];
+      const double acc = block_sum(strided_sum<kCta>(gat, v, off[v], off[v + 1], threadIdx.x), smem);
+      if (threadIdx.x == 0) fin(v, acc);
+    }
+  } else if (s == 2) {
+    rows_lanes<32>(rows, count, part, nparts, off, gat, fin);
+  } else if (s == 3) {
+    rows_lanes<16>(rows, count, part, nparts, off, gat, fin);
+  } else if (s == 4) {
+    rows_lanes<8>(rows, count, part, nparts, off, gat, fin);
+  } else if (s == 5) {
+    rows_lanes<4>(rows, count, part, nparts, off, gat, fin);
+  } else if (s == 6) {
+    rows_lanes<2>(rows, count, part, nparts, off, gat, fin);
+  } else {
+    rows_lanes<1>(rows, count, part, nparts, off, gat, fin);
   }
   finish_end(fin, 0);
 }
 
-template <class Gather>
-__global__ void __launch_bounds__(kCta) k_rows_chunks(const uint32_t* __restrict__ rows, const uint64_t* __restrict__ chunk_row,
-                                                       const uint64_t* __restrict__ chunk_begin, uint64_t nchunks, uint64_t chunk,
-                                                       const uint64_t* __restrict__ off, Gather gat, double* __restrict__ partial) {
-  __shared__ double smem[kCta / 32];
-  for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
-    const uint32_t v = rows[chunk_row[c]];
-    const uint64_t a0 = chunk_begin[c];
-    const uint64_t end = off[v + 1];
-    const uint64_t a1 = (a0 + chunk < end) ? a0 + chunk : end;
-    double acc = strided_sum<kCta>(gat, v, a0, a1, threadIdx.x);
-    acc = block_sum(acc, smem);
-    if (threadIdx.x == 0) partial[c] = acc;
-  }
-}
-
-// Window-split rows (DegreeBins::seg_*): CTA per chunk in processing order, partial sums by slot.
-template <class Gather>
-__global__ void __launch_bounds__(kCta) k_rows_seg(const uint32_t* __restrict__ row, const uint64_t* __restrict__ begin,
-                                                   const uint64_t* __restrict__ end, const uint64_t* __restrict__ slot,
-                                                   uint64_t nchunks, Gather gat, double* __restrict__ partial) {
-  __shared__ double smem[kCta / 32];
-  for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
-    const uint32_t v = row[c];
-    double acc = strided_sum<kCta>(gat, v, begin[c], end[c], threadIdx.x);
-    acc = block_sum(acc, smem);
-    if (threadIdx.x == 0) partial[slot[c]] = acc;
-  }
-}
-
-template <class Finish>
-__global__ void k_rows_seg_finish(const uint32_t* __restrict__ rows, uint64_t count, const uint64_t* __restrict__ first,
-                                  const double* __restrict__ partial, Finish fin) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (uint64_t c = first[i]; c < first[i + 1]; ++c) s += partial[c];
-    fin(rows[i], s);
-  }
-  finish_end(fin, 0);
-}
-
+// The partial sums of the chunked rows, added in chunk order.
 template <class Finish>
 __global__ void k_rows_chunk_finish(const uint32_t* __restrict__ rows, uint64_t count, const uint64_t* __restrict__ first,
                                     const double* __restrict__ partial, Finish fin) {
@@ -151,30 +168,39 @@ __global__ void k_rows_chunk_finish(const uint32_t* __restrict__ rows, uint64_t 
   finish_end(fin, 0);
 }
 
+// Blocks of one segment: enough for one pass, at most kSegBlocks an SM (the blocks of a long
+// segment stride over it).
+constexpr int kSegBlocks = 16;
+
 // Launch the reductions of every non-empty row.  `partial` holds bins.n_partials doubles.
 template <class Gather, class Finish>
 int reduce_rows(const DegreeBins& B, const uint64_t* off, Gather gat, Finish fin, double* partial, cudaStream_t s) {
-  const uint32_t* r = B.rows;
-  auto grid = [](uint64_t threads) { return grid_for(threads, 256, 8); };
-  if (B.count[0]) k_rows_lanes<1><<<grid(B.count[0]), 256, 0, s>>>(r + B.start[0], B.count[0], off, gat, fin);
-  if (B.count[1]) k_rows_lanes<2><<<grid(B.count[1] * 2), 256, 0, s>>>(r + B.start[1], B.count[1], off, gat, fin);
-  if (B.count[2]) k_rows_lanes<4><<<grid(B.count[2] * 4), 256, 0, s>>>(r + B.start[2], B.count[2], off, gat, fin);
-  if (B.count[3]) k_rows_lanes<8><<<grid(B.count[3] * 8), 256, 0, s>>>(r + B.start[3], B.count[3], off, gat, fin);
-  if (B.count[4]) k_rows_lanes<16><<<grid(B.count[4] * 16), 256, 0, s>>>(r + B.start[4], B.count[4], off, gat, fin);
-  if (B.count[5]) k_rows_lanes<32><<<grid(B.count[5] * 32), 256, 0, s>>>(r + B.start[5], B.count[5], off, gat, fin);
-  if (B.seg_nchunks) {  // rows above cta_min, window by window
-    k_rows_seg<<<grid_for(B.seg_nchunks * kCta, kCta, 8), kCta, 0, s>>>(B.seg_row, B.seg_begin, B.seg_end, B.seg_slot,
-                                                                         B.seg_nchunks, gat, partial);
-    k_rows_seg_finish<<<grid_for(B.seg_nrows, 128, 4), 128, 0, s>>>(B.seg_rows, B.seg_nrows, B.seg_first, partial, fin);
-    GRE_LAUNCH_CHECK();
-    return GRE_SUCCESS;
+  RowPlan P{};
+  const bool windows = B.seg_nchunks != 0;  // the rows above cta_min, window by window
+  P.rows = B.rows;
+  P.chunk_row = B.hub_chunk_row;
+  P.chunk_begin = B.hub_chunk_begin;
+  P.chunk = B.sched.hub_chunk;
+  if (windows) {
+    P.seg_row = B.seg_row;
+    P.seg_begin = B.seg_begin;
+    P.seg_end = B.seg_end;
+    P.seg_slot = B.seg_slot;
   }
-  if (B.count[6]) k_rows_cta<<<grid_for(B.count[6] * kCta, kCta, 8), kCta, 0, s>>>(r + B.start[6], B.count[6], off, gat, fin);
-  if (B.count[7]) {
-    k_rows_chunks<<<grid_for(B.n_hub_chunks * kCta, kCta, 8), kCta, 0, s>>>(r + B.start[7], B.hub_chunk_row, B.hub_chunk_begin,
-                                                                            B.n_hub_chunks, B.sched.hub_chunk, off, gat, partial);
-    k_rows_chunk_finish<<<grid_for(B.count[7], 128, 4), 128, 0, s>>>(r + B.start[7], B.count[7], B.hub_chunk_first, partial, fin);
+  for (int k = 0; k < 8; ++k) {
+    const int b = 7 - k;  // segment k holds bin 7 - k
+    const uint64_t items = k == 0 ? (windows ? B.seg_nchunks : B.n_hub_chunks) : (k == 1 && windows) ? 0 : B.count[b];
+    P.count[k] = (uint32_t)items;
+    P.row0[k] = (uint32_t)B.start[b];
+    const uint64_t threads = items * (k < 2 ? kCta : 1ull << b);
+    P.block[k + 1] = P.block[k] + (items ? grid_for(threads, kCta, kSegBlocks) : 0);
   }
+  if (!P.block[8]) return GRE_SUCCESS;
+  k_rows_all<<<P.block[8], kCta, 0, s>>>(P, off, gat, fin, partial);
+  if (windows)
+    k_rows_chunk_finish<<<grid_for(B.seg_nrows, 128, 4), 128, 0, s>>>(B.seg_rows, B.seg_nrows, B.seg_first, partial, fin);
+  else if (B.count[7])
+    k_rows_chunk_finish<<<grid_for(B.count[7], 128, 4), 128, 0, s>>>(B.rows + B.start[7], B.count[7], B.hub_chunk_first, partial, fin);
   GRE_LAUNCH_CHECK();
   return GRE_SUCCESS;
 }

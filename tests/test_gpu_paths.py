@@ -1,0 +1,58 @@
+"""The kernels' own edges: tiles, remainders and the sizes at which a dispatch changes path."""
+import numpy as np
+import pytest
+
+from graphine_b200 import gre as G
+
+pytestmark = pytest.mark.gpu
+
+
+def rows_graph(degrees, n, seed):
+    """A directed graph in which in-row i has degrees[i] arcs (columns drawn with a seed)."""
+    rng = np.random.default_rng(seed)
+    dst = np.repeat(np.arange(len(degrees)), degrees)
+    src = rng.integers(0, n, len(dst))
+    order = np.argsort(src, kind="stable")
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(src, minlength=n))
+    return off, dst[order].astype(np.uint32)
+
+
+def pagerank_ref(n, off, col, iters, base, d=0.85):
+    """Power iteration in float64 for the columns of `base` (n x k)."""
+    src = np.repeat(np.arange(n), np.diff(off.astype(np.int64)))
+    deg = np.diff(off.astype(np.int64))
+    x = base.copy()
+    for _ in range(iters):
+        c = x / np.maximum(deg, 1)[:, None]
+        s = np.stack([np.bincount(col, weights=c[src, j], minlength=n) for j in range(x.shape[1])], axis=1)
+        x = base + d * s
+    return x
+
+
+# degrees at and around every limit of the schedule lanes 2, CTA from 33, chunks of 64
+EDGES = [0, 1, 2, 3, 4, 5, 8, 9, 16, 17, 31, 32, 33, 34, 63, 64, 65, 127, 128, 129, 300, 1024, 1025]
+
+
+@pytest.mark.parametrize("schedule", ["", "2,32,64,0", "2,32,64,100", "8,512,65536,0"])
+@pytest.mark.parametrize("rows", [1, 23, 300, 5000])
+def test_rows_of_every_bin_in_one_launch(monkeypatch, schedule, rows):
+    """A superstep's bins share a launch: rows at the limits of each bin, from one row to several
+    blocks of each; the plain and the batched personalised form (rows of 513-1024 arcs may sit in
+    the CTA bin).  Positive sums of at most 1025 terms in float64: 1025 eps relative at most."""
+    if schedule:
+        monkeypatch.setenv("GRE_ROW_SCHEDULE", schedule)
+    degrees = [EDGES[(7 * i + 3) % len(EDGES)] for i in range(rows)]
+    n = max(rows, 400)
+    off, col = rows_graph(degrees, n, rows)
+    g = G.Graph.from_csr(n, off, col)
+    ref = pagerank_ref(n, off, col, 6, np.full((n, 1), 0.15))[:, 0]
+    pr, _ = G.pagerank(g, G.PR_ITER, 0.85, 6)
+    assert np.max(np.abs(pr - ref) / ref) <= 6 * 1025 * 2.3e-16
+    if rows <= 300:
+        seeds = np.array([0, 5, 399, 17], np.uint32)
+        base = np.zeros((n, 4))
+        base[seeds, np.arange(4)] = 0.15
+        ref = pagerank_ref(n, off, col, 4, base).T
+        out, _ = G.ppr(g, seeds, 0.85, 4)
+        assert np.max(np.abs(out.reshape(4, n) - ref)) <= 4 * 1025 * 2.3e-16
