@@ -5,8 +5,12 @@
 // vertex with the minimum vid of its (weakly) connected component.  Union-find reaches the
 // same labels directly: every arc {u, v} unites the two trees, and a root is only ever linked
 // under a smaller root (atomicCAS on the larger root's parent), so the root of each tree is
-// the minimum vid it contains.  A final pass writes find(v) for every v.  (Jayanti & Tarjan
-// style concurrent union-find as used by ECL-CC, Jaiganesh & Burtscher 2018.)
+// the smallest stored id it contains.  A final pass writes find(v) for every v.  (Jayanti & Tarjan
+// style concurrent union-find as used by ECL-CC, Jaiganesh & Burtscher 2018.)  On a relabelled
+// graph the stored ids put the hubs first, so that nearly every link is a vertex under the
+// first hub, each on its own word; the smallest caller id of each tree is then found by one pass
+// over the vertices.  (Linked by caller ids instead, the root of the giant tree changes whenever a
+// smaller id joins, and links and path writes meet on few words: RMAT-22 the first pass 1084 us.)
 //
 // Arcs are visited through the degree bins of the CSR (rows.cuh): groups of 1..32 lanes per
 // row, a CTA per long row, CTA chunks for hubs, so the column reads stay coalesced.  A directed
@@ -30,31 +34,92 @@ namespace gre {
 struct HookArcs {
   const uint32_t* __restrict__ col;
   uint32_t* parent;
-  const uint32_t* __restrict__ vid;  // internal -> caller id, null when not relabelled
-  bool half;                          // symmetric: use only arcs with col < row
   // Afforest's second pass: rows flagged in `skip` are left out and the first `sampled` arcs of
   // the others were already united (null: every arc)
   const uint32_t* __restrict__ skip = nullptr;
   const uint64_t* __restrict__ off = nullptr;
   uint32_t sampled = 0;
+  __device__ __forceinline__ bool skips(uint32_t u) const { return skip && ((__ldg(skip + (u >> 5)) >> (u & 31u)) & 1u); }
   __device__ __forceinline__ double operator()(uint32_t u, uint64_t a) const {
-    if (skip) {
-      if ((__ldg(skip + (u >> 5)) >> (u & 31u)) & 1u) return 0.0;
-      if (a < __ldg(off + u) + sampled) return 0.0;
-    }
-    const uint32_t v = __ldg(col + a);
-    if (!half || v < u) uf_union(parent, vid, u, v);
+    if (skip && a < __ldg(off + u) + sampled) return 0.0;
+    uf_union(parent, nullptr, u, __ldg(col + a));
     return 0.0;
   }
 };
 
 // Afforest (Sutton, Ben-Nun and Bar 2018), first pass: every vertex is united with its first k
-// neighbours (relabelled rows list the hubs first, which joins most of a giant component).
+// neighbours (relabelled rows list the hubs first, which joins most of a giant component).  The
+// first arc, where it leads to a smaller id, needs no union: it is the vertex's parent from the
+// start (ids fall along it, so no cycle), written with plain stores; most of the second arcs then
+// find both ends in one tree.  RMAT-22: 252 us with unions for both
+// arcs, 64 us (29 + 35) so; the whole call 1310 -> 240 us with it and the links by stored id.
+__global__ void k_uf_first(uint64_t n, const uint64_t* __restrict__ off, const uint32_t* __restrict__ col,
+                           uint32_t* __restrict__ parent) {
+  for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t a0 = off[u];
+    const uint32_t v = a0 < off[u + 1] ? __ldg(col + a0) : (uint32_t)u;
+    parent[u] = v < u ? v : (uint32_t)u;
+  }
+}
 __global__ void k_uf_sample(uint64_t n, const uint64_t* __restrict__ off, const uint32_t* __restrict__ col, uint32_t k,
-                            uint32_t* parent, const uint32_t* __restrict__ vid) {
+                            uint32_t* parent) {
   for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t a0 = off[u], a1 = off[u + 1];
-    for (uint64_t a = a0; a < a1 && a < a0 + k; ++a) uf_union(parent, vid, (uint32_t)u, __ldg(col + a));
+    for (uint64_t a = a0; a < a1 && a < a0 + k; ++a) {
+      const uint32_t v = __ldg(col + a);
+      if (a > a0 || v > u) uf_union(parent, nullptr, (uint32_t)u, v);
+    }
+  }
+}
+
+// The most frequent root among those of kSample evenly spaced vertices (the smallest of equals), found
+// by one CTA: the host is not asked.
+constexpr uint32_t kSample = 256;
+__global__ void __launch_bounds__(kSample) k_uf_mode(uint64_t n, uint64_t stride, uint32_t* parent, uint32_t* __restrict__ best) {
+  __shared__ uint32_t root[kSample];
+  __shared__ unsigned long long top;
+  const uint32_t ns = (uint32_t)((n + stride - 1) / stride < kSample ? (n + stride - 1) / stride : kSample);
+  const uint32_t t = threadIdx.x;
+  if (t == 0) top = 0;
+  if (t < ns) root[t] = uf_find(parent, (uint32_t)(t * stride));
+  __syncthreads();
+  if (t < ns) {
+    uint32_t same = 0;
+    for (uint32_t i = 0; i < ns; ++i) same += root[i] == root[t];
+    atomicMax(&top, (unsigned long long)same << 32 | (0xffffffffu - root[t]));
+  }
+  __syncthreads();
+  if (t == 0) *best = 0xffffffffu - (uint32_t)top;
+}
+
+// parent[v] = root of v; skip bit of every vertex in the tree of *best; counts[0] += arcs sampled,
+// counts[1] += arcs the second pass still visits (byte model)
+__global__ void k_uf_compress_skip(uint64_t n, uint32_t* parent, const uint64_t* __restrict__ off, const uint32_t* __restrict__ best,
+                                   uint32_t k, uint32_t* __restrict__ skip, unsigned long long* __restrict__ counts) {
+  const uint32_t b = *best;
+  unsigned long long sampled = 0, rest = 0;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < n; base += stride) {
+    const uint64_t v = base + (threadIdx.x & 31u);
+    bool in = false;
+    if (v < n) {
+      const uint32_t r = uf_find(parent, (uint32_t)v);
+      parent[v] = r;
+      in = r == b;
+      const uint64_t d = off[v + 1] - off[v];
+      sampled += d < k ? d : k;
+      if (!in && d > k) rest += d - k;
+    }
+    const uint32_t word = __ballot_sync(0xffffffffu, in);
+    if ((threadIdx.x & 31u) == 0) skip[base >> 5] = word;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    sampled += __shfl_xor_sync(0xffffffffu, sampled, o);
+    rest += __shfl_xor_sync(0xffffffffu, rest, o);
+  }
+  if ((threadIdx.x & 31u) == 0) {
+    if (sampled) atomicAdd(counts, sampled);
+    if (rest) atomicAdd(counts + 1, rest);
   }
 }
 
@@ -103,18 +168,35 @@ __global__ void k_uf_init(uint64_t n, uint32_t* __restrict__ parent) {
     parent[v] = (uint32_t)v;
 }
 
-// label (in caller ids) of every internal vertex: the key of its root
-__global__ void k_uf_flatten(uint64_t n, uint32_t* parent, const uint32_t* __restrict__ vid, uint32_t* __restrict__ label) {
+__global__ void k_uf_flatten(uint64_t n, uint32_t* parent, uint32_t* __restrict__ label) {
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
-    label[v] = uf_key(vid, uf_find(parent, (uint32_t)v));
+    label[v] = uf_find(parent, (uint32_t)v);
 }
 
-__global__ void k_count_roots(uint64_t n, const uint32_t* __restrict__ label, unsigned long long* __restrict__ c) {
-  unsigned long long s = 0;
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
-    s += label[v] == v;
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31u) == 0 && s) atomicAdd(c, s);
+// Relabelled graphs: least[r] = smallest caller id in the tree of root r (parent[v] = root of v on
+// the way; least starts as a copy of perm).  A warp's lanes in the tree of its first lane send one atomic, and an id that is not
+// smaller than the one already there sends none: the giant tree's word would serialise them.
+__global__ void k_uf_least(uint64_t n, uint32_t* parent, const uint32_t* __restrict__ perm, uint32_t* least) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < n; base += stride) {
+    const uint64_t v = base + (threadIdx.x & 31u);
+    uint32_t r = 0xffffffffu, id = 0xffffffffu;
+    if (v < n) {
+      r = uf_find(parent, (uint32_t)v);
+      parent[v] = r;
+      id = __ldg(perm + v);
+    }
+    const uint32_t first = __shfl_sync(0xffffffffu, r, 0);  // lane 0 holds a vertex
+    const uint32_t low = __reduce_min_sync(0xffffffffu, r == first ? id : 0xffffffffu);
+    const bool lead = (threadIdx.x & 31u) == 0;
+    if (lead) id = low;
+    if (v < n && (lead || r != first) && id < __ldcg(least + r)) atomicMin(least + r, id);
+  }
+}
+__global__ void k_uf_label(uint64_t n, const uint32_t* __restrict__ iperm, const uint32_t* __restrict__ parent,
+                           const uint32_t* __restrict__ least, uint32_t* __restrict__ label) {
+  for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x)
+    label[u] = __ldg(least + __ldg(parent + __ldg(iperm + u)));
 }
 
 uint32_t uf_most_frequent(std::vector<uint32_t>& hs, uint32_t ns) {
@@ -142,52 +224,54 @@ int gre_cc(gre_graph g, uint32_t* label, gre_stats* st) {
   stats_reset(st);
   const uint64_t n = g->n;
   GRE_CHECK(ensure_bins(g, false));
-  uint32_t *dfinal, *dl, *parent;
+  uint32_t *dlabel, *parent, *least = nullptr;
   double* partial;
   void* p;
-  GRE_CHECK(prepare_output(g, label, n, WS_OUTBUF, &dfinal));
-  GRE_CHECK(perm_out_begin(g, dfinal, 1, 4, (void**)&dl));
+  GRE_CHECK(prepare_output(g, label, n, WS_OUTBUF, &dlabel));
   GRE_CHECK(g->ws.get(WS_A, sizeof(uint32_t) * n, &p));
   parent = (uint32_t*)p;
   GRE_CHECK(g->ws.get(WS_B, sizeof(double) * (g->bins_out.n_partials + 1), &p));
   partial = (double*)p;
-  constexpr uint32_t kSampled = 2, kSample = 1024;
-  uint32_t *skip = nullptr, *sample = nullptr;
+  if (g->perm) {
+    GRE_CHECK(g->ws.get(WS_PERM_OUT, sizeof(uint32_t) * n, &p));
+    least = (uint32_t*)p;
+  }
+  constexpr uint32_t kSampled = 2;
+  uint32_t *skip = nullptr, *best = nullptr;
   unsigned long long* counts = nullptr;
   if (g->symmetric()) {
-    GRE_CHECK(g->ws.get(WS_C, sizeof(uint32_t) * (((n + 31) >> 5) + kSample), &p));
+    GRE_CHECK(g->ws.get(WS_C, sizeof(uint32_t) * ((n + 31) >> 5), &p));
     skip = (uint32_t*)p;
-    sample = skip + ((n + 31) >> 5);
-    GRE_CHECK(g->ws.get(WS_COUNTERS, 2 * sizeof(unsigned long long), &p));
+    GRE_CHECK(g->ws.get(WS_COUNTERS, 3 * sizeof(unsigned long long), &p));
     counts = (unsigned long long*)p;
+    best = (uint32_t*)(counts + 2);
   }
   RunTimer timer(g);
-  k_uf_init<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent);
   if (g->symmetric()) {
     // Afforest: unite the first arcs of every row, find the largest component from a sample,
     // then unite the remaining arcs of the vertices outside it only.  Undirected edges appear
     // in both rows, so an edge between the largest component and another vertex is seen from
     // the other side.
-    k_uf_sample<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->off, g->col, kSampled, parent, g->perm);
-    const uint64_t stride = n > kSample ? n / kSample : 1;
-    k_uf_compress<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent, stride, sample, kSample);
-    std::vector<uint32_t> hs(kSample, 0);
-    const uint32_t ns = (uint32_t)std::min<uint64_t>(kSample, (n + stride - 1) / stride);
-    GRE_CUDA(cudaMemcpyAsync(hs.data(), sample, sizeof(uint32_t) * ns, cudaMemcpyDeviceToHost, g->stream));
-    GRE_CUDA(cudaStreamSynchronize(g->stream));
-    const uint32_t best = uf_most_frequent(hs, ns);
     GRE_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), g->stream));
-    k_uf_skipbits<<<grid_for((n + 31) >> 5, 256), 256, 0, g->stream>>>(n, parent, g->off, best, kSampled, skip, counts);
-    HookArcs rest{g->col, parent, g->perm, false, skip, g->off, kSampled};
+    k_uf_first<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->off, g->col, parent);
+    k_uf_sample<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->off, g->col, kSampled, parent);
+    k_uf_mode<<<1, kSample, 0, g->stream>>>(n, n > kSample ? n / kSample : 1, parent, best);
+    k_uf_compress_skip<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent, g->off, best, kSampled, skip, counts);
+    HookArcs rest{g->col, parent, skip, g->off, kSampled};
     GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, rest, NoFinish{}, partial, g->stream));
   } else {
-    GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, HookArcs{g->col, parent, g->perm, false}, NoFinish{}, partial,
-                                g->stream));
+    k_uf_init<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent);
+    GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, HookArcs{g->col, parent}, NoFinish{}, partial, g->stream));
   }
-  k_uf_flatten<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent, g->perm, dl);
+  if (g->perm) {
+    GRE_CUDA(cudaMemcpyAsync(least, g->perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, g->stream));
+    k_uf_least<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent, g->perm, least);
+    k_uf_label<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->iperm, parent, least, dlabel);
+  } else {
+    k_uf_flatten<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent, dlabel);
+  }
   GRE_LAUNCH_CHECK();
-  GRE_CHECK(perm_out_end(g, dl, dfinal, 1, 4));
-  GRE_CHECK(finish_output(g, label, dfinal, n));
+  GRE_CHECK(finish_output(g, label, dlabel, n));
   GRE_CHECK(timer.stop(st));
   if (st) {
     uint64_t visited = g->m;

@@ -11,6 +11,7 @@
 // are contiguous (coalesced); the gathered value is the only random access.
 //
 //   Gather: __device__ double operator()(uint32_t row, uint64_t arc) const   value of one arc
+//           __device__ bool skips(uint32_t row) const   (optional) rows left out: no arcs, sum 0
 //   Finish: __device__ void operator()(uint32_t row, double sum)
 //           __device__ void end()   (optional) after the block's last row, by all its threads
 #pragma once
@@ -27,6 +28,10 @@ template <class F>
 __device__ __forceinline__ auto finish_end(F& f, int) -> decltype(f.end()) { f.end(); }
 template <class F>
 __device__ __forceinline__ void finish_end(F&, long) {}
+template <class G>
+__device__ __forceinline__ auto row_skipped(const G& g, uint32_t v, int) -> decltype(g.skips(v)) { return g.skips(v); }
+template <class G>
+__device__ __forceinline__ bool row_skipped(const G&, uint32_t, long) { return false; }
 
 // Sum of gat(v, a) over a = a0 + lig, a0 + lig + L, ... < a1.  Four arcs per pass so that each
 // lane has four independent (column, gathered value) load chains in flight: the loop is bound
@@ -61,7 +66,7 @@ __device__ __forceinline__ void rows_lanes(const uint32_t* __restrict__ rows, ui
     uint32_t v = 0;
     if (valid) {
       v = rows[i];
-      acc = strided_sum<L>(gat, v, off[v], off[v + 1], lig);
+      if (!row_skipped(gat, v, 0)) acc = strided_sum<L>(gat, v, off[v], off[v + 1], lig);
     }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -129,6 +134,7 @@ __global__ void __launch_bounds__(kCta) k_rows_all(const __grid_constant__ RowPl
         const uint64_t end = off[v + 1];
         a1 = (a0 + P.chunk < end) ? a0 + P.chunk : end;
       }
+      if (row_skipped(gat, v, 0)) a1 = a0;
       const double acc = block_sum(strided_sum<kCta>(gat, v, a0, a1, threadIdx.x), smem);
       if (threadIdx.x == 0) partial[slot] = acc;
     }
@@ -137,7 +143,8 @@ __global__ void __launch_bounds__(kCta) k_rows_all(const __grid_constant__ RowPl
   if (s == 1) {
     for (uint64_t i = part; i < count; i += nparts) {
       const uint32_t v = rows[i];
-      const double acc = block_sum(strided_sum<kCta>(gat, v, off[v], off[v + 1], threadIdx.x), smem);
+      const uint64_t a0 = off[v], a1 = row_skipped(gat, v, 0) ? a0 : off[v + 1];
+      const double acc = block_sum(strided_sum<kCta>(gat, v, a0, a1, threadIdx.x), smem);
       if (threadIdx.x == 0) fin(v, acc);
     }
   } else if (s == 2) {

@@ -24,6 +24,8 @@ __device__ __forceinline__ uint32_t uf_find(uint32_t* parent, uint32_t x) {
 // key(x): the caller's id of vertex x (null map: x itself) - roots are linked by it
 __device__ __forceinline__ uint32_t uf_key(const uint32_t* __restrict__ key, uint32_t x) { return key ? __ldg(key + x) : x; }
 
+// The loads may come from L1 and be old: an old parent is still an ancestor.  A failed link goes on
+// from the value the atomic returned, never from a second look at what may be the same old line.
 __device__ __forceinline__ void uf_union(uint32_t* parent, const uint32_t* __restrict__ key, uint32_t a, uint32_t b) {
   while (true) {
     a = uf_find(parent, a);
@@ -32,9 +34,9 @@ __device__ __forceinline__ void uf_union(uint32_t* parent, const uint32_t* __res
     const bool a_hi = uf_key(key, a) > uf_key(key, b);
     const uint32_t hi = a_hi ? a : b;
     const uint32_t lo = a_hi ? b : a;
-    if (atomicCAS(parent + hi, hi, lo) == hi) return;
-    // hi gained a parent meanwhile: retry from the new roots
-    a = hi;
+    const uint32_t old = atomicCAS(parent + hi, hi, lo);
+    if (old == hi) return;
+    a = old;  // hi gained a parent meanwhile
     b = lo;
   }
 }

@@ -56,3 +56,32 @@ def test_rows_of_every_bin_in_one_launch(monkeypatch, schedule, rows):
         ref = pagerank_ref(n, off, col, 4, base).T
         out, _ = G.ppr(g, seeds, 0.85, 4)
         assert np.max(np.abs(out.reshape(4, n) - ref)) <= 4 * 1025 * 2.3e-16
+
+
+@pytest.mark.parametrize("reorder", [False, True])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 257, 4000])
+def test_components_whatever_the_first_arc(n, reorder):
+    """Rows in any order, first arcs to larger ids, a hub with the largest id, isolated vertices, many
+    components: labels equal the smallest caller id of each component."""
+    rng = np.random.default_rng(n)
+    part = rng.integers(0, max(1, n // 40) + 1, n)
+    u = rng.integers(0, n, 2 * n)
+    v = rng.integers(0, n, 2 * n)
+    keep = part[u] == part[v]
+    star = np.flatnonzero(part == part[n - 1])[::2]
+    u, v = np.concatenate([u[keep], np.full(len(star), n - 1)]), np.concatenate([v[keep], star])
+    src, dst = np.concatenate([u, v]), np.concatenate([v, u])
+    order = np.lexsort((rng.random(len(src)), src))
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(src, minlength=n))
+    g = G.Graph.from_csr(n, off, dst[order].astype(np.uint32), symmetric=True)
+    if reorder:
+        g.reorder()
+    want = np.arange(n)
+    while True:
+        low = want.copy()
+        np.minimum.at(low, src, want[dst])
+        if (low == want).all():
+            break
+        want = low
+    np.testing.assert_array_equal(G.cc(g)[0], want.astype(np.uint32))
