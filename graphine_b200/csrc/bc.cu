@@ -180,7 +180,7 @@ static int bc_single(gre_graph g, const std::vector<uint32_t>& hs, double* dbc, 
   uint64_t arcs = 0, bytes = 0;
   for (size_t i = 0; i < hs.size(); ++i) {
     const uint32_t s = hs[i];
-    GRE_CHECK(bfs_levels(g, roots + i, 1, level, nullptr, false));
+    GRE_CHECK(bfs_levels(g, roots + i, 1, level, nullptr));
     // vertices grouped by level
     uint32_t nl = 0;
     {

@@ -4,15 +4,18 @@
 // vertex over its arcs, claims unvisited neighbours first-writer-wins under a lock and makes
 // them the next frontier; levels are the superstep of discovery.  Here:
 //
-//  * gre_bfs / gre_bfs_multiroot: direction-optimising BFS (Beamer, Asanovic, Patterson 2012).
-//    Top-down steps expand a frontier queue edge-balanced: one thread per frontier arc, the
-//    owning vertex found by binary search in the exclusive scan of frontier degrees; a visited
-//    bitmap (n/8 bytes, L2-resident) filters claims, atomicOr claims a vertex.  Bottom-up steps
-//    give each unvisited vertex one thread that scans its in-arcs for a parent in the frontier
-//    bitmap and stops at the first; a warp covers 32 consecutive vertices, so the next-frontier
-//    word is one __ballot_sync and needs no atomics.  Switch rule: to bottom-up when the
+//  * gre_bfs / gre_bfs_multiroot: direction-optimising BFS (Beamer, Asanovic, Patterson 2012), the
+//    level loop inside one cooperative kernel (bfs_persist.cu).  Switch rule: to bottom-up when the
 //    frontier's arcs exceed (unvisited arcs)/15, back to top-down when the frontier holds fewer
 //    than n/18 vertices.
+//  * the step kernels of the searches whose level loop stays on the host: the partitioned one (an
+//    exchange a level, partition.cu) and gre_bfs_noalloc (noalloc.cu).  Top-down steps expand a
+//    frontier queue edge-balanced: one thread per frontier arc, the owning vertex found by binary
+//    search in the exclusive scan of frontier degrees; a visited bitmap (n/8 bytes, L2-resident)
+//    filters claims, atomicOr claims a vertex.  Bottom-up steps give each unvisited vertex one
+//    thread that scans its in-arcs for a parent in the frontier bitmap and stops at the first; a
+//    warp covers 32 consecutive vertices, so the next-frontier word is one __ballot_sync and needs
+//    no atomics.
 //  * gre_msbfs: 64 sources per uint64 word (multi-source BFS, Then et al. 2014): seen/frontier
 //    words per vertex; a level is one pull over in-arcs OR-ing neighbour frontier words, so the
 //    topology is read once per level for all 64 sources.
@@ -25,6 +28,7 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "bfs_persist.cuh"
 #include "gre_internal.cuh"
 #include "msbfs.cuh"
 
@@ -207,96 +211,6 @@ __global__ void k_bits_to_queue(uint64_t n, const uint32_t* __restrict__ bits, u
   }
 }
 
-// One direction-optimising BFS from `roots`, levels written into `level` (n int32).
-int bfs_levels(gre_graph g, const uint32_t* droots, uint32_t nroots, int32_t* level, gre_stats* st, bool record) {
-  const uint64_t n = g->n, m = g->m;
-  const uint64_t nwords = (n + 31) >> 5;
-  uint32_t *vis, *qa, *qb, *bits_a, *bits_b;
-  uint64_t *deg, *prefix;
-  BfsCounters* c;
-  GRE_CHECK(ws_array(g, WS_A, nwords, &vis));
-  GRE_CHECK(ws_array(g, WS_B, n, &qa));
-  GRE_CHECK(ws_array(g, WS_C, n, &qb));
-  GRE_CHECK(ws_array(g, WS_D, nwords, &bits_a));
-  GRE_CHECK(ws_array(g, WS_E, nwords, &bits_b));
-  GRE_CHECK(ws_array(g, WS_F, n + 1, &deg));
-  GRE_CHECK(ws_array(g, WS_G, n + 1, &prefix));
-  GRE_CHECK(ws_array(g, WS_COUNTERS, 4, &c));
-  void* cubtmp = nullptr;
-  size_t cubbytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, cubbytes, deg, prefix, n + 1, g->stream);
-  GRE_CHECK(g->ws.get(WS_CUB, cubbytes, &cubtmp));
-
-  GRE_CUDA(cudaMemsetAsync(level, 0xff, sizeof(int32_t) * n, g->stream));
-  GRE_CUDA(cudaMemsetAsync(vis, 0, sizeof(uint32_t) * nwords, g->stream));
-  GRE_CUDA(cudaMemsetAsync(c, 0, sizeof(BfsCounters), g->stream));
-  k_bfs_seed<<<1, 32, 0, g->stream>>>(droots, nroots, level, vis, qa, g->off, c);
-  BfsCounters h;
-  GRE_CUDA(cudaMemcpyAsync(&h, c, sizeof h, cudaMemcpyDeviceToHost, g->stream));
-  GRE_CUDA(cudaStreamSynchronize(g->stream));
-  uint64_t nf = h.next_count, mf = h.next_arcs;
-  int64_t mu = (int64_t)m - (int64_t)mf;
-  bool bottom_up = false;
-  uint32_t* queue = qa;
-  uint32_t* nqueue = qb;
-  uint32_t* front = bits_a;
-  uint32_t* nbits = bits_b;
-  int32_t d = 0;
-  uint64_t scanned_total = 0, bytes = 0, visited = nf;
-  const int sms = num_sms();
-  while (nf > 0) {
-    // direction choice
-    if (!bottom_up && (double)mf > (double)mu / 15.0 && nf > 64) {
-      GRE_CUDA(cudaMemsetAsync(front, 0, sizeof(uint32_t) * nwords, g->stream));
-      k_queue_to_bits<<<grid_for(nf, 256), 256, 0, g->stream>>>(queue, nf, front);
-      bottom_up = true;
-    } else if (bottom_up && nf < n / 18) {
-      GRE_CUDA(cudaMemsetAsync(c, 0, sizeof(BfsCounters), g->stream));
-      k_bits_to_queue<<<grid_for(nwords, 256), 256, 0, g->stream>>>(n, front, queue, &c->next_count);
-      bottom_up = false;
-    }
-    GRE_CUDA(cudaMemsetAsync(c, 0, sizeof(BfsCounters), g->stream));
-    if (!bottom_up) {
-      k_frontier_degrees<<<grid_for(nf, 256), 256, 0, g->stream>>>(queue, nf, g->off, deg);
-      GRE_CUDA(cub::DeviceScan::ExclusiveSum(cubtmp, cubbytes, deg, prefix, nf + 1, g->stream));
-      uint64_t total = 0;
-      GRE_CUDA(cudaMemcpyAsync(&total, prefix + nf, sizeof total, cudaMemcpyDeviceToHost, g->stream));
-      GRE_CUDA(cudaStreamSynchronize(g->stream));
-      if (total) {
-        int grid = (int)std::min<uint64_t>((total + 255) / 256, (uint64_t)sms * 16);
-        k_td_expand<<<grid, 256, 0, g->stream>>>(queue, nf, prefix, total, g->off, g->col, vis, level, d + 1, nqueue, c);
-      }
-      GRE_LAUNCH_CHECK();
-      GRE_CUDA(cudaMemcpyAsync(&h, c, sizeof h, cudaMemcpyDeviceToHost, g->stream));
-      GRE_CUDA(cudaStreamSynchronize(g->stream));
-      h.next_count = h.pad;  // slot counter of warp_append
-      scanned_total += total;
-      bytes += 16 * nf + 8 * total + 8 * h.next_count;
-      std::swap(queue, nqueue);
-    } else {
-      k_bu_step<<<grid_for(nwords * 32, 256, 8), 256, 0, g->stream>>>(n, g->roff, g->rcol, g->off, front, nbits, vis, level, d + 1, c);
-      GRE_LAUNCH_CHECK();
-      GRE_CUDA(cudaMemcpyAsync(&h, c, sizeof h, cudaMemcpyDeviceToHost, g->stream));
-      GRE_CUDA(cudaStreamSynchronize(g->stream));
-      scanned_total += h.scanned;
-      bytes += 16 * (n - visited) + (uint64_t)(4.125 * (double)h.scanned) + 4 * h.next_count + n / 8;
-      std::swap(front, nbits);
-    }
-    nf = h.next_count;
-    mf = h.next_arcs;
-    mu -= (int64_t)mf;
-    visited += nf;
-    ++d;
-    if (record) stats_record(st, nf);
-  }
-  if (st) {
-    st->supersteps += (uint32_t)(d > 0 ? d - 1 : 0);  // getSuperstepCount: the empty level is not counted
-    st->arcs_traversed += scanned_total;
-    st->algo_bytes += bytes;
-  }
-  return GRE_SUCCESS;
-}
-
 // Undirected edges with a reached endpoint: sum over reached v of outdeg(v) / 2 (symmetric).
 // sum of the degrees of reached vertices over `rows` level arrays of n entries each
 __global__ void k_reached_degree(uint64_t n, uint64_t rows, const int32_t* __restrict__ level, const uint32_t* __restrict__ deg,
@@ -384,55 +298,6 @@ __global__ void __launch_bounds__(256) k_ms_pull(uint64_t n, uint32_t k, unsigne
   }
 }
 
-// Several roots, one search (graphs batched as one block-diagonal union: every root in its own
-// component): the roots share source bit 0 of the 64-source word, so the persistent level loop
-// of persist.cu runs the whole search in one cooperative launch.  Levels and per-level counts
-// equal bfs_levels' (the same levels, found in the same order of levels).  Used on request only
-// (see gre_bfs_multiroot).
-__global__ void k_ms_seed_roots(const uint32_t* __restrict__ roots, uint32_t k, unsigned long long* __restrict__ seen,
-                                unsigned long long* __restrict__ front, int32_t* __restrict__ levels) {
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < k; j += gridDim.x * blockDim.x) {
-    const uint32_t r = roots[j];
-    seen[r] = 1ull;
-    front[r] = 1ull;
-    levels[r] = 0;
-  }
-}
-
-static int bfs_multiroot_persistent(gre_graph g, const uint32_t* droots, uint32_t nroots, int32_t* level, gre_stats* st) {
-  const uint64_t n = g->n;
-  unsigned long long *seen, *fa, *fb, *acc;
-  uint32_t *flist, *flist2;
-  unsigned char* ctl;
-  GRE_CHECK(ws_array(g, WS_A, n, &seen));
-  GRE_CHECK(ws_array(g, WS_B, n, &fa));
-  GRE_CHECK(ws_array(g, WS_C, n, &fb));
-  GRE_CHECK(ws_array(g, WS_E, n, &acc));
-  GRE_CHECK(ws_array(g, WS_F, n, &flist));
-  GRE_CHECK(ws_array(g, WS_G, n, &flist2));
-  GRE_CHECK(ws_array(g, WS_I, msbfs_ctl_bytes(), &ctl));
-  GRE_CHECK(ensure_bins(g, true));
-  GRE_CUDA(cudaMemsetAsync(level, 0xff, sizeof(int32_t) * n, g->stream));
-  GRE_CUDA(cudaMemsetAsync(seen, 0, sizeof(unsigned long long) * n, g->stream));
-  GRE_CUDA(cudaMemsetAsync(fa, 0, sizeof(unsigned long long) * n, g->stream));
-  GRE_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long) * n, g->stream));
-  k_ms_seed_roots<<<grid_for(nroots, 256), 256, 0, g->stream>>>(droots, nroots, seen, fa, level);
-  GRE_LAUNCH_CHECK();
-  uint32_t nl = 0;
-  uint64_t scanned = 0, bytes = 0;
-  std::vector<unsigned long long> found;
-  GRE_CHECK(msbfs_word_persistent(g, 1ull, seen, fa, fb, acc, flist, flist2, level, ctl,
-                                  (unsigned long long*)(ctl + msbfs_ctl_bytes()) - GRE_MAX_RECORDED_SUPERSTEPS, &nl, &scanned,
-                                  &bytes, &found));
-  for (unsigned long long f : found) stats_record(st, f);
-  if (st) {
-    st->supersteps += nl;  // the empty level is not counted, as bfs_levels
-    st->arcs_traversed += scanned;
-    st->algo_bytes += bytes;
-  }
-  return GRE_SUCCESS;
-}
-
 }  // namespace gre
 
 using namespace gre;
@@ -447,24 +312,19 @@ int gre_bfs(gre_graph g, const uint32_t* srcs, uint32_t nsrc, int32_t* levels, g
   std::vector<uint32_t> hs(nsrc);
   if (nsrc) GRE_CUDA(cudaMemcpy(hs.data(), srcs, sizeof(uint32_t) * nsrc, cudaMemcpyDefault));
   GRE_CHECK(map_ids(g, &hs, "gre_bfs"));
-  int32_t *dfinal, *dl;
-  uint32_t* droot;
-  GRE_CHECK(prepare_output(g, levels, (uint64_t)nsrc * n, WS_OUTBUF, &dfinal));
-  GRE_CHECK(perm_out_begin(g, dfinal, nsrc, 4, (void**)&dl));
-  GRE_CHECK(ws_array(g, WS_H, nsrc ? nsrc : 1, &droot));
+  int32_t* dl;
+  GRE_CHECK(prepare_output(g, levels, (uint64_t)nsrc * n, WS_OUTBUF, &dl));
   RunTimer timer(g);
-  if (nsrc) GRE_CUDA(cudaMemcpyAsync(droot, hs.data(), sizeof(uint32_t) * nsrc, cudaMemcpyHostToDevice, g->stream));
-  uint64_t edges = 0;
-  for (uint32_t i = 0; i < nsrc; ++i) {
-    GRE_CHECK(bfs_levels(g, droot + i, 1, dl + (uint64_t)i * n, st, nsrc == 1));
-    uint64_t e = 0;
-    GRE_CHECK(count_reached_edges(g, dl + (uint64_t)i * n, &e));
-    edges += e;
+  uint64_t arcs = 0;
+  if (nsrc) {
+    BfsPlan plan;
+    GRE_CHECK(plan.prepare(g, nsrc, true, st && nsrc == 1));
+    for (uint32_t i = 0; i < nsrc; ++i) GRE_CHECK(plan.search(i, nullptr, 1, hs[i], dl + (uint64_t)i * n));
+    GRE_CHECK(plan.collect(st, &arcs));
   }
-  GRE_CHECK(perm_out_end(g, dl, dfinal, nsrc, 4));
-  GRE_CHECK(finish_output(g, levels, dfinal, (uint64_t)nsrc * n));
+  GRE_CHECK(finish_output(g, levels, dl, (uint64_t)nsrc * n));
   GRE_CHECK(timer.stop(st));
-  if (st) st->traversed_edges = edges;
+  if (st) st->traversed_edges = g->symmetric() ? arcs / 2 : arcs;
   return GRE_SUCCESS;
 }
 
@@ -476,26 +336,20 @@ int gre_bfs_multiroot(gre_graph g, const uint32_t* roots, uint32_t nroots, int32
   std::vector<uint32_t> hs(nroots);
   if (nroots) GRE_CUDA(cudaMemcpy(hs.data(), roots, sizeof(uint32_t) * nroots, cudaMemcpyDefault));
   GRE_CHECK(map_ids(g, &hs, "gre_bfs_multiroot"));
-  int32_t *dfinal, *dl;
+  int32_t* dl;
   uint32_t* droot;
-  GRE_CHECK(prepare_output(g, level, n, WS_OUTBUF, &dfinal));
-  GRE_CHECK(perm_out_begin(g, dfinal, 1, 4, (void**)&dl));
+  GRE_CHECK(prepare_output(g, level, n, WS_OUTBUF, &dl));
   GRE_CHECK(ws_array(g, WS_H, nroots ? nroots : 1, &droot));
   RunTimer timer(g);
   if (nroots) GRE_CUDA(cudaMemcpyAsync(droot, hs.data(), sizeof(uint32_t) * nroots, cudaMemcpyHostToDevice, g->stream));
-  // the persistent form only on request (GRE_PERSIST=1): 32 uneven RMAT graphs (scales 12-18,
-  // 2.65M vertices, 6 levels) took 1.86 ms against 1.13 ms for the host loop, whose few levels
-  // cost less than the persistent loop's 8-byte words per vertex
-  const char* pe = getenv("GRE_PERSIST");
-  if (nroots > 1 && pe && strtoul(pe, nullptr, 10) != 0 && msbfs_persistent_available(n))
-    GRE_CHECK(bfs_multiroot_persistent(g, droot, nroots, dl, st));
-  else GRE_CHECK(bfs_levels(g, droot, nroots, dl, st, true));
-  uint64_t e = 0;
-  GRE_CHECK(count_reached_edges(g, dl, &e));
-  GRE_CHECK(perm_out_end(g, dl, dfinal, 1, 4));
-  GRE_CHECK(finish_output(g, level, dfinal, n));
+  BfsPlan plan;
+  uint64_t arcs = 0;
+  GRE_CHECK(plan.prepare(g, 1, true, st != nullptr));
+  GRE_CHECK(plan.search(0, droot, nroots, 0, dl));
+  GRE_CHECK(plan.collect(st, &arcs));
+  GRE_CHECK(finish_output(g, level, dl, n));
   GRE_CHECK(timer.stop(st));
-  if (st) st->traversed_edges = e;
+  if (st) st->traversed_edges = g->symmetric() ? arcs / 2 : arcs;
   return GRE_SUCCESS;
 }
 

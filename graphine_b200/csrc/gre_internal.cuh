@@ -132,6 +132,7 @@ struct gre_graph_s {
   uint64_t* rarc = nullptr;  // CSC slot -> CSR arc id (built on demand)
   uint32_t* outdeg = nullptr;
   uint32_t* indeg = nullptr;  // aliases outdeg when symmetric
+  uint32_t* in_bits = nullptr;  // bit per vertex: it has in-arcs (built by the first BFS)
   bool csr_sorted = false;    // every CSR row lists its columns in increasing order (the CSC always does)
   // weights
   uint32_t* w32 = nullptr;
@@ -398,8 +399,8 @@ uint64_t sssp_pull_arcs_divisor();
 int sssp_relax_tiles(cudaStream_t stream, const uint32_t* queue, uint64_t nq, const uint64_t* prefix, uint64_t total,
                      uint32_t* tstart, const uint64_t* base, const uint32_t* col, const uint32_t* w, const uint32_t* srcdist,
                      uint32_t* dist, uint32_t* changed, uint32_t* error, const uint32_t* known, const OwnHeads& own);
-// Direction-optimising BFS levels from device roots (uses slots WS_A..WS_G, WS_COUNTERS, WS_CUB).
-int bfs_levels(gre_graph g, const uint32_t* droots, uint32_t nroots, int32_t* level, gre_stats* st, bool record);
+// Direction-optimising BFS levels from device roots, by internal id (uses slots WS_A..WS_D).
+int bfs_levels(gre_graph g, const uint32_t* droots, uint32_t nroots, int32_t* level, gre_stats* st);
 
 // ---------------------------------------------------------------------------------------------
 // Relabelled graphs: caller ids <-> internal ids.  All no-ops when g->perm is null.

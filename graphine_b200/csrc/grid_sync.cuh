@@ -1,0 +1,63 @@
+// Grid barrier of the persistent kernels, with a bounded wait.
+//
+// The kernels are launched cooperatively (at most the resident block count), so every block a
+// barrier waits for is running.  A wait has a time budget (GRE_GRID_WAIT_MS, default 2000 ms; 0
+// fails every wait at once, which the tests use): one that runs out sets an error flag and
+// returns false, as does every block that sees the flag, so a launch ends within about two
+// budgets and the context stays usable.
+//
+// Arrivals count up and never reset (one atomic and one polled word a barrier).  Thread 0's fences
+// around the wait order the block's memory before and after it: plain loads after a barrier see
+// what other blocks wrote before it (loads of such data must not go through the read-only path).
+#pragma once
+#include <cstdlib>
+
+#include "gre_internal.cuh"
+
+namespace gre {
+
+struct GridBar {
+  unsigned int arrived;  // zero at launch
+  unsigned int err;
+};
+
+// Budget of a wait in ns.
+inline long long grid_wait_ns() {
+  if (const char* e = getenv("GRE_GRID_WAIT_MS")) return (long long)strtoll(e, nullptr, 10) * 1000000ll;
+  return 2000ll * 1000000ll;
+}
+
+#ifdef __CUDACC__
+__device__ __forceinline__ unsigned long long globaltimer_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// `target` is thread 0's running count of arrivals (0 at the kernel's start).
+__device__ __forceinline__ bool grid_barrier(GridBar* b, unsigned int& target, long long wait_ns) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    target += gridDim.x;
+    __threadfence();
+    atomicAdd(&b->arrived, 1u);
+    int ok = 1;
+    const unsigned long long t0 = globaltimer_ns();
+    for (unsigned int spin = 0; (int)(*(volatile unsigned int*)&b->arrived - target) < 0; ++spin) {
+      if (wait_ns == 0 || ((spin & 63u) == 63u && (long long)(globaltimer_ns() - t0) >= wait_ns)) atomicOr(&b->err, 1u);
+      if ((wait_ns == 0 || (spin & 63u) == 63u) && *(volatile unsigned int*)&b->err) {
+        ok = 0;
+        break;
+      }
+    }
+    if (*(volatile unsigned int*)&b->err) ok = 0;
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+#endif
+
+}  // namespace gre

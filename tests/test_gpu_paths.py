@@ -85,3 +85,61 @@ def test_components_whatever_the_first_arc(n, reorder):
             break
         want = low
     np.testing.assert_array_equal(G.cc(g)[0], want.astype(np.uint32))
+
+
+def bfs_ref(n, off, col, roots):
+    level = np.full(n, -1, np.int32)
+    level[roots] = 0
+    front, d = np.unique(roots), 0
+    while len(front):
+        d += 1
+        heads = np.concatenate([col[int(off[u]):int(off[u + 1])] for u in front] + [np.empty(0, np.uint32)])
+        front = np.unique(heads[level[heads] < 0])
+        level[front] = d
+    return level
+
+
+def shaped_graph(n, seed, directed):
+    """A star with a row at the limit of a queue item, a long path, dense and sparse random parts,
+    vertices without arcs, in any id order."""
+    rng = np.random.default_rng(seed)
+    ids = rng.permutation(n)
+    u, v = [], []
+    hub = min(n - 1, [127, 128, 129, 1000][seed % 4])
+    u += [0] * hub
+    v += list(range(1, hub + 1))
+    p = n // 3  # a path from the hub's last leaf
+    u += list(range(hub, min(n - 1, hub + p)))
+    v += list(range(hub + 1, min(n, hub + p + 1)))
+    k = 6 * n
+    a, b = rng.integers(0, max(1, n // 4), k), rng.integers(0, max(1, n // 2), k)
+    u, v = np.concatenate([u, a]).astype(np.int64), np.concatenate([v, b]).astype(np.int64)
+    u, v = ids[u], ids[v]
+    if not directed:
+        u, v = np.concatenate([u, v]), np.concatenate([v, u])
+    keys = np.unique(u * n + v)
+    keys = keys[keys // n != keys % n]
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(keys // n, minlength=n))
+    return off, (keys % n).astype(np.uint32), ids
+
+
+@pytest.mark.parametrize("directed,reorder", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("n", [1, 2, 33, 127, 128, 129, 1100, 5000, 70000])
+def test_bfs_shapes(n, directed, reorder):
+    """Levels of single and several roots (some twice, some without arcs) equal a plain BFS's."""
+    off, col, ids = shaped_graph(n, n, directed)
+    g = G.Graph.from_csr(n, off, col, symmetric=not directed)
+    if reorder:
+        g.reorder()
+    roots = np.array([ids[0], ids[n - 1], ids[n // 2], ids[n - 1]], np.uint32)
+    lv, _ = G.bfs(g, roots)
+    for i, r in enumerate(roots):
+        np.testing.assert_array_equal(lv[i * n:(i + 1) * n], bfs_ref(n, off, col, [r]))
+    one, st = G.bfs(g, roots[:1])
+    np.testing.assert_array_equal(one, lv[:n])
+    assert st.active == [int((one == d).sum()) for d in range(1, st.supersteps + 2)]
+    many, st = G.bfs_multiroot(g, roots)
+    np.testing.assert_array_equal(many, bfs_ref(n, off, col, roots))
+    deg = np.diff(off.astype(np.int64))
+    assert st.traversed_edges == deg[many >= 0].sum() // (1 if directed else 2)
