@@ -16,8 +16,8 @@
 //     (an earlier one would have found it), so the visited bits serve as the frontier and none is
 //     kept; what is found goes to the other buffer.  Back to top-down, the queue is the difference
 //     of the two buffers.
-// Vertices without in-arcs count as visited from the start (RMAT: about half of all): their words
-// are skipped.  Levels go straight to the caller's order (perm), so nothing is reordered after.
+// Vertices without any arc count as visited from the start (RMAT: about half of all): their words
+// are skipped.  (Those with out-arcs only do not: they are nobody's parent until a search starts there.)  Levels go straight to the caller's order (perm), so nothing is reordered after.
 //
 // Measured against the host-driven loop: RMAT-22, 16 sources one after the other, 7240 -> 2870 us;
 // 32 graphs of 2^12..2^18 vertices in one union 517 -> 203 us; 4000 vertices 310 -> 104 us.  A
@@ -54,7 +54,7 @@ struct BfsRun {
   const uint32_t* __restrict__ col;
   const uint64_t* __restrict__ roff;
   const uint32_t* __restrict__ rcol;
-  const uint32_t* __restrict__ in_bits;
+  const uint32_t* __restrict__ arc_bits;
   const uint32_t* __restrict__ perm;
   const uint32_t* __restrict__ roots;  // null: the one root is `root`
   uint32_t nroots, root;
@@ -69,12 +69,13 @@ struct BfsRun {
   long long wait_ns;
 };
 
-// Bit per vertex: it has in-arcs.  Bits past n are 0.
-__global__ void k_in_bits(uint64_t n, uint64_t nwords, const uint64_t* __restrict__ roff, uint32_t* __restrict__ bits) {
+// Bit per vertex: it has arcs, in or out.  Bits past n are 0.
+__global__ void k_arc_bits(uint64_t n, uint64_t nwords, const uint64_t* __restrict__ off, const uint64_t* __restrict__ roff,
+                           uint32_t* __restrict__ bits) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < nwords * 32; base += stride) {
     const uint64_t v = base + (threadIdx.x & 31u);
-    const uint32_t w = __ballot_sync(0xffffffffu, v < n && roff[v + 1] > roff[v]);
+    const uint32_t w = __ballot_sync(0xffffffffu, v < n && (roff[v + 1] > roff[v] || off[v + 1] > off[v]));
     if ((threadIdx.x & 31u) == 0) bits[base >> 5] = w;
   }
 }
@@ -260,7 +261,7 @@ __device__ __forceinline__ void bottom_up(const BfsRun& R, const uint32_t* cur, 
     }
     const uint32_t vw[4] = {raw.x, raw.y, raw.z, raw.w};
     uint64_t a[4];
-    uint32_t len[4], c[4];  // arcs left from a; an open vertex has in-arcs (the others count as visited)
+    uint32_t len[4], c[4];  // arcs left from a
     bool open[4], got[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -271,6 +272,7 @@ __device__ __forceinline__ void bottom_up(const BfsRun& R, const uint32_t* cur, 
       if (open[j]) {
         a[j] = R.roff[v];
         len[j] = (uint32_t)(R.roff[v + 1] - a[j]);
+        open[j] = len[j] != 0;
       }
       got[j] = false;
     }
@@ -362,7 +364,7 @@ __global__ void __launch_bounds__(kBfsThreads, 2) k_bfs_persist(const __grid_con
   unsigned int target = 0;
   const bool first = blockIdx.x == 0 && threadIdx.x == 0;
   for (uint64_t v = gtid; v < R.n; v += nthreads) R.level[v] = -1;
-  for (uint64_t w = gtid; w < R.nwords; w += nthreads) R.vis0[w] = ~R.in_bits[w];
+  for (uint64_t w = gtid; w < R.nwords; w += nthreads) R.vis0[w] = ~R.arc_bits[w];
   if (!grid_barrier(&c->bar, target, R.wait_ns)) return;
   if (blockIdx.x == 0) {  // the roots, each once
     unsigned long long nf = 0, mf = 0;
@@ -372,7 +374,7 @@ __global__ void __launch_bounds__(kBfsThreads, 2) k_bfs_persist(const __grid_con
       uint32_t r = 0, nit = 0;
       if (i < R.nroots) {
         r = R.roots ? R.roots[i] : R.root;
-        // a root without in-arcs has its bit already: its level says whether it was seen
+        // a root without arcs has its bit already: its level says whether it was seen
         int32_t* lv = R.level + (R.perm ? R.perm[r] : r);
         if (atomicExch(lv, 0) == -1) {
           atomicOr(R.vis0 + (r >> 5), 1u << (r & 31u));
@@ -445,10 +447,10 @@ static int ws_array(gre_graph g, int slot, uint64_t count, T** p) {
   return GRE_SUCCESS;
 }
 
-static int ensure_in_bits(gre_graph g, uint64_t nwords) {
-  if (g->in_bits) return GRE_SUCCESS;
-  GRE_CUDA(cudaMalloc(&g->in_bits, sizeof(uint32_t) * nwords));
-  k_in_bits<<<grid_for(nwords * 32, 256), 256, 0, g->stream>>>(g->n, nwords, g->roff, g->in_bits);
+static int ensure_arc_bits(gre_graph g, uint64_t nwords) {
+  if (g->arc_bits) return GRE_SUCCESS;
+  GRE_CUDA(cudaMalloc(&g->arc_bits, sizeof(uint32_t) * nwords));
+  k_arc_bits<<<grid_for(nwords * 32, 256), 256, 0, g->stream>>>(g->n, nwords, g->off, g->roff, g->arc_bits);
   GRE_LAUNCH_CHECK();
   return GRE_SUCCESS;
 }
@@ -456,7 +458,7 @@ static int ensure_in_bits(gre_graph g, uint64_t nwords) {
 int BfsPlan::prepare(gre_graph graph, uint32_t nsearch, bool caller_order, bool record) {
   g = graph;
   const uint64_t n = g->n, nwords = ((n + 127) >> 7) << 2;
-  GRE_CHECK(ensure_in_bits(g, nwords));
+  GRE_CHECK(ensure_arc_bits(g, nwords));
   uint32_t* vis;
   uint2 *q0, *q1;
   BfsCtl* c;
@@ -488,7 +490,7 @@ int BfsPlan::prepare(gre_graph graph, uint32_t nsearch, bool caller_order, bool 
   R.col = g->col;
   R.roff = g->roff;
   R.rcol = g->rcol;
-  R.in_bits = g->in_bits;
+  R.arc_bits = g->arc_bits;
   R.perm = caller_order ? g->perm : nullptr;
   R.vis0 = vis;
   R.vis1 = vis + nwords;

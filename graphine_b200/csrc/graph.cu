@@ -287,7 +287,7 @@ void destroy_graph(gre_graph g) {
     cudaFree(g->rcol);
   }
   cudaFree(g->rarc);
-  cudaFree(g->in_bits);
+  cudaFree(g->arc_bits);
   if (g->indeg != g->outdeg) cudaFree(g->indeg);
   cudaFree(g->outdeg);
   cudaFree(g->w32);
@@ -431,8 +431,8 @@ static void drop_derived(gre_graph g) {
   g->rarc = nullptr;
   cudaFree(g->rw64);
   g->rw64 = nullptr;
-  cudaFree(g->in_bits);
-  g->in_bits = nullptr;
+  cudaFree(g->arc_bits);
+  g->arc_bits = nullptr;
   if (g->indeg != g->outdeg) cudaFree(g->indeg);
   cudaFree(g->outdeg);
   g->indeg = g->outdeg = nullptr;

@@ -132,7 +132,7 @@ struct gre_graph_s {
   uint64_t* rarc = nullptr;  // CSC slot -> CSR arc id (built on demand)
   uint32_t* outdeg = nullptr;
   uint32_t* indeg = nullptr;  // aliases outdeg when symmetric
-  uint32_t* in_bits = nullptr;  // bit per vertex: it has in-arcs (built by the first BFS)
+  uint32_t* arc_bits = nullptr;  // bit per vertex: it has arcs (built by the first BFS)
   bool csr_sorted = false;    // every CSR row lists its columns in increasing order (the CSC always does)
   // weights
   uint32_t* w32 = nullptr;

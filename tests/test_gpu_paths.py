@@ -143,3 +143,17 @@ def test_bfs_shapes(n, directed, reorder):
     np.testing.assert_array_equal(many, bfs_ref(n, off, col, roots))
     deg = np.diff(off.astype(np.int64))
     assert st.traversed_edges == deg[many >= 0].sum() // (1 if directed else 2)
+
+
+@pytest.mark.parametrize("n", [300, 4099, 66000])
+def test_bfs_directed_sources_only(n):
+    """Half of the vertices have out-arcs only: nobody's parent, though they never become visited."""
+    rng = np.random.default_rng(n)
+    u, v = rng.integers(0, n, 16 * n), rng.integers(0, n // 2, 16 * n)
+    keys = np.unique(u * n + v)
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(keys // n, minlength=n))
+    col = (keys % n).astype(np.uint32)
+    g = G.Graph.from_csr(n, off, col)
+    for r in (0, n - 1):
+        np.testing.assert_array_equal(G.bfs(g, [r])[0], bfs_ref(n, off, col, [r]))
