@@ -28,11 +28,11 @@
 
 #include "bfs_persist.cuh"
 #include "grid_sync.cuh"
+#include "item_queue.cuh"
 
 namespace gre {
 
 constexpr int kBfsThreads = 512;
-constexpr uint32_t kPiece = 128;  // arcs per queue item: one pass of a warp
 
 struct BfsSlot {  // the frontier of one level
   unsigned long long nf, mf;      // vertices, their out-arcs
@@ -80,112 +80,23 @@ __global__ void k_arc_bits(uint64_t n, uint64_t nwords, const uint64_t* __restri
   }
 }
 
-// Queue appends of one block in one phase.  Vertices of one item are gathered per warp in shared
-// memory and moved out kStage at a time, the rest of all warps with one atomic a block at the
-// phase's end: an atomic a warp and step on the one counter bounded the large levels (RMAT-22, a
-// frontier of hubs: 73 us).  Vertices of several items go straight to the queue.
-constexpr uint32_t kStage = 96;
 struct BfsStage {
-  uint32_t item[kBfsThreads / 32][kStage];
-  uint32_t held[kBfsThreads / 32];
-  uint32_t base;
-  unsigned long long sum[3];
+  unsigned long long nf, mf, scanned;  // this level's slot
+  unsigned int nitems;
+  ItemStage<kBfsThreads> items;
+  BlockSums<3> sums;
 };
+using BfsAppend = ItemAppend<kBfsThreads, uint2>;
 
-struct BfsAppend {
-  uint32_t* buf;
-  uint32_t held = 0;
-  unsigned int* count;
-  uint2* queue;
-  __device__ __forceinline__ BfsAppend(BfsStage& st, unsigned int* c, uint2* q)
-      : buf(st.item[threadIdx.x >> 5]), count(c), queue(q) {}
-  __device__ __forceinline__ void move(uint32_t base) {
-    for (uint32_t i = lane_id(); i < held; i += 32) queue[base + i] = make_uint2(buf[i], 0);
-    held = 0;
-  }
-  // `nit` items of vertex v per lane (warp-uniform call)
-  __device__ __forceinline__ void push(uint32_t v, uint32_t nit) {
-    const uint32_t lane = lane_id();
-    const uint32_t one = __ballot_sync(0xffffffffu, nit == 1);
-    if (one) {
-      if (held + 32 > kStage) {
-        __syncwarp();
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(count, held);
-        move(__shfl_sync(0xffffffffu, base, 0));
-        __syncwarp();
-      }
-      if (nit == 1) buf[held + __popc(one & ((1u << lane) - 1u))] = v;
-      held += __popc(one);
-    }
-    uint32_t many = __ballot_sync(0xffffffffu, nit > 1);
-    if (many) {
-      uint32_t incl = nit > 1 ? nit : 0;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (uint32_t)o) incl += x;
-      }
-      uint32_t base = 0;
-      if (lane == 31) base = atomicAdd(count, incl);
-      base = __shfl_sync(0xffffffffu, base, 31) + incl - nit;
-      while (many) {  // the warp writes the items of each
-        const int src = __ffs(many) - 1;
-        many &= many - 1;
-        const uint32_t sv = __shfl_sync(0xffffffffu, v, src), sn = __shfl_sync(0xffffffffu, nit, src);
-        const uint32_t sb = __shfl_sync(0xffffffffu, base, src);
-        for (uint32_t i = lane; i < sn; i += 32) queue[sb + i] = make_uint2(sv, i);
-      }
-    }
-  }
-  // the block's last call of a phase (all threads)
-  __device__ __forceinline__ void finish(BfsStage& st) {
-    const uint32_t w = threadIdx.x >> 5;
-    if (lane_id() == 0) st.held[w] = held;
-    __syncthreads();
-    uint32_t before = 0, total = 0;
-    for (uint32_t i = 0; i < kBfsThreads / 32; ++i) {
-      const uint32_t h = st.held[i];
-      if (i < w) before += h;
-      total += h;
-    }
-    if (total) {  // uniform
-      if (threadIdx.x == 0) st.base = atomicAdd(count, total);
-      __syncthreads();
-      move(st.base + before);
-    }
-  }
-};
-
-__device__ __forceinline__ uint32_t items_of(uint64_t degree) { return (uint32_t)((degree + kPiece - 1) / kPiece); }
-
-// The block's counts of a phase, one atomic each a block (all threads call).
 __device__ __forceinline__ void add_found(BfsStage& st, BfsSlot* s, unsigned long long nf, unsigned long long mf,
                                           unsigned long long scanned) {
-  if (threadIdx.x < 3) st.sum[threadIdx.x] = 0;
-  for (int o = 16; o > 0; o >>= 1) {
-    nf += __shfl_xor_sync(0xffffffffu, nf, o);
-    mf += __shfl_xor_sync(0xffffffffu, mf, o);
-    scanned += __shfl_xor_sync(0xffffffffu, scanned, o);
-  }
-  __syncthreads();
-  if (lane_id() == 0) {
-    if (nf) atomicAdd(&st.sum[0], nf);
-    if (mf) atomicAdd(&st.sum[1], mf);
-    if (scanned) atomicAdd(&st.sum[2], scanned);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (st.sum[0]) atomicAdd(&s->nf, st.sum[0]);
-    if (st.sum[1]) atomicAdd(&s->mf, st.sum[1]);
-    if (st.sum[2]) atomicAdd(&s->scanned, st.sum[2]);
-  }
+  st.sums.add({nf, mf, scanned}, {&s->nf, &s->mf, &s->scanned});
 }
 
 __device__ __forceinline__ void top_down(const BfsRun& R, const uint2* queue, uint32_t nitems, uint32_t* vis, int32_t next_level,
                                          uint2* out, BfsSlot* s, BfsStage& st, uint32_t gwarp, uint32_t nwarps) {
   constexpr int U = 4;
-  BfsAppend append(st, &s->nitems, out);
+  BfsAppend append(st.items, &s->nitems, out);
   const uint32_t lane = lane_id();
   // few items: one a warp, so that all warps share the arcs
   const uint32_t per = min(32u, max(1u, (nitems + nwarps - 1) / nwarps));
@@ -198,25 +109,15 @@ __device__ __forceinline__ void top_down(const BfsRun& R, const uint2* queue, ui
       a0 = R.off[it.x] + (uint64_t)it.y * kPiece;
       len = (uint32_t)min((uint64_t)kPiece, R.off[it.x + 1] - a0);
     }
-    uint32_t incl = len;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += x;
-    }
-    const uint32_t excl = incl - len, total = __shfl_sync(0xffffffffu, incl, 31);
-    for (uint32_t t = 0; t < total; t += 32 * U) {
+    const ItemSpan span(a0, len);
+    for (uint32_t t = 0; t < span.total; t += 32 * U) {
       uint32_t u[U];
       bool want[U];
 #pragma unroll
       for (int k = 0; k < U; ++k) {
         const uint32_t pos = t + 32 * k + lane;
-        uint32_t own = 0;  // last item that begins at or before pos
-#pragma unroll
-        for (uint32_t step = 16; step; step >>= 1)
-          if (__shfl_sync(0xffffffffu, excl, own + step) <= pos) own += step;
-        const uint64_t arc = __shfl_sync(0xffffffffu, a0, own) + (pos - __shfl_sync(0xffffffffu, excl, own));
-        want[k] = pos < total;
+        const uint64_t arc = span.arc_of(pos, span.owner(pos));
+        want[k] = pos < span.total;
         u[k] = want[k] ? __ldg(R.col + arc) : 0u;
       }
 #pragma unroll
@@ -224,21 +125,22 @@ __device__ __forceinline__ void top_down(const BfsRun& R, const uint2* queue, ui
 #pragma unroll
       for (int k = 0; k < U; ++k)
         if (want[k]) want[k] = !((atomicOr(vis + (u[k] >> 5), 1u << (u[k] & 31u)) >> (u[k] & 31u)) & 1u);
+      uint32_t nit[U];
 #pragma unroll
       for (int k = 0; k < U; ++k) {
-        uint32_t nit = 0;
+        nit[k] = 0;
         if (want[k]) {
           R.level[R.perm ? __ldg(R.perm + u[k]) : u[k]] = next_level;
           const uint64_t d = R.off[u[k] + 1] - R.off[u[k]];
-          nit = items_of(d);
+          nit[k] = items_of(d);
           mf += d;
           ++nf;
         }
-        append.push(u[k], nit);
       }
+      append.push(u, nit);
     }
   }
-  append.finish(st);
+  append.finish();
   add_found(st, s, nf, mf, 0);
 }
 
@@ -337,22 +239,16 @@ __device__ __forceinline__ void bottom_up(const BfsRun& R, const uint32_t* cur, 
 // The vertices set in `now` and not in `before`, as items.
 __device__ __forceinline__ void bits_to_items(const BfsRun& R, const uint32_t* now, const uint32_t* before, uint2* queue,
                                               unsigned int* count, BfsStage& st, uint32_t gwarp, uint32_t nwarps) {
-  const uint32_t lane = lane_id();
-  BfsAppend append(st, count, queue);
-  for (uint64_t base = (uint64_t)gwarp * 32; base < R.nwords; base += (uint64_t)nwarps * 32) {
-    const uint64_t w = base + lane;
-    uint32_t bits = w < R.nwords ? now[w] & ~before[w] : 0u;
-    while (__any_sync(0xffffffffu, bits != 0)) {
-      uint32_t v = 0, nit = 0;
-      if (bits) {
-        v = (uint32_t)(w << 5) + __ffs(bits) - 1;
-        bits &= bits - 1;
-        nit = items_of(R.off[v + 1] - R.off[v]);
-      }
+  BfsAppend append(st.items, count, queue);
+  const uint64_t chunks = bit_chunks(R.nwords);
+  for (uint64_t ch = gwarp; ch < chunks; ch += nwarps) {
+    const uint64_t num = chunk_word(ch, chunks);
+    for_bits<1>(num, num < R.nwords ? now[num] & ~before[num] : 0u, [&](const bool (&valid)[1], const uint32_t (&v)[1]) {
+      const uint32_t nit[1] = {valid[0] ? items_of(R.off[v[0] + 1] - R.off[v[0]]) : 0u};
       append.push(v, nit);
-    }
+    });
   }
-  append.finish(st);
+  append.finish();
 }
 
 __global__ void __launch_bounds__(kBfsThreads, 2) k_bfs_persist(const __grid_constant__ BfsRun R) {
@@ -368,28 +264,27 @@ __global__ void __launch_bounds__(kBfsThreads, 2) k_bfs_persist(const __grid_con
   if (!grid_barrier(&c->bar, target, R.wait_ns)) return;
   if (blockIdx.x == 0) {  // the roots, each once
     unsigned long long nf = 0, mf = 0;
-    BfsAppend append(st, &c->slot[0].nitems, R.q0);
+    BfsAppend append(st.items, &c->slot[0].nitems, R.q0);
     for (uint32_t base = 0; base < R.nroots; base += kBfsThreads) {
       const uint32_t i = base + threadIdx.x;
-      uint32_t r = 0, nit = 0;
+      uint32_t rv[1] = {0}, nit[1] = {0};
       if (i < R.nroots) {
-        r = R.roots ? R.roots[i] : R.root;
+        const uint32_t r = rv[0] = R.roots ? R.roots[i] : R.root;
         // a root without arcs has its bit already: its level says whether it was seen
         int32_t* lv = R.level + (R.perm ? R.perm[r] : r);
         if (atomicExch(lv, 0) == -1) {
           atomicOr(R.vis0 + (r >> 5), 1u << (r & 31u));
           const uint64_t d = R.off[r + 1] - R.off[r];
-          nit = items_of(d);
+          nit[0] = items_of(d);
           mf += d;
           ++nf;
         }
       }
-      append.push(r, nit);
+      append.push(rv, nit);
     }
-    append.finish(st);
+    append.finish();
     add_found(st, &c->slot[0], nf, mf, 0);
   }
-  if (!grid_barrier(&c->bar, target, R.wait_ns)) return;
   uint32_t* cur = R.vis0;
   uint32_t* other = R.vis1;
   long long mu = (long long)R.m;
@@ -399,9 +294,16 @@ __global__ void __launch_bounds__(kBfsThreads, 2) k_bfs_persist(const __grid_con
   for (;; ++d) {
     BfsSlot* s = &c->slot[d % 3];
     BfsSlot* sn = &c->slot[(d + 1) % 3];
-    const unsigned long long nf = __ldcg(&s->nf), mf = __ldcg(&s->mf);
+    if (!grid_barrier(&c->bar, target, R.wait_ns, [&] {
+          st.nf = __ldcg(&s->nf);
+          st.mf = __ldcg(&s->mf);
+          st.nitems = __ldcg(&s->nitems);
+          st.scanned = __ldcg(&s->scanned);
+        }))
+      return;
+    const unsigned long long nf = st.nf, mf = st.mf;
     if (first) {
-      const unsigned long long sc = __ldcg(&s->scanned);
+      const unsigned long long sc = st.scanned;
       c->reached_arcs += mf;
       c->arcs_bu += sc;
       c->bytes += bu ? sc * 4 + sc / 8 + 4 * nf : 8 * nf;
@@ -418,7 +320,7 @@ __global__ void __launch_bounds__(kBfsThreads, 2) k_bfs_persist(const __grid_con
       bu = true;
     } else if (bu && nf < R.n / 18) {
       bits_to_items(R, cur, other, queue, &s->nitems, st, gwarp, nwarps);
-      if (!grid_barrier(&c->bar, target, R.wait_ns)) return;
+      if (!grid_barrier(&c->bar, target, R.wait_ns, [&] { st.nitems = __ldcg(&s->nitems); })) return;
       bu = false;
     }
     if (bu) {
@@ -432,9 +334,8 @@ __global__ void __launch_bounds__(kBfsThreads, 2) k_bfs_persist(const __grid_con
         c->arcs_td += mf;
         c->bytes += 16 * nf + 8 * mf;
       }
-      top_down(R, queue, __ldcg(&s->nitems), cur, (int32_t)d + 1, (d & 1) ? R.q0 : R.q1, sn, st, gwarp, nwarps);
+      top_down(R, queue, st.nitems, cur, (int32_t)d + 1, (d & 1) ? R.q0 : R.q1, sn, st, gwarp, nwarps);
     }
-    if (!grid_barrier(&c->bar, target, R.wait_ns)) return;
   }
   if (first) c->levels = d;
 }

@@ -50,8 +50,6 @@ enum WsSlot {
   WS_PERM_IN,    // inputs permuted to internal order
   WS_PERM_IN2,
   WS_PERM_OFF,   // caller-order row offsets
-  WS_SSSP_L,     // SSSP: vertices with light arcs (bitmap)
-  WS_SSSP_H,     // SSSP: vertices with heavy arcs (bitmap)
   WS_NSLOTS
 };
 
@@ -362,9 +360,8 @@ struct OwnHeads {
 // One edge-balanced relaxation pass (sssp.cu): the frontier `queue` (nq vertices, exclusive
 // scan `prefix` of their arc counts, `total` arcs starting at base[u]) offers srcdist[u] + w to
 // dist[head] (atomic min), and sets the head's bit in `changed` (may be null) on improvement.
-// srcdist == dist: the one-GPU relaxation; otherwise dist is a separate offer array, an offer at
-// or above known[head] (an upper bound of the head's distance; may be null) is dropped, and the
-// heads in `own` are relaxed in place.  tstart holds ceil(total / sssp_tile_arcs()) entries;
+// dist is a separate offer array, an offer at or above known[head] (an upper bound of the head's
+// distance; may be null) is dropped, and the heads in `own` are relaxed in place.  tstart holds ceil(total / sssp_tile_arcs()) entries;
 // error is set if a tile holds too many owners.
 uint64_t sssp_tile_arcs();
 // The binned form of a relaxation pass as offers (sssp.cu): every row of the bins whose bit is set

@@ -105,6 +105,34 @@ struct RowPlan {
   const uint64_t* seg_slot;
 };
 
+// Blocks of one segment: enough for one pass, at most kSegBlocks an SM (the blocks of a long
+// segment stride over it).
+constexpr int kSegBlocks = 16;
+
+// The bins' rows (the window chunks instead of bins 6 and 7 with `windows`).
+inline RowPlan plan_rows(const DegreeBins& B, bool windows, int seg_blocks = kSegBlocks) {
+  RowPlan P{};
+  P.rows = B.rows;
+  P.chunk_row = B.hub_chunk_row;
+  P.chunk_begin = B.hub_chunk_begin;
+  P.chunk = B.sched.hub_chunk;
+  if (windows) {
+    P.seg_row = B.seg_row;
+    P.seg_begin = B.seg_begin;
+    P.seg_end = B.seg_end;
+    P.seg_slot = B.seg_slot;
+  }
+  for (int k = 0; k < 8; ++k) {
+    const int b = 7 - k;  // segment k holds bin 7 - k
+    const uint64_t items = k == 0 ? (windows ? B.seg_nchunks : B.n_hub_chunks) : (k == 1 && windows) ? 0 : B.count[b];
+    P.count[k] = (uint32_t)items;
+    P.row0[k] = (uint32_t)B.start[b];
+    const uint64_t threads = items * (k < 2 ? kCta : 1ull << b);
+    P.block[k + 1] = P.block[k] + (items ? grid_for(threads, kCta, seg_blocks) : 0);
+  }
+  return P;
+}
+
 // Every bin of a superstep in one launch.  Latency and tails bound a superstep of a small graph
 // when its bins run one after the other (RMAT-16, seven bins: 40 us a superstep, each bin 7-20 us
 // alone); side by side they take as long as the slowest.  The blocks of the longest rows come
@@ -175,33 +203,11 @@ __global__ void k_rows_chunk_finish(const uint32_t* __restrict__ rows, uint64_t 
   finish_end(fin, 0);
 }
 
-// Blocks of one segment: enough for one pass, at most kSegBlocks an SM (the blocks of a long
-// segment stride over it).
-constexpr int kSegBlocks = 16;
-
 // Launch the reductions of every non-empty row.  `partial` holds bins.n_partials doubles.
 template <class Gather, class Finish>
 int reduce_rows(const DegreeBins& B, const uint64_t* off, Gather gat, Finish fin, double* partial, cudaStream_t s) {
-  RowPlan P{};
   const bool windows = B.seg_nchunks != 0;  // the rows above cta_min, window by window
-  P.rows = B.rows;
-  P.chunk_row = B.hub_chunk_row;
-  P.chunk_begin = B.hub_chunk_begin;
-  P.chunk = B.sched.hub_chunk;
-  if (windows) {
-    P.seg_row = B.seg_row;
-    P.seg_begin = B.seg_begin;
-    P.seg_end = B.seg_end;
-    P.seg_slot = B.seg_slot;
-  }
-  for (int k = 0; k < 8; ++k) {
-    const int b = 7 - k;  // segment k holds bin 7 - k
-    const uint64_t items = k == 0 ? (windows ? B.seg_nchunks : B.n_hub_chunks) : (k == 1 && windows) ? 0 : B.count[b];
-    P.count[k] = (uint32_t)items;
-    P.row0[k] = (uint32_t)B.start[b];
-    const uint64_t threads = items * (k < 2 ? kCta : 1ull << b);
-    P.block[k + 1] = P.block[k] + (items ? grid_for(threads, kCta, kSegBlocks) : 0);
-  }
+  const RowPlan P = plan_rows(B, windows);
   if (!P.block[8]) return GRE_SUCCESS;
   k_rows_all<<<P.block[8], kCta, 0, s>>>(P, off, gat, fin, partial);
   if (windows)

@@ -10,16 +10,12 @@
 //     split of delta-stepping (Meyer and Sanders 2003) only arcs lighter than delta are relaxed
 //     inside a bucket and a settled bucket's heavy arcs once.  On RMAT this relaxes each arc
 //     about 1.1 times instead of about 2.2 for a plain Bellman-Ford frontier (delta = 0);
-//   * the frontier is expanded edge-balanced in tiles of 2048 consecutive frontier arcs (the
-//     owners staged in shared memory, owner of each arc by a block max-scan), so hubs do not
-//     serialise a warp;
-//   * an improvement is a fire-and-forget atomic min on the distance plus a bit in a changed
-//     bitmap: no thread waits for an atomic's reply (hub heads receive thousands per superstep),
-//     and a pass over the bitmap builds the next frontier and far set without duplicates;
-//   * the far set is a bitmap: a limit rise scans it, reading the far vertices' distances in
-//     vertex order, 32 to a word (against a list of far vertices, read at random: RMAT-26 SSSP
-//     18.5 -> 17.8 ms);
-//   * the distance of a frontier vertex is read when its tile starts (not a copy taken at the
+//   * the superstep loop runs in one cooperative kernel (sssp_loop.cu): frontiers are queues of
+//     128-arc items, so hubs do not serialise a warp, and sets (near, bucket, far) are bitmaps;
+//   * passes over a large share of the graph go through the degree bins (below), where an
+//     improvement is a fire-and-forget atomic min on the distance plus a bit in a changed bitmap: no
+//     thread waits for an atomic's reply (hub heads receive thousands per superstep);
+//   * the distance of a frontier vertex is read when its arcs are relaxed (not a copy taken at the
 //     start of the superstep), which can only lower the values sent;
 //   * vertices without out-arcs are never queued (they have nothing to relax).
 //
@@ -31,11 +27,10 @@
 #include <cstdlib>
 
 #include "gre_internal.cuh"
+#include "rows.cuh"
+#include "sssp_loop.cuh"
 
 namespace gre {
-
-// defined in bfs.cu
-__global__ void k_queue_to_bits(const uint32_t* __restrict__ queue, uint64_t nq, uint32_t* __restrict__ bits);
 
 template <class T>
 static int ws_array(gre_graph g, int slot, uint64_t count, T** p) {
@@ -45,17 +40,6 @@ static int ws_array(gre_graph g, int slot, uint64_t count, T** p) {
   return GRE_SUCCESS;
 }
 
-
-// Arc counts of the queued vertices in the range being relaxed (light: [off[v], lend[v]),
-// heavy: [lend[v], off[v+1])), for the scan.
-template <bool HEAVY>
-__global__ void k_sssp_degrees(const uint32_t* __restrict__ queue, uint64_t nq, const uint64_t* __restrict__ off,
-                               const uint64_t* __restrict__ lend, uint64_t* __restrict__ deg) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nq; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t v = queue[i];
-    deg[i] = HEAVY ? off[v + 1] - lend[v] : lend[v] - off[v];
-  }
-}
 
 // Light/heavy split of each row for bucket width delta (warp per row, stable within a class).
 __global__ void k_split_light_heavy(uint64_t n, const uint64_t* __restrict__ off, const uint32_t* __restrict__ col,
@@ -91,7 +75,8 @@ __global__ void k_split_light_heavy(uint64_t n, const uint64_t* __restrict__ off
   }
 }
 
-// Edge-balanced expansion in tiles of kTile consecutive frontier arcs.  k_tile_starts records,
+// Edge-balanced expansion in tiles of kTile consecutive frontier arcs (the partitioned path, whose
+// offers are exchanged between the supersteps).  k_tile_starts records,
 // for every tile, the frontier index owning its first arc (each frontier vertex writes the
 // tiles that begin inside its arc range, so every entry is written exactly once).  A CTA then
 // stages the owners of its tile (at most kTile + 1 of them, since queued vertices have at least
@@ -142,10 +127,8 @@ struct OfferArc {
   }
 };
 
-// OFFER: the owners' distances come from srcdist and `dist` is a separate offer array (the
-// partitioned path); otherwise from dist itself.  Either way an improved entry sets its bit in
-// `changed` when that bitmap is given.
-template <bool OFFER>
+// The partitioned path's relaxation: the owners' distances come from srcdist and `dist` is a separate
+// offer array; an improved entry sets its bit in `changed` when that bitmap is given.
 __global__ void __launch_bounds__(kTileThreads) k_sssp_relax(const uint32_t* __restrict__ queue, uint64_t nq,
                                                              const uint64_t* __restrict__ prefix, uint64_t total, const uint32_t* __restrict__ start,
                                                              const uint64_t* __restrict__ base, const uint32_t* __restrict__ col,
@@ -177,7 +160,7 @@ __global__ void __launch_bounds__(kTileThreads) k_sssp_relax(const uint32_t* __r
       const uint64_t r = p > t0 ? p - t0 : 0;
       s_rel[j] = (uint16_t)r;
       s_arc[j] = base[u] + (t0 + r - p);
-      s_du[j] = __ldcg((OFFER ? srcdist : dist) + u);
+      s_du[j] = __ldcg(srcdist + u);
     }
     __syncthreads();
     // owner of every tile position: mark where each owner's arcs begin, then a running maximum
@@ -213,33 +196,16 @@ __global__ void __launch_bounds__(kTileThreads) k_sssp_relax(const uint32_t* __r
       v[k] = ok ? __ldg(col + arc) : 0u;
       wt[k] = ok ? __ldg(w + arc) : 0u;
     }
-    if (OFFER) {
-      OfferArc oa[kTileItems];
+    OfferArc oa[kTileItems];
 #pragma unroll
-      for (int k = 0; k < kTileItems; ++k) {
-        const bool ok = (uint32_t)k * kTileThreads + threadIdx.x < len;
-        dv[k] = ok ? oa[k].probe(own, known, dist, v[k], du[k] + wt[k]) : 0u;
-      }
+    for (int k = 0; k < kTileItems; ++k) {
+      const bool ok = (uint32_t)k * kTileThreads + threadIdx.x < len;
+      dv[k] = ok ? oa[k].probe(own, known, dist, v[k], du[k] + wt[k]) : 0u;
+    }
 #pragma unroll
-      for (int k = 0; k < kTileItems; ++k) {
-        const uint32_t nd = du[k] + wt[k];
-        if (nd < dv[k]) oa[k].commit(own, dist, changed, v[k], nd);
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < kTileItems; ++k) {
-        const bool ok = (uint32_t)k * kTileThreads + threadIdx.x < len;
-        dv[k] = ok ? __ldcg(dist + v[k]) : 0u;
-      }
-#pragma unroll
-      for (int k = 0; k < kTileItems; ++k) {
-        const bool ok = (uint32_t)k * kTileThreads + threadIdx.x < len;
-        const uint32_t nd = du[k] + wt[k];
-        if (ok && nd < dv[k]) {
-          atomicMin(dist + v[k], nd);
-          if (changed) atomicOr(changed + (v[k] >> 5), 1u << (v[k] & 31u));
-        }
-      }
+    for (int k = 0; k < kTileItems; ++k) {
+      const uint32_t nd = du[k] + wt[k];
+      if (nd < dv[k]) oa[k].commit(own, dist, changed, v[k], nd);
     }
     __syncthreads();
   }
@@ -315,81 +281,68 @@ struct RelaxRange {
   }
 };
 
-// c may be null (the caller counts the arcs another way)
-__device__ __forceinline__ void add_arcs(unsigned long long* c, unsigned long long k) {
-  for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
-  if ((threadIdx.x & 31u) == 0 && k && c) atomicAdd(c, k);
-}
-
+// Rows of one bin (G lanes each) of block `part` of `nparts`.
 template <int G, bool OFFER>
-__global__ void __launch_bounds__(256) k_relax_lanes(const uint32_t* __restrict__ rows, uint64_t count, RelaxRange R) {
-  const uint32_t lane = threadIdx.x & 31u, lig = lane % G;
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  unsigned long long arcs = 0;
-  for (uint64_t base = warp * (32 / G); base < count; base += nwarps * (32 / G)) {
-    const uint64_t i = base + lane / G;
-    if (i >= count) continue;
+__device__ __forceinline__ void relax_lanes(const uint32_t* __restrict__ rows, uint64_t count, uint32_t part, uint32_t nparts,
+                                            const RelaxRange& R, unsigned long long* arcs) {
+  const uint32_t lig = threadIdx.x % G;
+  for (uint64_t i = (uint64_t)part * (256 / G) + threadIdx.x / G; i < count; i += (uint64_t)nparts * (256 / G)) {
     const uint32_t v = rows[i];
     if (!R.in(v)) continue;
     uint64_t lo, hi;
     R.range(v, &lo, &hi);
     if (lo >= hi) continue;
-    if (lig == 0) arcs += hi - lo;
+    if (lig == 0) *arcs += hi - lo;
     R.template relax<OFFER>(R.template own<OFFER>(v), lo + lig, hi, G);
   }
-  add_arcs(R.arcs, arcs);
 }
 
+// All bins in one launch, the longest rows first (rows::k_rows_all's plan): one after the other each
+// bin's own tail of 15-25 us added up (RMAT-22, four sources: 10.1 -> 8.2 ms).
 template <bool OFFER>
-__global__ void __launch_bounds__(256) k_relax_cta(const uint32_t* __restrict__ rows, uint64_t count, RelaxRange R) {
-  unsigned long long arcs = 0;
-  for (uint64_t i = blockIdx.x; i < count; i += gridDim.x) {
-    const uint32_t v = rows[i];
-    if (!R.in(v)) continue;
-    uint64_t lo, hi;
-    R.range(v, &lo, &hi);
-    if (threadIdx.x == 0 && hi > lo) arcs += hi - lo;
-    R.template relax<OFFER>(R.template own<OFFER>(v), lo + threadIdx.x, hi, blockDim.x);
+__global__ void __launch_bounds__(256) k_relax_all(const __grid_constant__ rows::RowPlan P, const RelaxRange R) {
+  uint32_t s = 0;
+  while (blockIdx.x >= P.block[s + 1]) ++s;
+  const uint32_t part = blockIdx.x - P.block[s], nparts = P.block[s + 1] - P.block[s], count = P.count[s];
+  const uint32_t* rows = P.rows + P.row0[s];
+  unsigned long long arcs[1] = {0};
+  if (s < 2) {
+    // a CTA per row, or per chunk of a longer row: arcs [chunk_begin[c], + chunk) cut to the range
+    for (uint64_t c = part; c < count; c += nparts) {
+      const uint32_t v = rows[s == 0 ? P.chunk_row[c] : c];
+      if (!R.in(v)) continue;
+      uint64_t lo, hi;
+      R.range(v, &lo, &hi);
+      if (s == 0) {
+        const uint64_t c0 = P.chunk_begin[c], c1 = c0 + P.chunk;
+        lo = lo > c0 ? lo : c0;
+        hi = hi < c1 ? hi : c1;
+      }
+      if (lo >= hi) continue;
+      if (threadIdx.x == 0) arcs[0] += hi - lo;
+      R.template relax<OFFER>(R.template own<OFFER>(v), lo + threadIdx.x, hi, 256);
+    }
+  } else if (s == 2) {
+    relax_lanes<32, OFFER>(rows, count, part, nparts, R, arcs);
+  } else if (s == 3) {
+    relax_lanes<16, OFFER>(rows, count, part, nparts, R, arcs);
+  } else if (s == 4) {
+    relax_lanes<8, OFFER>(rows, count, part, nparts, R, arcs);
+  } else if (s == 5) {
+    relax_lanes<4, OFFER>(rows, count, part, nparts, R, arcs);
+  } else if (s == 6) {
+    relax_lanes<2, OFFER>(rows, count, part, nparts, R, arcs);
+  } else {
+    relax_lanes<1, OFFER>(rows, count, part, nparts, R, arcs);
   }
-  add_arcs(R.arcs, arcs);
-}
-
-// chunk c: arcs [chunk_begin[c], + chunk) of the row, cut to the light or heavy range
-template <bool OFFER>
-__global__ void __launch_bounds__(256) k_relax_chunks(const uint32_t* __restrict__ rows, const uint64_t* __restrict__ chunk_row,
-                                                      const uint64_t* __restrict__ chunk_begin, uint64_t nchunks, uint64_t chunk,
-                                                      RelaxRange R) {
-  unsigned long long arcs = 0;
-  for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
-    const uint32_t v = rows[chunk_row[c]];
-    if (!R.in(v)) continue;
-    uint64_t lo, hi;
-    R.range(v, &lo, &hi);
-    const uint64_t c0 = chunk_begin[c], c1 = c0 + chunk;
-    lo = lo > c0 ? lo : c0;
-    hi = hi < c1 ? hi : c1;
-    if (lo >= hi) continue;
-    if (threadIdx.x == 0) arcs += hi - lo;
-    R.template relax<OFFER>(R.template own<OFFER>(v), lo + threadIdx.x, hi, blockDim.x);
-  }
-  add_arcs(R.arcs, arcs);
+  __shared__ BlockSums<1> sums;
+  if (R.arcs) sums.add(arcs, {R.arcs});  // null: the caller counts the arcs another way
 }
 
 template <bool OFFER>
 static int relax_binned(const DegreeBins& B, const RelaxRange& R, cudaStream_t s) {
-  const uint32_t* r = B.rows;
-  auto grid = [](uint64_t threads) { return grid_for(threads, 256, 8); };
-  if (B.count[0]) k_relax_lanes<1, OFFER><<<grid(B.count[0]), 256, 0, s>>>(r + B.start[0], B.count[0], R);
-  if (B.count[1]) k_relax_lanes<2, OFFER><<<grid(B.count[1] * 2), 256, 0, s>>>(r + B.start[1], B.count[1], R);
-  if (B.count[2]) k_relax_lanes<4, OFFER><<<grid(B.count[2] * 4), 256, 0, s>>>(r + B.start[2], B.count[2], R);
-  if (B.count[3]) k_relax_lanes<8, OFFER><<<grid(B.count[3] * 8), 256, 0, s>>>(r + B.start[3], B.count[3], R);
-  if (B.count[4]) k_relax_lanes<16, OFFER><<<grid(B.count[4] * 16), 256, 0, s>>>(r + B.start[4], B.count[4], R);
-  if (B.count[5]) k_relax_lanes<32, OFFER><<<grid(B.count[5] * 32), 256, 0, s>>>(r + B.start[5], B.count[5], R);
-  if (B.count[6]) k_relax_cta<OFFER><<<grid(B.count[6] * 256), 256, 0, s>>>(r + B.start[6], B.count[6], R);
-  if (B.count[7])
-    k_relax_chunks<OFFER><<<grid(B.n_hub_chunks * 256), 256, 0, s>>>(r + B.start[7], B.hub_chunk_row, B.hub_chunk_begin,
-                                                                     B.n_hub_chunks, B.sched.hub_chunk, R);
+  const rows::RowPlan P = rows::plan_rows(B, false);
+  if (P.block[8]) k_relax_all<OFFER><<<P.block[8], 256, 0, s>>>(P, R);
   GRE_LAUNCH_CHECK();
   return GRE_SUCCESS;
 }
@@ -458,37 +411,22 @@ struct PullRange {
   }
 };
 
-__device__ __forceinline__ void add_counts(unsigned long long* c, unsigned long long scanned, unsigned long long hits) {
-  for (int o = 16; o > 0; o >>= 1) {
-    scanned += __shfl_xor_sync(0xffffffffu, scanned, o);
-    hits += __shfl_xor_sync(0xffffffffu, hits, o);
-  }
-  if ((threadIdx.x & 31u) == 0) {
-    if (scanned) atomicAdd(c, scanned);
-    if (hits) atomicAdd(c + 1, hits);
-  }
-}
-
 // G lanes per row; the group's lanes share the row, so they take every branch together and the
 // group minimum is a shuffle over the group's own lanes
 template <int G>
-__global__ void __launch_bounds__(256) k_pull_lanes(const uint32_t* __restrict__ rows, uint64_t count, PullRange R) {
+__device__ __forceinline__ void pull_lanes(const uint32_t* __restrict__ rows, uint64_t count, uint32_t part, uint32_t nparts,
+                                           const PullRange& R, unsigned long long (&n)[2]) {
   const uint32_t lane = threadIdx.x & 31u, lig = lane % G;
   const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane - lig));
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  unsigned long long scanned = 0, hits = 0;
-  for (uint64_t base = warp * (32 / G); base < count; base += nwarps * (32 / G)) {
-    const uint64_t i = base + lane / G;
-    if (i >= count) continue;
+  for (uint64_t i = (uint64_t)part * (256 / G) + threadIdx.x / G; i < count; i += (uint64_t)nparts * (256 / G)) {
     const uint32_t v = rows[i];
     const uint32_t dv = __ldcg(R.dist + v);
     if (dv < R.lo) continue;
     uint64_t a0, a1;
     R.range(v, &a0, &a1);
     if (a0 >= a1) continue;
-    if (lig == 0) scanned += a1 - a0;
-    uint32_t b = R.best(a0 + lig, a1, G, &hits);
+    if (lig == 0) n[0] += a1 - a0;
+    uint32_t b = R.best(a0 + lig, a1, G, &n[1]);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) {
       const uint32_t x = __shfl_xor_sync(gmask, b, o);
@@ -496,92 +434,56 @@ __global__ void __launch_bounds__(256) k_pull_lanes(const uint32_t* __restrict__
     }
     if (lig == 0) R.improve(v, dv, b);
   }
-  add_counts(R.counts, scanned, hits);
 }
 
-__device__ __forceinline__ uint32_t warp_min(uint32_t b) {
-  for (int o = 16; o > 0; o >>= 1) {
-    const uint32_t x = __shfl_xor_sync(0xffffffffu, b, o);
-    b = x < b ? x : b;
+// All bins in one launch, as k_relax_all.
+__global__ void __launch_bounds__(256) k_pull_all(const __grid_constant__ rows::RowPlan P, const PullRange R) {
+  uint32_t s = 0;
+  while (blockIdx.x >= P.block[s + 1]) ++s;
+  const uint32_t part = blockIdx.x - P.block[s], nparts = P.block[s + 1] - P.block[s], count = P.count[s];
+  const uint32_t* rows = P.rows + P.row0[s];
+  unsigned long long n[2] = {0, 0};  // arcs scanned, frontier hits
+  if (s < 2) {
+    // a CTA per row, or per chunk of a longer row, cut to the light or heavy range; each warp
+    // offers its own minimum (at most 8 atomics per improved row or chunk)
+    for (uint64_t c = part; c < count; c += nparts) {
+      const uint32_t v = rows[s == 0 ? P.chunk_row[c] : c];
+      const uint32_t dv = __ldcg(R.dist + v);
+      if (dv < R.lo) continue;
+      uint64_t a0, a1;
+      R.range(v, &a0, &a1);
+      if (s == 0) {
+        const uint64_t c0 = P.chunk_begin[c], c1 = c0 + P.chunk;
+        a0 = a0 > c0 ? a0 : c0;
+        a1 = a1 < c1 ? a1 : c1;
+      }
+      if (a0 >= a1) continue;
+      if (threadIdx.x == 0) n[0] += a1 - a0;
+      const uint32_t b = __reduce_min_sync(0xffffffffu, R.best(a0 + threadIdx.x, a1, 256, &n[1]));
+      if ((threadIdx.x & 31u) == 0) R.improve(v, dv, b);
+    }
+  } else if (s == 2) {
+    pull_lanes<32>(rows, count, part, nparts, R, n);
+  } else if (s == 3) {
+    pull_lanes<16>(rows, count, part, nparts, R, n);
+  } else if (s == 4) {
+    pull_lanes<8>(rows, count, part, nparts, R, n);
+  } else if (s == 5) {
+    pull_lanes<4>(rows, count, part, nparts, R, n);
+  } else if (s == 6) {
+    pull_lanes<2>(rows, count, part, nparts, R, n);
+  } else {
+    pull_lanes<1>(rows, count, part, nparts, R, n);
   }
-  return b;
-}
-
-// a CTA per row; each warp offers its own minimum (at most 8 atomics per improved row)
-__global__ void __launch_bounds__(256) k_pull_cta(const uint32_t* __restrict__ rows, uint64_t count, PullRange R) {
-  unsigned long long scanned = 0, hits = 0;
-  for (uint64_t i = blockIdx.x; i < count; i += gridDim.x) {
-    const uint32_t v = rows[i];
-    const uint32_t dv = __ldcg(R.dist + v);
-    if (dv < R.lo) continue;
-    uint64_t a0, a1;
-    R.range(v, &a0, &a1);
-    if (a0 >= a1) continue;
-    if (threadIdx.x == 0) scanned += a1 - a0;
-    const uint32_t b = warp_min(R.best(a0 + threadIdx.x, a1, blockDim.x, &hits));
-    if ((threadIdx.x & 31u) == 0) R.improve(v, dv, b);
-  }
-  add_counts(R.counts, scanned, hits);
-}
-
-// a CTA per 65536-arc chunk of the longest rows, cut to the light or heavy range
-__global__ void __launch_bounds__(256) k_pull_chunks(const uint32_t* __restrict__ rows, const uint64_t* __restrict__ chunk_row,
-                                                     const uint64_t* __restrict__ chunk_begin, uint64_t nchunks, uint64_t chunk,
-                                                     PullRange R) {
-  unsigned long long scanned = 0, hits = 0;
-  for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
-    const uint32_t v = rows[chunk_row[c]];
-    const uint32_t dv = __ldcg(R.dist + v);
-    if (dv < R.lo) continue;
-    uint64_t a0, a1;
-    R.range(v, &a0, &a1);
-    const uint64_t c0 = chunk_begin[c], c1 = c0 + chunk;
-    a0 = a0 > c0 ? a0 : c0;
-    a1 = a1 < c1 ? a1 : c1;
-    if (a0 >= a1) continue;
-    if (threadIdx.x == 0) scanned += a1 - a0;
-    const uint32_t b = warp_min(R.best(a0 + threadIdx.x, a1, blockDim.x, &hits));
-    if ((threadIdx.x & 31u) == 0) R.improve(v, dv, b);
-  }
-  add_counts(R.counts, scanned, hits);
+  __shared__ BlockSums<2> sums;
+  sums.add(n, {R.counts, R.counts + 1});
 }
 
 static int pull_binned(const DegreeBins& B, const PullRange& R, cudaStream_t s) {
-  const uint32_t* r = B.rows;
-  auto grid = [](uint64_t threads) { return grid_for(threads, 256, 8); };
-  if (B.count[0]) k_pull_lanes<1><<<grid(B.count[0]), 256, 0, s>>>(r + B.start[0], B.count[0], R);
-  if (B.count[1]) k_pull_lanes<2><<<grid(B.count[1] * 2), 256, 0, s>>>(r + B.start[1], B.count[1], R);
-  if (B.count[2]) k_pull_lanes<4><<<grid(B.count[2] * 4), 256, 0, s>>>(r + B.start[2], B.count[2], R);
-  if (B.count[3]) k_pull_lanes<8><<<grid(B.count[3] * 8), 256, 0, s>>>(r + B.start[3], B.count[3], R);
-  if (B.count[4]) k_pull_lanes<16><<<grid(B.count[4] * 16), 256, 0, s>>>(r + B.start[4], B.count[4], R);
-  if (B.count[5]) k_pull_lanes<32><<<grid(B.count[5] * 32), 256, 0, s>>>(r + B.start[5], B.count[5], R);
-  if (B.count[6]) k_pull_cta<<<grid(B.count[6] * 256), 256, 0, s>>>(r + B.start[6], B.count[6], R);
-  if (B.count[7])
-    k_pull_chunks<<<grid(B.n_hub_chunks * 256), 256, 0, s>>>(r + B.start[7], B.hub_chunk_row, B.hub_chunk_begin, B.n_hub_chunks,
-                                                            B.sched.hub_chunk, R);
+  const rows::RowPlan P = rows::plan_rows(B, false);
+  if (P.block[8]) k_pull_all<<<P.block[8], 256, 0, s>>>(P, R);
   GRE_LAUNCH_CHECK();
   return GRE_SUCCESS;
-}
-
-// Which vertices have light arcs ([off, lend) non-empty) and which heavy ones ([lend, off+1)):
-// one bit each, so that the passes below test a word instead of reading three offsets per vertex.
-__global__ void k_sssp_classes(uint64_t n, const uint64_t* __restrict__ off, const uint64_t* __restrict__ lend,
-                               uint32_t* __restrict__ lbits, uint32_t* __restrict__ hbits) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < n; base += stride) {
-    const uint64_t v = base + (threadIdx.x & 31u);
-    bool light = false, heavy = false;
-    if (v < n) {
-      const uint64_t a0 = off[v], am = lend[v], a1 = off[v + 1];
-      light = am > a0;
-      heavy = a1 > am;
-    }
-    const uint32_t lw = __ballot_sync(0xffffffffu, light), hw = __ballot_sync(0xffffffffu, heavy);
-    if ((threadIdx.x & 31u) == 0) {
-      lbits[base >> 5] = lw;
-      hbits[base >> 5] = hw;
-    }
-  }
 }
 
 int sssp_relax_binned_offer(cudaStream_t stream, const DegreeBins& B, const uint32_t* front, const uint64_t* off,
@@ -604,150 +506,6 @@ int sssp_split_rows(cudaStream_t stream, uint64_t rows, const uint64_t* off, con
   if (rows) k_split_light_heavy<<<grid_for(rows * 32, 256), 256, 0, stream>>>(rows, off, col, w, delta, ocol, ow, lend);
   GRE_LAUNCH_CHECK();
   return GRE_SUCCESS;
-}
-
-constexpr int kStage = 512;  // items per list that a warp stages in shared memory (2 lists x 8 warps: 32 KB)
-
-// Classify the vertices improved by a pass (bits of `changed`, one lane per word, cleared here):
-// below the limit a vertex with light arcs joins the near queue and one with heavy arcs the
-// bucket list (once: `inbucket`), and leaves the far set; at or above the limit it joins the far
-// set (a bitmap, `infar`).  Vertices without out-arcs are dropped.  counters[0] and [4] are the
-// queue and list lengths, counters[2] the far set's size.
-__global__ void __launch_bounds__(256) k_sssp_classify(uint64_t nwords, uint32_t* __restrict__ changed, const uint32_t* __restrict__ dist,
-                                const uint32_t* __restrict__ lbits, const uint32_t* __restrict__ hbits, uint32_t near_limit,
-                                uint32_t* __restrict__ near, uint32_t* __restrict__ infar,
-                                uint32_t* __restrict__ inbucket, uint32_t* __restrict__ blist, uint32_t* __restrict__ counters) {
-  __shared__ uint32_t stage[8][2 * kStage];
-  WarpLists<2, kStage> out(stage[threadIdx.x >> 5]);
-  int far_delta = 0;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < nwords; base += stride) {
-    const uint64_t wi = base + (threadIdx.x & 31u);
-    uint32_t bits = 0, fbits = 0, bbits = 0, lw = 0, hw = 0;
-    if (wi < nwords) {
-      bits = changed[wi];
-      if (bits) {
-        changed[wi] = 0;
-        fbits = infar[wi];
-        bbits = inbucket[wi];
-        lw = lbits[wi];
-        hw = hbits[wi];
-      }
-    }
-    uint32_t set_far = 0, clear_far = 0, set_bucket = 0;
-    while (__any_sync(0xffffffffu, bits != 0)) {
-      bool to_near = false, to_bucket = false;
-      uint32_t v = 0;
-      if (bits) {
-        const uint32_t b = __ffs(bits) - 1;
-        bits &= bits - 1;
-        v = (uint32_t)(wi << 5) + b;
-        const bool light = (lw >> b) & 1u, heavy = (hw >> b) & 1u;
-        if (light || heavy) {
-          if (dist[v] < near_limit) {
-            to_near = light;
-            if (heavy && !(bbits & (1u << b))) {
-              to_bucket = true;
-              set_bucket |= 1u << b;
-            }
-            if (fbits & (1u << b)) clear_far |= 1u << b;
-          } else if (!(fbits & (1u << b))) {
-            set_far |= 1u << b;
-          }
-        }
-      }
-      out.push<0>(to_near, v, counters, near);
-      out.push<1>(to_bucket, v, counters + 4, blist);
-    }
-    if (set_far | clear_far) infar[wi] = (fbits | set_far) & ~clear_far;  // one lane owns the word
-    if (set_bucket) inbucket[wi] = bbits | set_bucket;
-    far_delta += __popc(set_far) - __popc(clear_far);
-  }
-  out.flush<0>(counters, near);
-  out.flush<1>(counters + 4, blist);
-  far_delta = __reduce_add_sync(0xffffffffu, far_delta);
-  if ((threadIdx.x & 31u) == 0 && far_delta) atomicAdd(counters + 2, (uint32_t)far_delta);
-}
-
-// The bucket's heavy arcs have been relaxed: its members leave the bucket list.
-__global__ void k_bucket_clear(const uint32_t* __restrict__ blist, uint64_t nb, uint32_t* __restrict__ inbucket) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nb; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t v = blist[i];
-    atomicAnd(inbucket + (v >> 5), ~(1u << (v & 31u)));
-  }
-}
-
-// The source joins the near queue (light arcs) and the bucket list (heavy arcs).
-__global__ void k_sssp_seed(uint32_t src, const uint64_t* __restrict__ off, const uint64_t* __restrict__ lend,
-                            uint32_t* __restrict__ dist, uint32_t* __restrict__ near, uint32_t* __restrict__ inbucket,
-                            uint32_t* __restrict__ blist, uint32_t* __restrict__ counters) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  dist[src] = 0;
-  if (lend[src] > off[src]) near[counters[0]++] = src;
-  if (off[src + 1] > lend[src]) {
-    blist[counters[4]++] = src;
-    inbucket[src >> 5] |= 1u << (src & 31u);
-  }
-}
-
-// Near-far split when the limit rises: every vertex of the far set (bitmap `infar`) whose
-// distance is now below the limit leaves it for the near queue (light arcs) and the bucket list
-// (heavy arcs; once: `inbucket`), as in k_sssp_classify; the others stay.  counters[2] (the far
-// set's size) drops by the vertices that left, counters[3] gets the smallest distance left.  A
-// scan of the bitmap reads the distances of far vertices in vertex order, 32 to a word.
-__global__ void __launch_bounds__(256) k_far_split(uint64_t nwords, uint32_t* __restrict__ infar, const uint32_t* __restrict__ dist,
-                                                   uint32_t near_limit, const uint32_t* __restrict__ lbits,
-                                                   const uint32_t* __restrict__ hbits, uint32_t* __restrict__ near,
-                                                   uint32_t* __restrict__ inbucket, uint32_t* __restrict__ blist,
-                                                   uint32_t* __restrict__ counters) {
-  __shared__ uint32_t stage[8][2 * kStage];
-  WarpLists<2, kStage> out(stage[threadIdx.x >> 5]);
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  uint32_t dmin = 0xffffffffu, nmoved = 0;
-  for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < nwords; base += stride) {
-    const uint64_t wi = base + (threadIdx.x & 31u);
-    uint32_t bits = wi < nwords ? infar[wi] : 0u;
-    const uint32_t fbits = bits;
-    uint32_t moved = 0, set_bucket = 0, bbits = 0, lw = 0, hw = 0;
-    if (bits) {
-      bbits = inbucket[wi];
-      lw = lbits[wi];
-      hw = hbits[wi];
-    }
-    while (__any_sync(0xffffffffu, bits != 0)) {
-      bool to_near = false, to_bucket = false;
-      uint32_t v = 0;
-      if (bits) {
-        const uint32_t b = __ffs(bits) - 1;
-        bits &= bits - 1;
-        v = (uint32_t)(wi << 5) + b;
-        const uint32_t d = dist[v];
-        if (d < near_limit) {
-          moved |= 1u << b;
-          to_near = (lw >> b) & 1u;
-          if (((hw >> b) & 1u) && !(bbits & (1u << b))) {
-            to_bucket = true;
-            set_bucket |= 1u << b;
-          }
-        } else {
-          dmin = min(dmin, d);
-        }
-      }
-      out.push<0>(to_near, v, counters, near);
-      out.push<1>(to_bucket, v, counters + 4, blist);
-    }
-    if (moved) infar[wi] = fbits & ~moved;
-    if (set_bucket) inbucket[wi] = bbits | set_bucket;
-    nmoved += __popc(moved);
-  }
-  out.flush<0>(counters, near);
-  out.flush<1>(counters + 4, blist);
-  dmin = __reduce_min_sync(0xffffffffu, dmin);
-  nmoved = __reduce_add_sync(0xffffffffu, nmoved);
-  if ((threadIdx.x & 31u) == 0) {
-    if (dmin != 0xffffffffu) atomicMin(counters + 3, dmin);
-    if (nmoved) atomicSub(counters + 2, nmoved);
-  }
 }
 
 struct AddU64 {
@@ -781,22 +539,13 @@ int sssp_delta(gre_graph g, uint32_t* delta) {
   return GRE_SUCCESS;
 }
 
-// counters: [0] near appends, [1] overflow flag, [2] size of the far set, [3] smallest far
-// distance left by a split, [4] bucket-list appends (from its size)
-static int init_counters(gre_graph g, uint32_t* cnt, uint32_t near, uint32_t nfar, uint32_t nbucket) {
-  const uint32_t h[8] = {near, 0, nfar, 0xffffffffu, nbucket, 0, 0, 0};  // pageable: staged before the call returns
-  GRE_CUDA(cudaMemcpyAsync(cnt, h, sizeof h, cudaMemcpyHostToDevice, g->stream));
-  return GRE_SUCCESS;
-}
-
 // Resident CTAs of the relaxation kernel per SM: the grid is exactly one wave, so that no
 // CTA starts its tiles late.
-template <bool OFFER>
 static int relax_blocks_per_sm() {
   static int per_sm = 0;
   if (!per_sm) {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_sssp_relax<OFFER>, kTileThreads, 0) != cudaSuccess || b < 1) b = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_sssp_relax, kTileThreads, 0) != cudaSuccess || b < 1) b = 1;
     per_sm = b;
   }
   return per_sm;
@@ -811,6 +560,19 @@ static uint64_t binned_frontier() {
   return 16;
 }
 uint64_t sssp_binned_divisor() { return binned_frontier(); }
+
+// A pass of the loop's kernel with at least this many arcs takes the wide form: no lane waits for
+// its atomics, and a second phase over the bitmap classifies
+// (GRE_SSSP_WIDE=<arcs> overrides).  RMAT-22, a pass of 8.5M arcs: 304 us classified on the spot, 145 us
+// wide; thresholds of 2^16, 2^18 and 2^20 arcs measured alike (10.0-10.6 ms for four sources).
+static uint64_t wide_pass() {
+  if (const char* e = getenv("GRE_SSSP_WIDE")) return strtoull(e, nullptr, 10);
+  return 1ull << 18;
+}
+
+// Below this many arcs no pass is long enough to leave the loop's kernel for (about 35 us of
+// launches and a counter read), unless GRE_SSSP_BINNED asks for it.
+constexpr uint64_t kBinnedMinArcs = 1ull << 22;
 
 // Whether the large heavy passes pull (over the vertices that can still improve) instead of
 // pushing (along the bucket's heavy arcs), where the weights allow it (g->w32_symmetric).
@@ -853,7 +615,8 @@ int sssp_bins(gre_graph g, bool in, const DegreeBins** out) {
   return GRE_SUCCESS;
 }
 
-// The relaxation of one frontier pass: tile starts, then k_sssp_relax over one wave of CTAs.
+// The relaxation of one frontier pass of the partitioned path: tile starts, then k_sssp_relax over one
+// wave of CTAs.
 int sssp_relax_tiles(cudaStream_t stream, const uint32_t* queue, uint64_t nq, const uint64_t* prefix, uint64_t total,
                      uint32_t* tstart, const uint64_t* base, const uint32_t* col, const uint32_t* w, const uint32_t* srcdist,
                      uint32_t* dist, uint32_t* changed, uint32_t* error, const uint32_t* known, const OwnHeads& own) {
@@ -862,14 +625,9 @@ int sssp_relax_tiles(cudaStream_t stream, const uint32_t* queue, uint64_t nq, co
   k_tile_starts<<<grid_for(nq, 256), 256, 0, stream>>>(prefix, nq, tstart);
   // the arc count is a launch argument: read inside the kernel instead, the relaxation
   // measured 1.7x slower on RMAT-26
-  const bool offer = srcdist != dist;
-  const int grid = (int)std::min<uint64_t>(ntiles, (uint64_t)num_sms() * (offer ? relax_blocks_per_sm<true>() : relax_blocks_per_sm<false>()));
-  if (!offer)
-    k_sssp_relax<false><<<grid, kTileThreads, 0, stream>>>(queue, nq, prefix, total, tstart, base, col, w, nullptr, dist, changed,
-                                                           error, nullptr, OwnHeads());
-  else
-    k_sssp_relax<true><<<grid, kTileThreads, 0, stream>>>(queue, nq, prefix, total, tstart, base, col, w, srcdist, dist, changed,
-                                                          error, known, own);
+  const int grid = (int)std::min<uint64_t>(ntiles, (uint64_t)num_sms() * relax_blocks_per_sm());
+  k_sssp_relax<<<grid, kTileThreads, 0, stream>>>(queue, nq, prefix, total, tstart, base, col, w, srcdist, dist, changed, error,
+                                                  known, own);
   GRE_LAUNCH_CHECK();
   return GRE_SUCCESS;
 }
@@ -897,196 +655,125 @@ static int ensure_split(gre_graph g, uint32_t delta) {
 // delta-stepping (Meyer and Sanders 2003): inside a bucket only light arcs (w < delta) are
 // relaxed, repeatedly, as the bucket's distances settle; when the bucket is done, the heavy arcs
 // of every vertex it settled are relaxed once (they can only reach later buckets).  delta = 0:
-// Bellman-Ford frontier over all arcs.
-static int sssp_one(gre_graph g, uint32_t src, uint32_t* dist, gre_stats* st, bool record, uint32_t delta) {
-  const uint64_t n = g->n;
+// Bellman-Ford frontier over all arcs.  The loop runs in sssp_loop.cu's kernel, which comes back
+// for the passes over a large share of the graph.
+static int sssp_one(gre_graph g, uint32_t src, uint32_t* dist, gre_stats* st, bool record, uint32_t delta, uint64_t* reached_arcs) {
+  const uint64_t n = g->n, m = g->m;
   const uint64_t nwords = (n + 31) >> 5;
   if (delta) GRE_CHECK(ensure_split(g, delta));
-  const uint64_t* off = g->off;
-  const uint64_t* lend = delta ? g->sssp_split.lsplit : g->off + 1;  // end of each row's light arcs
-  const uint32_t* col = delta ? g->sssp_split.col : g->col;
-  const uint32_t* w = delta ? g->sssp_split.w : g->w32;
-  uint32_t *qa, *qb, *changed, *cnt, *infar, *tstart, *inbucket, *blist;
-  uint64_t *deg, *prefix;
-  GRE_CHECK(ws_array(g, WS_A, n, &qa));
-  GRE_CHECK(ws_array(g, WS_B, n, &qb));
-  GRE_CHECK(ws_array(g, WS_C, nwords, &changed));
-  GRE_CHECK(ws_array(g, WS_F, n + 1, &deg));
-  GRE_CHECK(ws_array(g, WS_G, n + 1, &prefix));
-  GRE_CHECK(ws_array(g, WS_I, g->m / kTile + 2, &tstart));
-  GRE_CHECK(ws_array(g, WS_J, nwords, &infar));
-  GRE_CHECK(ws_array(g, WS_K, nwords, &inbucket));
-  GRE_CHECK(ws_array(g, WS_L, n, &blist));
-  uint32_t *lbits, *hbits;
-  GRE_CHECK(ws_array(g, WS_SSSP_L, nwords, &lbits));
-  GRE_CHECK(ws_array(g, WS_SSSP_H, nwords, &hbits));
-  // 8 uint32 counters, then the binned passes' arc count and the pull passes' scanned arcs and hits
-  GRE_CHECK(ws_array(g, WS_COUNTERS, 14, &cnt));
-  unsigned long long* binned_arcs = (unsigned long long*)(cnt + 8);
-  unsigned long long* pull_counts = (unsigned long long*)(cnt + 10);
+  SsspRun R{};
+  R.n = n;
+  R.m = m;
+  R.nwords = nwords;
+  R.off = g->off;
+  R.lend = delta ? g->sssp_split.lsplit : g->off + 1;
+  R.col = delta ? g->sssp_split.col : g->col;
+  R.w = delta ? g->sssp_split.w : g->w32;
+  R.outdeg = g->outdeg;
+  R.dist = dist;
+  const uint64_t cap = n + m / kPiece + 1;
+  uint32_t *bits, *front;
+  GRE_CHECK(ws_array(g, WS_A, cap, &R.near[0]));
+  GRE_CHECK(ws_array(g, WS_B, cap, &R.near[1]));
+  GRE_CHECK(ws_array(g, WS_C, cap, &R.heavy[0]));
+  GRE_CHECK(ws_array(g, WS_D, cap, &R.heavy[1]));
+  GRE_CHECK(ws_array(g, WS_E, 7 * nwords, &bits));
+  R.changed = bits;
+  R.infar = bits + nwords;
+  R.nbits[0] = bits + 2 * nwords;
+  R.nbits[1] = bits + 3 * nwords;
+  R.hbits[0] = bits + 4 * nwords;
+  R.hbits[1] = bits + 5 * nwords;
+  front = bits + 6 * nwords;
+  R.all_out = g->symmetric();
+  GRE_CHECK(ws_array(g, WS_F, 1, &R.ctl));
+  if (record) GRE_CHECK(ws_array(g, WS_G, GRE_MAX_RECORDED_SUPERSTEPS, &R.rec));
+  R.nrec = GRE_MAX_RECORDED_SUPERSTEPS;
+  R.wait_ns = grid_wait_ns();
+  R.src = src;
+  R.delta = delta;
+  R.limit = delta ? delta : 0xffffffffu;
+  R.fresh = true;
+  // the passes that go through the degree bins of the CSR (the symmetric CSC is the CSR)
   const bool pull = g->w32_symmetric && pull_enabled();
-  // large frontiers go through the degree bins of the CSR (the symmetric CSC is the CSR)
-  const bool sym = g->symmetric();
-  const DegreeBins* pbins = nullptr;
-  GRE_CHECK(sssp_bins(g, sym, &pbins));
-  const DegreeBins& bins = *pbins;
-  const uint64_t bdiv = binned_frontier();
-  const uint64_t pdiv = pull_arcs_divisor();
-  size_t cubbytes = 0;
-  void* cubtmp = nullptr;
-  cub::DeviceScan::ExclusiveSum(nullptr, cubbytes, deg, prefix, n + 1, g->stream);
-  GRE_CHECK(g->ws.get(WS_CUB, cubbytes, &cubtmp));
-  GRE_CUDA(cudaMemsetAsync(dist, 0xff, sizeof(uint32_t) * n, g->stream));
-  GRE_CUDA(cudaMemsetAsync(changed, 0, sizeof(uint32_t) * nwords, g->stream));
-  GRE_CUDA(cudaMemsetAsync(infar, 0, sizeof(uint32_t) * nwords, g->stream));
-  GRE_CUDA(cudaMemsetAsync(inbucket, 0, sizeof(uint32_t) * nwords, g->stream));
-  GRE_CUDA(cudaMemsetAsync(binned_arcs, 0, 3 * sizeof(unsigned long long), g->stream));
-  k_sssp_classes<<<grid_for(n, 256, 8), 256, 0, g->stream>>>(n, off, lend, lbits, hbits);
-  uint32_t limit = delta ? delta : 0xffffffffu;
-  uint64_t nq = 0, nfar = 0, nb = 0, relaxed = 0, bytes = 0;
-  uint32_t* q = qa;
-  uint32_t* nqueue = qb;
-  uint32_t steps = 0;
-  uint32_t h[8];
-  auto read_counters = [&]() -> int {
-    GRE_CUDA(cudaMemcpyAsync(h, cnt, sizeof h, cudaMemcpyDeviceToHost, g->stream));
+  const uint64_t bdiv = binned_frontier(), pdiv = pull_arcs_divisor();
+  R.big_verts = R.big_arcs = ~0ull;
+  R.wide_arcs = wide_pass();
+  const DegreeBins* bins = nullptr;
+  if (bdiv && (getenv("GRE_SSSP_BINNED") || m >= kBinnedMinArcs)) {
+    GRE_CHECK(sssp_bins(g, g->symmetric(), &bins));
+    R.big_verts = std::max<uint64_t>(1, n / bdiv);
+    if (pull && pdiv) R.big_arcs = std::max<uint64_t>(1, (m + pdiv - 1) / pdiv);
+  }
+  SsspCtl h{};
+  h.dmin[0] = h.dmin[1] = h.dmin[2] = 0xffffffffu;
+  GRE_CUDA(cudaMemcpyAsync(R.ctl, &h, sizeof h, cudaMemcpyHostToDevice, g->stream));  // pageable: staged before the call returns
+  uint64_t bytes = 0;
+  uint32_t big = 0;
+  for (;;) {
+    GRE_CHECK(sssp_loop_launch(g, R));
+    GRE_CUDA(cudaMemcpyAsync(&h, R.ctl, sizeof h, cudaMemcpyDeviceToHost, g->stream));
     GRE_CUDA(cudaStreamSynchronize(g->stream));
-    if (h[1]) {
-      set_error("gre_sssp: frontier tile overflow");
+    if (h.bar.err) {
+      set_error("gre_sssp: a grid barrier wait of the superstep loop ran out (%lld ms budget)", (long long)(R.wait_ns / 1000000ll));
+      return GRE_TIMEOUT;
+    }
+    if (h.reason == SSSP_DONE) break;
+    if (h.reason == SSSP_STUCK) {
+      set_error("gre_sssp: near-far split made no progress");
       return GRE_FAILURE;
     }
-    return GRE_SUCCESS;
-  };
-  GRE_CHECK(init_counters(g, cnt, 0, 0, 0));
-  k_sssp_seed<<<1, 32, 0, g->stream>>>(src, off, lend, dist, q, inbucket, blist, cnt);
-  GRE_LAUNCH_CHECK();
-  GRE_CHECK(read_counters());
-  nq = h[0];
-  nb = h[4];
-  // one relaxation pass over `list` (light or heavy ranges), the improvements classified into
-  // the next near queue, the bucket list and the far set
-  auto pass = [&](const uint32_t* list, uint64_t nlist, bool heavy, uint32_t* out_near) -> int {
-    bool bins_form = bdiv && nlist >= n / bdiv && nlist > 0;
-    uint64_t total = 0;
-    if (!bins_form) {  // the arcs of the frontier, for the tiles
-      if (heavy) k_sssp_degrees<true><<<grid_for(nlist, 256), 256, 0, g->stream>>>(list, nlist, off, lend, deg);
-      else k_sssp_degrees<false><<<grid_for(nlist, 256), 256, 0, g->stream>>>(list, nlist, off, lend, deg);
-      GRE_CUDA(cub::DeviceScan::ExclusiveSum(cubtmp, cubbytes, deg, prefix, nlist + 1, g->stream));
-      GRE_CUDA(cudaMemcpyAsync(&total, prefix + nlist, sizeof total, cudaMemcpyDeviceToHost, g->stream));
-      GRE_CUDA(cudaStreamSynchronize(g->stream));
-      // a small bucket with many heavy arcs (hubs among its members) pulls them instead
-      if (heavy && pull && bdiv && pdiv && total && total * pdiv >= g->m) bins_form = true;
+    R.fresh = false;
+    R.record_entry = true;
+    R.limit = h.limit;
+    ++big;
+    const uint32_t* of = front;  // the pass's frontier as bits
+    if (h.reason == SSSP_BIG_HEAVY) of = R.hbits[h.hb];
+    else GRE_CHECK(sssp_items_to_bits(g, R.near[h.nb], h.near[h.p].items, nwords, front));
+    if (h.reason == SSSP_BIG_HEAVY && pull) {
+      // only vertices at or above the limit can improve (heavy arcs from the bucket land there).
+      // (Light passes push: every unsettled vertex would have to scan its light arcs at every pass
+      // of the bucket, measured slower than the push.)
+      PullRange P{of, R.off, R.lend, R.col, R.w, dist, R.changed, R.ctl->pull_counts, true, R.limit, dist};
+      GRE_CHECK(pull_binned(*bins, P, g->stream));
+      bytes += 16 * n;  // per row: its id, distance and range bounds (arcs at the end)
+    } else {
+      RelaxRange P{of, R.off, R.lend, R.col, R.w, dist, R.changed, &R.ctl->big_arcs, h.reason == SSSP_BIG_HEAVY, nullptr};
+      GRE_CHECK(relax_binned<false>(*bins, P, g->stream));
     }
-    if (bins_form) {
-      // the heavy pass's frontier is the bucket, already a bitmap; a light frontier is made one
-      // in the scan buffer (free in this form of the pass)
-      uint32_t* front = inbucket;
-      if (!heavy) {
-        front = (uint32_t*)deg;
-        GRE_CUDA(cudaMemsetAsync(front, 0, sizeof(uint32_t) * nwords, g->stream));
-        k_queue_to_bits<<<grid_for(nlist, 256), 256, 0, g->stream>>>(list, nlist, front);
-      }
-      GRE_CHECK(init_counters(g, cnt, 0, (uint32_t)nfar, (uint32_t)nb));
-      if (pull && heavy) {
-        // the bucket's heavy arcs: only vertices at or above the limit can improve (heavy arcs
-        // from the bucket land there).  (Light passes push: every unsettled vertex would have to
-        // scan its light arcs at every pass of the bucket, measured slower than the push.)
-        PullRange P{front, off, lend, col, w, dist, changed, pull_counts, true, limit, dist};
-        GRE_CHECK(pull_binned(bins, P, g->stream));
-        bytes += 16 * n;  // per row: its id, distance and range bounds (arcs at the end)
-      } else {
-        RelaxRange R{front, off, lend, col, w, dist, changed, binned_arcs, heavy, nullptr};
-        GRE_CHECK(relax_binned<false>(bins, R, g->stream));
-      }
-      k_sssp_classify<<<grid_for(nwords, 256, 4), 256, 0, g->stream>>>(nwords, changed, dist, lbits, hbits, limit, out_near, infar,
-                                                                        inbucket, blist, cnt);
-      GRE_LAUNCH_CHECK();
-      GRE_CHECK(read_counters());
-      bytes += 4 * n + n / 8 + 8 * (uint64_t)(h[0] + h[2] - nfar + h[4] - nb);  // rows scanned, bitmap (arcs below)
-      nfar = h[2];
-      nb = h[4];
-      ++steps;
-      return GRE_SUCCESS;
+    // the frontier is used up, and the next counters' successors are empty again
+    uint32_t* used = h.reason == SSSP_BIG_HEAVY ? R.hbits[h.hb] : R.nbits[h.nb];
+    GRE_CUDA(cudaMemsetAsync(used, 0, sizeof(uint32_t) * nwords, g->stream));
+    R.p = (h.p + 1) % 3;
+    R.nb = h.nb ^ 1;
+    GRE_CUDA(cudaMemsetAsync(&R.ctl->near[(h.p + 2) % 3], 0, sizeof(SsspQueue), g->stream));
+    R.q = h.q;
+    R.hb = h.hb;
+    R.r = h.r;
+    if (h.reason == SSSP_BIG_HEAVY) {
+      R.q = (h.q + 1) % 3;
+      R.hb = h.hb ^ 1;
+      GRE_CUDA(cudaMemsetAsync(&R.ctl->heavy[(h.q + 2) % 3], 0, sizeof(SsspQueue), g->stream));
     }
-    GRE_CHECK(init_counters(g, cnt, 0, (uint32_t)nfar, (uint32_t)nb));
-    if (total) {
-      GRE_CHECK(sssp_relax_tiles(g->stream, list, nlist, prefix, total, tstart, heavy ? lend : off, col, w, dist, dist, changed,
-                                 cnt + 1, nullptr, OwnHeads()));
-      k_sssp_classify<<<grid_for(nwords, 256, 4), 256, 0, g->stream>>>(nwords, changed, dist, lbits, hbits, limit, out_near, infar,
-                                                                        inbucket, blist, cnt);
-    }
-    GRE_LAUNCH_CHECK();
-    GRE_CHECK(read_counters());
-    relaxed += total;
-    bytes += 16 * nlist + 12 * total + 8 * (uint64_t)(h[0] + h[2] - nfar + h[4] - nb);
-    nfar = h[2];
-    nb = h[4];
-    ++steps;
-    return GRE_SUCCESS;
-  };
-  for (;;) {
-    while (nq > 0) {  // light supersteps of the bucket
-      GRE_CHECK(pass(q, nq, false, nqueue));
-      nq = h[0];
-      std::swap(q, nqueue);
-      if (record) stats_record(st, nq);
-    }
-    if (nb > 0) {  // the bucket is settled: its heavy arcs, once
-      // heavy arcs land at or above the limit, so the pass normally appends nothing below it;
-      // anything it does append (a distance that wrapped around 2^32) goes after the members
-      const uint64_t members = nb;
-      GRE_CHECK(pass(blist, members, true, q));
-      k_bucket_clear<<<grid_for(members, 256), 256, 0, g->stream>>>(blist, members, inbucket);
-      GRE_LAUNCH_CHECK();
-      if (nb > members) {  // move them to the front through scratch (the ranges may overlap)
-        const size_t bytes_extra = sizeof(uint32_t) * (nb - members);
-        GRE_CUDA(cudaMemcpyAsync(deg, blist + members, bytes_extra, cudaMemcpyDeviceToDevice, g->stream));
-        GRE_CUDA(cudaMemcpyAsync(blist, deg, bytes_extra, cudaMemcpyDeviceToDevice, g->stream));
-      }
-      nb -= members;
-      nq = h[0];
-      if (record) stats_record(st, nq);
-      if (nq > 0 || nb > 0) continue;
-    }
-    if (nfar == 0) break;
-    // the near queue is empty: raise the limit (past empty buckets) and pull the far vertices below it
-    uint32_t lowest = 0;
-    for (int p = 0; nq == 0 && nb == 0 && nfar > 0; ++p) {
-      if (p == 2) {  // the second pass starts at the smallest distance left: cannot come back empty
-        set_error("gre_sssp: near-far split made no progress");
-        return GRE_FAILURE;
-      }
-      if (p == 0) limit = limit > 0xffffffffu - delta ? 0xffffffffu : limit + delta;
-      else limit = lowest > 0xffffffffu - delta ? 0xffffffffu : lowest + delta;
-      GRE_CHECK(init_counters(g, cnt, 0, (uint32_t)nfar, 0));
-      k_far_split<<<grid_for(nwords, 256, 4), 256, 0, g->stream>>>(nwords, infar, dist, limit, lbits, hbits, q, inbucket, blist,
-                                                                    cnt);
-      GRE_LAUNCH_CHECK();
-      GRE_CHECK(read_counters());
-      bytes += 4 * nwords + 4 * nfar + 4 * (uint64_t)(h[0] + h[4]);
-      nq = h[0];
-      nfar = h[2];
-      nb = h[4];
-      lowest = h[3];
-    }
+    GRE_CHECK(sssp_classify_bits(g, R));
+    bytes += 4 * n + n / 8;  // rows scanned, bitmap (arcs at the end)
   }
-  unsigned long long bc[3] = {0, 0, 0};
-  GRE_CUDA(cudaMemcpyAsync(bc, binned_arcs, sizeof bc, cudaMemcpyDeviceToHost, g->stream));
-  GRE_CUDA(cudaStreamSynchronize(g->stream));
-  relaxed += bc[0] + bc[1];
-  bytes += 12 * bc[0];              // push: column + weight + distance probe per arc
-  bytes += 4 * bc[1] + 8 * bc[2];   // pull: column per arc scanned (+ L2-held bitmap), weight + distance per hit
+  *reached_arcs = h.reached_arcs;
+  bytes += h.bytes + 12 * h.big_arcs;                          // push: column + weight + distance probe per arc
+  bytes += 4 * h.pull_counts[0] + 8 * h.pull_counts[1];        // pull: column per arc scanned (+ L2-held bitmap), weight + distance per hit
   if (st) {
+    const uint32_t steps = h.steps + big;
     st->supersteps += steps ? steps - 1 : 0;
-    st->arcs_traversed += relaxed;
+    st->arcs_traversed += h.relaxed + h.big_arcs + h.pull_counts[0];
     st->algo_bytes += bytes;
+    if (record) {
+      const uint32_t k = std::min<uint32_t>(h.nrec, GRE_MAX_RECORDED_SUPERSTEPS);
+      std::vector<unsigned long long> a(k);
+      if (k) GRE_CUDA(cudaMemcpy(a.data(), R.rec, sizeof(unsigned long long) * k, cudaMemcpyDeviceToHost));
+      for (unsigned long long x : a) stats_record(st, x);
+    }
   }
   return GRE_SUCCESS;
-}
-
-__global__ void k_dist_to_level(uint64_t n, const uint32_t* __restrict__ dist, int32_t* __restrict__ lv) {
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
-    lv[v] = dist[v] == 0xffffffffu ? -1 : 0;
 }
 
 }  // namespace gre
@@ -1110,18 +797,14 @@ int gre_sssp(gre_graph g, const uint32_t* srcs, uint32_t nsrc, uint32_t* dist, g
   uint32_t delta = 0;
   GRE_CHECK(sssp_delta(g, &delta));  // before any workspace pointer is taken (it may grow WS_CUB)
   uint32_t *dfinal, *dd;
-  int32_t* lv;
   GRE_CHECK(prepare_output(g, dist, (uint64_t)nsrc * n, WS_OUTBUF, &dfinal));
   GRE_CHECK(perm_out_begin(g, dfinal, nsrc, 4, (void**)&dd));
-  GRE_CHECK(ws_array(g, WS_H, n, &lv));
   RunTimer timer(g);
   uint64_t edges = 0;
   for (uint32_t i = 0; i < nsrc; ++i) {
-    GRE_CHECK(sssp_one(g, hs[i], dd + (uint64_t)i * n, st, nsrc == 1, delta));
-    k_dist_to_level<<<grid_for(n, 256), 256, 0, g->stream>>>(n, dd + (uint64_t)i * n, lv);
-    uint64_t e = 0;
-    GRE_CHECK(count_reached_edges(g, lv, &e));
-    edges += e;
+    uint64_t arcs = 0;
+    GRE_CHECK(sssp_one(g, hs[i], dd + (uint64_t)i * n, st, st && nsrc == 1, delta, &arcs));
+    edges += g->symmetric() ? arcs / 2 : arcs;
   }
   GRE_CHECK(perm_out_end(g, dd, dfinal, nsrc, 4));
   GRE_CHECK(finish_output(g, dist, dfinal, (uint64_t)nsrc * n));

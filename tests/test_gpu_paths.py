@@ -157,3 +157,41 @@ def test_bfs_directed_sources_only(n):
     g = G.Graph.from_csr(n, off, col)
     for r in (0, n - 1):
         np.testing.assert_array_equal(G.bfs(g, [r])[0], bfs_ref(n, off, col, [r]))
+
+
+def sssp_ref(n, off, col, w, src):
+    inf = np.iinfo(np.int64).max // 2
+    d = np.full(n, inf)
+    d[src] = 0
+    u = np.repeat(np.arange(n), np.diff(off.astype(np.int64)))
+    while True:
+        new = d.copy()
+        np.minimum.at(new, col, d[u] + w)
+        if (new == d).all():
+            return np.where(d >= inf, 0xFFFFFFFF, d).astype(np.uint32)
+        d = new
+
+
+@pytest.mark.parametrize("wide", ["0", "1000", "1000000000000"], ids=["wide", "mixed", "narrow"])
+@pytest.mark.parametrize("binned", ["0", "16"], ids=["loop", "bins"])
+@pytest.mark.parametrize("delta", ["", "0", "7", "100000"], ids=["auto", "none", "7", "100000"])
+@pytest.mark.parametrize("n,directed", [(2, False), (130, True), (1100, False), (1100, True), (20000, True), (20000, False)])
+def test_sssp_shapes(monkeypatch, n, directed, delta, binned, wide):
+    """Every form of a pass (classified on the spot, as bits, through the bins) at every kind of bucket:
+    distances equal a plain Bellman-Ford's; zero weights, sinks, long paths and unreached vertices."""
+    monkeypatch.setenv("GRE_SSSP_WIDE", wide)
+    monkeypatch.setenv("GRE_SSSP_BINNED", binned)
+    if delta:
+        monkeypatch.setenv("GRE_SSSP_DELTA", delta)
+    off, col, ids = shaped_graph(n, n, directed)
+    rng = np.random.default_rng(n)
+    w = rng.integers(0, 256, len(col)).astype(np.uint32)
+    w[rng.random(len(col)) < 0.02] = 100000
+    g = G.Graph.from_csr(n, off, col, symmetric=not directed)
+    g.loadEdgeProperty(w)
+    if n == 1100:
+        g.reorder()
+    srcs = [int(ids[0]), int(ids[n - 1])]
+    d, _ = G.sssp(g, srcs)
+    for i, s in enumerate(srcs):
+        np.testing.assert_array_equal(d[i * n:(i + 1) * n], sssp_ref(n, off, col, w, s))
