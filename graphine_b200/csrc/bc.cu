@@ -41,41 +41,6 @@ static int ws_array(gre_graph g, int slot, uint64_t count, T** p) {
 __device__ __forceinline__ double dep_term(double dep_w, double sigma_w) { return __ddiv_rn(__dadd_rn(1.0, dep_w), sigma_w); }
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
 
-static int ensure_bc_chunks(gre_graph g) {
-  ChunkTable& T = g->bc_chunks;
-  if (T.ready) return GRE_SUCCESS;
-  const uint64_t n = g->n;
-  std::vector<uint64_t> ho(n + 1);
-  GRE_CUDA(cudaMemcpy(ho.data(), g->roff, sizeof(uint64_t) * (n + 1), cudaMemcpyDeviceToHost));
-  std::vector<uint32_t> rows;
-  std::vector<uint64_t> crow, cbeg, first;
-  for (uint64_t v = 0; v < n; ++v) {
-    if (ho[v + 1] - ho[v] <= kBcChunk) continue;
-    first.push_back(crow.size());
-    for (uint64_t a = ho[v]; a < ho[v + 1]; a += kBcChunk) {
-      crow.push_back(rows.size());
-      cbeg.push_back(a);
-    }
-    rows.push_back((uint32_t)v);
-  }
-  first.push_back(crow.size());
-  T.ch = kBcChunk;
-  T.nrows = rows.size();
-  T.nchunks = crow.size();
-  GRE_CUDA(cudaMalloc(&T.rows, sizeof(uint32_t) * (rows.size() + 1)));
-  GRE_CUDA(cudaMalloc(&T.chunk_row, sizeof(uint64_t) * (crow.size() + 1)));
-  GRE_CUDA(cudaMalloc(&T.chunk_begin, sizeof(uint64_t) * (cbeg.size() + 1)));
-  GRE_CUDA(cudaMalloc(&T.first, sizeof(uint64_t) * first.size()));
-  if (!rows.empty()) {
-    GRE_CUDA(cudaMemcpy(T.rows, rows.data(), sizeof(uint32_t) * rows.size(), cudaMemcpyHostToDevice));
-    GRE_CUDA(cudaMemcpy(T.chunk_row, crow.data(), sizeof(uint64_t) * crow.size(), cudaMemcpyHostToDevice));
-    GRE_CUDA(cudaMemcpy(T.chunk_begin, cbeg.data(), sizeof(uint64_t) * cbeg.size(), cudaMemcpyHostToDevice));
-  }
-  GRE_CUDA(cudaMemcpy(T.first, first.data(), sizeof(uint64_t) * first.size(), cudaMemcpyHostToDevice));
-  T.ready = true;
-  return GRE_SUCCESS;
-}
-
 // ---------------------------------------------------------------------------------------------
 // single source
 // ---------------------------------------------------------------------------------------------
@@ -582,7 +547,7 @@ int gre_bc(gre_graph g, const uint32_t* srcs, uint32_t nsrc, int batched, double
   std::vector<uint32_t> hs(nsrc);
   if (nsrc) GRE_CUDA(cudaMemcpy(hs.data(), srcs, sizeof(uint32_t) * nsrc, cudaMemcpyDefault));
   GRE_CHECK(map_ids(g, &hs, "gre_bc"));
-  GRE_CHECK(ensure_bc_chunks(g));
+  GRE_CHECK(ensure_chunk_table(g, g->bc_chunks, kBcChunk));
   double *dfinal, *dbc;
   GRE_CHECK(prepare_output(g, bc, n, WS_OUTBUF, &dfinal));
   GRE_CHECK(perm_out_begin(g, dfinal, 1, 8, (void**)&dbc));

@@ -454,6 +454,50 @@ int ensure_bins(gre_graph g, bool in) {
   return build_bins(g, B, off, col, sched);
 }
 
+// Chunks of `ch` arcs of the in-arc rows longer than that; built once per graph.
+int ensure_chunk_table(gre_graph g, ChunkTable& T, uint64_t ch) {
+  if (T.ready) return GRE_SUCCESS;
+  const uint64_t n = g->n;
+  std::vector<uint64_t> ho(n + 1);
+  GRE_CUDA(cudaMemcpy(ho.data(), g->roff, sizeof(uint64_t) * (n + 1), cudaMemcpyDeviceToHost));
+  std::vector<uint32_t> rows;
+  std::vector<uint64_t> crow, cbeg, first;
+  for (uint64_t v = 0; v < n; ++v) {
+    if (ho[v + 1] - ho[v] <= ch) continue;
+    first.push_back(crow.size());
+    for (uint64_t a = ho[v]; a < ho[v + 1]; a += ch) {
+      crow.push_back(rows.size());
+      cbeg.push_back(a);
+    }
+    rows.push_back((uint32_t)v);
+  }
+  first.push_back(crow.size());
+  free_chunk_table(T);  // what a failed build left
+  T.ch = ch;
+  T.nrows = rows.size();
+  T.nchunks = crow.size();
+  GRE_CUDA(cudaMalloc(&T.rows, sizeof(uint32_t) * (rows.size() + 1)));
+  GRE_CUDA(cudaMalloc(&T.chunk_row, sizeof(uint64_t) * (crow.size() + 1)));
+  GRE_CUDA(cudaMalloc(&T.chunk_begin, sizeof(uint64_t) * (cbeg.size() + 1)));
+  GRE_CUDA(cudaMalloc(&T.first, sizeof(uint64_t) * first.size()));
+  if (!rows.empty()) {
+    GRE_CUDA(cudaMemcpy(T.rows, rows.data(), sizeof(uint32_t) * rows.size(), cudaMemcpyHostToDevice));
+    GRE_CUDA(cudaMemcpy(T.chunk_row, crow.data(), sizeof(uint64_t) * crow.size(), cudaMemcpyHostToDevice));
+    GRE_CUDA(cudaMemcpy(T.chunk_begin, cbeg.data(), sizeof(uint64_t) * cbeg.size(), cudaMemcpyHostToDevice));
+  }
+  GRE_CUDA(cudaMemcpy(T.first, first.data(), sizeof(uint64_t) * first.size(), cudaMemcpyHostToDevice));
+  T.ready = true;
+  return GRE_SUCCESS;
+}
+
+void free_chunk_table(ChunkTable& T) {
+  cudaFree(T.rows);
+  cudaFree(T.chunk_row);
+  cudaFree(T.chunk_begin);
+  cudaFree(T.first);
+  T = ChunkTable();
+}
+
 }  // namespace gre
 
 extern "C" int gre_row_schedule(gre_graph g, int in, uint32_t* lane_arcs, uint64_t* cta_min, uint64_t* hub_chunk,

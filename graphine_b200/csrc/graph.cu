@@ -296,10 +296,8 @@ void destroy_graph(gre_graph g) {
   free_bins(g->bins_in);
   free_bins(g->bins_out);
   free_bins(g->bins_sssp);
-  cudaFree(g->bc_chunks.rows);
-  cudaFree(g->bc_chunks.chunk_row);
-  cudaFree(g->bc_chunks.chunk_begin);
-  cudaFree(g->bc_chunks.first);
+  free_chunk_table(g->bc_chunks);
+  free_chunk_table(g->ppr_chunks);
   cudaFree(g->bc_fpool);
   cudaFree(g->perm);
   cudaFree(g->iperm);
@@ -439,11 +437,8 @@ static void drop_derived(gre_graph g) {
   free_bins(g->bins_in);
   free_bins(g->bins_out);
   free_bins(g->bins_sssp);
-  cudaFree(g->bc_chunks.rows);
-  cudaFree(g->bc_chunks.chunk_row);
-  cudaFree(g->bc_chunks.chunk_begin);
-  cudaFree(g->bc_chunks.first);
-  g->bc_chunks = ChunkTable();
+  free_chunk_table(g->bc_chunks);
+  free_chunk_table(g->ppr_chunks);
 }
 
 // Relabel by decreasing degree: new row i = old row perm[i], neighbour ids mapped through

@@ -172,6 +172,7 @@ struct gre_graph_s {
   // arc a within its caller row (caller arc = caller_off[perm[row]] + arc_rank[a]).
   uint32_t* arc_rank = nullptr;
   gre::ChunkTable bc_chunks;       // in-arc rows longer than 512 arcs (betweenness)
+  gre::ChunkTable ppr_chunks;      // in-arc rows longer than 1024 arcs (batched personalised PageRank)
   uint64_t* bc_fpool = nullptr;    // per-level frontier words of the batched betweenness
   uint64_t bc_fpool_levels = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -342,6 +343,9 @@ int ensure_bins(gre_graph g, bool in);
 // Degree bins of the rows of `off` (g->n rows) under a fixed schedule (replacing what B held).
 int build_bins(gre_graph g, DegreeBins& B, const uint64_t* off, const uint32_t* col, const RowSchedule& sched);
 void free_bins(DegreeBins& B);
+// Chunks of `ch` arcs of the in-arc rows longer than that; built once per graph.
+int ensure_chunk_table(gre_graph g, ChunkTable& T, uint64_t ch);
+void free_chunk_table(ChunkTable& T);
 // CSC slot -> CSR arc map; built once per graph.
 int ensure_rarc(gre_graph g);
 // Undirected edge count with both endpoints in a reached set (Graph500 TEPS numerator).

@@ -15,7 +15,6 @@
 // HBM bytes per superstep (algorithmic): 8(n+1) offsets + 4m columns + 8m gathered contrib
 // + 4n outdeg + 16n (pr and contrib writes) = 8(n+1) + 12m + 20n.
 #include <algorithm>
-#include <memory>
 
 #include "gre_internal.cuh"
 #include "rows.cuh"
@@ -69,194 +68,274 @@ static int ws_array(gre_graph g, int slot, uint64_t count, T** p) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// personalised PageRank, batched: X[v][k] row-major, one warp per in-arc row, each lane owns
-// kCols/32 columns; rows longer than kPprChunk arcs are split into chunks whose partial
-// vectors are added in order.
+// personalised PageRank, batched: the vectors in slices of C = 64 (or 32) columns, X[v][C]
+// row-major, a warp per in-arc row, each lane C/32 columns; rows longer than kPprChunk arcs are
+// split into chunks whose partial vectors are added in order.
+//
+// A superstep gathers a row of X per arc, 8C bytes, from L2 where it is there.  128 columns a row
+// (1 KB) kept an eighth of RMAT-20's rows in L2 and two arcs in flight a warp: 2.85 ms a superstep, DRAM
+// at 43%, L2 at 46%, warps waiting for loads (ncu).  64 columns keep a quarter of the rows there (which
+// draw nine tenths of the arcs), one 16-byte load a lane and arc, eight arcs in flight; the columns' second
+// reading of the topology is 4 bytes an arc: 0.95 ms a slice and superstep, 17 TB/s of gathered rows,
+// L2 and L1 at 64% (RMAT-20, 128 vectors, 20 supersteps: 61.1 -> 41.5 ms; slices of 32 columns: 46.2).
+//
+// The columns are independent: a slice runs all its supersteps before the next.  The values
+// themselves are written by the last superstep only, in place of the next contributions.
 // ---------------------------------------------------------------------------------------------
-constexpr int kCols = 128;
 constexpr uint64_t kPprChunk = 1024;
+constexpr int kPprBatch = 8;           // short rows a warp takes together
+constexpr uint32_t kPprShort = 32;     // arcs of a short row at most
 
-__global__ void k_ppr_init(uint64_t n, uint32_t k, const uint32_t* __restrict__ seeds, const uint32_t* __restrict__ outdeg,
-                           double tele, double* __restrict__ x, double* __restrict__ c0, double* __restrict__ c1) {
-  // zero everything, then place the restart mass
-  const uint64_t total = n * kCols;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-    x[i] = 0.0;
-    c0[i] = 0.0;
-    c1[i] = 0.0;
+template <int C>
+struct PprVec;  // a lane's columns of a row: C/32 of them, side by side
+template <>
+struct PprVec<64> {
+  double a = 0.0, b = 0.0;
+  static __device__ __forceinline__ PprVec load(const double* row) {
+    const double2 x = __ldg((const double2*)row + lane_id());
+    PprVec r;
+    r.a = x.x;
+    r.b = x.y;
+    return r;
   }
-}
-
-__global__ void k_ppr_seed(uint32_t k, const uint32_t* __restrict__ seeds, const uint32_t* __restrict__ outdeg, double tele,
-                           double* __restrict__ x, double* __restrict__ c0, double* __restrict__ c1) {
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < k; j += gridDim.x * blockDim.x) {
-    const uint32_t s = seeds[j];
-    const uint32_t od = outdeg[s];
-    x[(uint64_t)s * kCols + j] = tele;
-    const double c = od ? tele / (double)od : 0.0;
-    c0[(uint64_t)s * kCols + j] = c;
-    c1[(uint64_t)s * kCols + j] = c;
+  __device__ __forceinline__ void add(const PprVec& o) {
+    a += o.a;
+    b += o.b;
   }
-}
+  __device__ __forceinline__ void store(double* row) const { ((double2*)row)[lane_id()] = make_double2(a, b); }
+};
+template <>
+struct PprVec<32> {
+  double a = 0.0;
+  static __device__ __forceinline__ PprVec load(const double* row) {
+    PprVec r;
+    r.a = __ldg(row + lane_id());
+    return r;
+  }
+  __device__ __forceinline__ void add(const PprVec& o) { a += o.a; }
+  __device__ __forceinline__ void store(double* row) const { row[lane_id()] = a; }
+};
 
-struct PprRow {
+struct PprStep {
   const uint64_t* __restrict__ roff;
   const uint32_t* __restrict__ rcol;
-  const double* __restrict__ contrib;
-  // adds contrib rows of arcs [a0, a1) into acc (each lane its 4 columns); two arcs per pass
-  // keep eight independent loads per lane in flight
-  __device__ __forceinline__ void accumulate(uint64_t a0, uint64_t a1, double acc[kCols / 32]) const {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint64_t a = a0;
-    for (; a + 1 < a1; a += 2) {
-      const uint32_t u0 = __ldg(rcol + a), u1 = __ldg(rcol + a + 1);
-      const double* r0 = contrib + (uint64_t)u0 * kCols + lane;
-      const double* r1 = contrib + (uint64_t)u1 * kCols + lane;
-      double x0[kCols / 32], x1[kCols / 32];
-#pragma unroll
-      for (int j = 0; j < kCols / 32; ++j) {
-        x0[j] = __ldg(r0 + 32 * j);
-        x1[j] = __ldg(r1 + 32 * j);
-      }
-#pragma unroll
-      for (int j = 0; j < kCols / 32; ++j) {
-        acc[j] += x0[j];
-        acc[j] += x1[j];
-      }
-    }
-    for (; a < a1; ++a) {
-      const uint32_t u = __ldg(rcol + a);
-      const double* row = contrib + (uint64_t)u * kCols + lane;
-#pragma unroll
-      for (int j = 0; j < kCols / 32; ++j) acc[j] += __ldg(row + 32 * j);
-    }
-  }
-};
-
-struct PprFinish {
-  double* __restrict__ x;
-  double* __restrict__ cnext;
   const uint32_t* __restrict__ outdeg;
-  const uint32_t* __restrict__ seeds;
-  uint32_t k;
+  const uint32_t* __restrict__ seeds;  // kk of them
+  const double* __restrict__ cur;      // contributions
+  double* __restrict__ next;           // the next ones; the values themselves in the last superstep
+  double* __restrict__ partial;        // chunk sums
+  const uint32_t* __restrict__ rows;   // the bins' rows, short bins first
+  uint32_t nrows, nshort;              // of which the first nshort have at most kPprShort arcs
+  ChunkTable chunks;
+  uint32_t kk;
+  bool last;
   double tele, d;
-  __device__ __forceinline__ void operator()(uint32_t v, const double acc[kCols / 32]) const {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t od = outdeg[v];
-#pragma unroll
-    for (int j = 0; j < kCols / 32; ++j) {
-      const uint32_t col = lane + 32 * j;
-      const double t = (col < k && seeds[col] == v) ? tele : 0.0;
-      const double val = t + d * acc[j];
-      x[(uint64_t)v * kCols + col] = val;
-      cnext[(uint64_t)v * kCols + col] = od ? val / (double)od : 0.0;
-    }
-  }
 };
 
-// rows of up to kPprChunk arcs, whatever their bin: one warp per row
-__global__ void __launch_bounds__(256) k_ppr_rows(const uint32_t* __restrict__ rows, uint64_t count, PprRow R, PprFinish F) {
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t i = warp; i < count; i += nwarps) {
-    const uint32_t v = rows[i];
-    double acc[kCols / 32] = {0.0, 0.0, 0.0, 0.0};
-    const uint64_t a0 = R.roff[v], a1 = R.roff[v + 1];
-    if (a1 - a0 > kPprChunk) continue;  // chunked (uniform: one row per warp)
-    R.accumulate(a0, a1, acc);
-    F(v, acc);
+// The place of the restart mass in a row: bit j of a lane's mask, its column j seeds vertex v.
+template <int C>
+__device__ __forceinline__ void ppr_finish(const PprStep& P, uint32_t v, uint32_t od, PprVec<C> acc, uint32_t seed0, uint32_t seed1) {
+  acc.a = (seed0 == v ? P.tele : 0.0) + P.d * acc.a;
+  if constexpr (C == 64) acc.b = (seed1 == v ? P.tele : 0.0) + P.d * acc.b;
+  if (!P.last) {
+    acc.a = od ? acc.a / (double)od : 0.0;
+    if constexpr (C == 64) acc.b = od ? acc.b / (double)od : 0.0;
   }
+  acc.store(P.next + (uint64_t)v * C);
 }
 
-// long rows: chunk c covers arcs [chunk_begin[c], +kPprChunk) of row chunk_row[c]
-__global__ void __launch_bounds__(256) k_ppr_chunks(const uint32_t* __restrict__ rows, const uint64_t* __restrict__ chunk_row,
-                                                     const uint64_t* __restrict__ chunk_begin, uint64_t nchunks, PprRow R,
-                                                     double* __restrict__ partial) {
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint64_t c = warp; c < nchunks; c += nwarps) {
-    const uint32_t v = rows[chunk_row[c]];
-    const uint64_t a0 = chunk_begin[c];
-    const uint64_t end = R.roff[v + 1];
-    const uint64_t a1 = a0 + kPprChunk < end ? a0 + kPprChunk : end;
-    double acc[kCols / 32] = {0.0, 0.0, 0.0, 0.0};
-    R.accumulate(a0, a1, acc);
+// acc += the rows of the columns that lanes 0 .. cnt-1 hold, in order; eight in flight
+template <int C>
+__device__ __forceinline__ void ppr_gather(const double* __restrict__ cur, uint32_t idx, uint32_t cnt, PprVec<C>& acc) {
+  uint32_t i = 0;
+  for (; i + 8 <= cnt; i += 8) {
+    PprVec<C> x[8];
 #pragma unroll
-    for (int j = 0; j < kCols / 32; ++j) partial[c * kCols + lane + 32 * j] = acc[j];
+    for (int j = 0; j < 8; ++j) x[j] = PprVec<C>::load(cur + (uint64_t)__shfl_sync(0xffffffffu, idx, i + j) * C);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc.add(x[j]);
   }
+  if (i + 4 <= cnt) {
+    PprVec<C> x[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = PprVec<C>::load(cur + (uint64_t)__shfl_sync(0xffffffffu, idx, i + j) * C);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc.add(x[j]);
+    i += 4;
+  }
+  if (i + 2 <= cnt) {
+    const PprVec<C> x = PprVec<C>::load(cur + (uint64_t)__shfl_sync(0xffffffffu, idx, i) * C);
+    const PprVec<C> y = PprVec<C>::load(cur + (uint64_t)__shfl_sync(0xffffffffu, idx, i + 1) * C);
+    acc.add(x);
+    acc.add(y);
+    i += 2;
+  }
+  if (i < cnt) acc.add(PprVec<C>::load(cur + (uint64_t)__shfl_sync(0xffffffffu, idx, i) * C));
 }
 
-__global__ void k_ppr_chunk_finish(const uint32_t* __restrict__ rows, uint64_t count, const uint64_t* __restrict__ first,
-                                   const double* __restrict__ partial, PprFinish F) {
+template <int C>
+__device__ __forceinline__ PprVec<C> ppr_sum(const PprStep& P, uint64_t a0, uint64_t a1) {
+  const uint32_t lane = lane_id();
+  PprVec<C> acc;
+  uint32_t idx = a0 + lane < a1 ? __ldg(P.rcol + a0 + lane) : 0u;
+  for (uint64_t b = a0; b < a1; b += 32) {
+    const uint32_t following = b + 32 + lane < a1 ? __ldg(P.rcol + b + 32 + lane) : 0u;
+    ppr_gather(P.cur, idx, a1 - b < 32 ? (uint32_t)(a1 - b) : 32u, acc);
+    idx = following;
+  }
+  return acc;
+}
+
+// One superstep but for the chunked rows' finish: first the chunks, then the rows from long to short
+// (the resident warps stride over them, each a share of every length).
+template <int C>
+__global__ void __launch_bounds__(256) k_ppr_step(const __grid_constant__ PprStep P) {
+  const uint32_t lane = lane_id();
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint64_t i = warp; i < count; i += nwarps) {
-    double acc[kCols / 32] = {0.0, 0.0, 0.0, 0.0};
-    for (uint64_t c = first[i]; c < first[i + 1]; ++c)
-#pragma unroll
-      for (int j = 0; j < kCols / 32; ++j) acc[j] += partial[c * kCols + lane + 32 * j];
-    F(rows[i], acc);
+  constexpr int V = C / 32;
+  const uint32_t seed0 = V * lane < P.kk ? P.seeds[V * lane] : 0xffffffffu;
+  const uint32_t seed1 = V == 2 && V * lane + 1 < P.kk ? P.seeds[V * lane + 1] : 0xffffffffu;
+  uint64_t i = warp;
+  for (; i < P.chunks.nchunks; i += nwarps) {
+    const uint64_t a0 = P.chunks.chunk_begin[i], end = P.roff[P.chunks.rows[P.chunks.chunk_row[i]] + 1];
+    ppr_sum<C>(P, a0, a0 + kPprChunk < end ? a0 + kPprChunk : end).store(P.partial + i * C);
   }
-}
-
-__global__ void k_ppr_transpose(uint64_t n, uint32_t k, const double* __restrict__ x, double* __restrict__ out) {
-  // out[j*n + v] = x[v*kCols + j]
-  const uint64_t total = (uint64_t)k * n;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t j = i / n, v = i % n;
-    out[i] = x[v * kCols + j];
+  i -= P.chunks.nchunks;
+  const uint64_t nlong = P.nrows - P.nshort;
+  for (; i < nlong; i += nwarps) {
+    const uint32_t v = P.rows[P.nrows - 1 - i];
+    const uint64_t a0 = P.roff[v], a1 = P.roff[v + 1];
+    const uint32_t od = P.outdeg[v];
+    if (a1 - a0 > kPprChunk) continue;  // chunked
+    ppr_finish<C>(P, v, od, ppr_sum<C>(P, a0, a1), seed0, seed1);
   }
-}
-
-struct PprChunks {
-  uint64_t nchunks = 0;
-  uint64_t* row = nullptr;    // chunk -> index into the long-row list
-  uint64_t* begin = nullptr;  // chunk -> first arc
-  uint64_t* first = nullptr;  // long row -> first chunk
-  uint64_t nrows = 0;
-  uint32_t* rows = nullptr;   // long rows (bins 6 and 7, contiguous in the bin list)
-};
-
-static int ppr_chunks(gre_graph g, PprChunks* pc) {
-  // candidates: rows of more than 64 arcs (bins 5..7, contiguous in the bin list); only those
-  // longer than kPprChunk are chunked, the others stay with the warp-per-row kernel
-  const DegreeBins& B = g->bins_in;
-  const uint64_t cand = B.count[5] + B.count[6] + B.count[7];
-  pc->nrows = 0;
-  pc->nchunks = 0;
-  if (!cand) return GRE_SUCCESS;
-  std::vector<uint32_t> rows(cand), lrows;
-  std::vector<uint64_t> ho(g->n + 1);
-  GRE_CUDA(cudaMemcpy(rows.data(), B.rows + B.start[5], sizeof(uint32_t) * cand, cudaMemcpyDeviceToHost));
-  GRE_CUDA(cudaMemcpy(ho.data(), g->roff, sizeof(uint64_t) * (g->n + 1), cudaMemcpyDeviceToHost));
-  std::vector<uint64_t> crow, cbeg, first;
-  for (uint64_t i = 0; i < cand; ++i) {
-    const uint32_t v = rows[i];
-    if (ho[v + 1] - ho[v] <= kPprChunk) continue;
-    first.push_back(crow.size());
-    for (uint64_t a = ho[v]; a < ho[v + 1]; a += kPprChunk) {
-      crow.push_back(lrows.size());
-      cbeg.push_back(a);
+  i -= nlong;
+  const uint64_t nbatches = ((uint64_t)P.nshort + kPprBatch - 1) / kPprBatch;
+  for (; i < nbatches; i += nwarps) {
+    // lane j < kPprBatch: row j of the batch; then the columns of all of them
+    uint64_t a0 = 0;
+    uint32_t v = 0, len = 0, od = 0;
+    const uint64_t at = i * kPprBatch + lane;
+    if (lane < kPprBatch && at < P.nshort) {
+      v = P.rows[P.nshort - 1 - at];
+      a0 = P.roff[v];
+      len = (uint32_t)(P.roff[v + 1] - a0);
+      od = P.outdeg[v];
     }
-    lrows.push_back(v);
+    uint32_t idx[kPprBatch];
+#pragma unroll
+    for (int j = 0; j < kPprBatch; ++j) {
+      const uint64_t b = __shfl_sync(0xffffffffu, a0, j);
+      idx[j] = lane < __shfl_sync(0xffffffffu, len, j) ? __ldg(P.rcol + b + lane) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < kPprBatch; ++j) {
+      const uint32_t n = __shfl_sync(0xffffffffu, len, j);
+      PprVec<C> acc;
+      ppr_gather(P.cur, idx[j], n, acc);
+      if (n) ppr_finish<C>(P, __shfl_sync(0xffffffffu, v, j), __shfl_sync(0xffffffffu, od, j), acc, seed0, seed1);
+    }
   }
-  first.push_back(crow.size());
-  pc->nrows = lrows.size();
-  pc->nchunks = crow.size();
-  if (!pc->nrows) return GRE_SUCCESS;
-  void* p;
-  GRE_CHECK(g->ws.get(WS_L, sizeof(uint64_t) * (crow.size() * 2 + first.size()) + sizeof(uint32_t) * lrows.size(), &p));
-  pc->row = (uint64_t*)p;
-  pc->begin = pc->row + crow.size();
-  pc->first = pc->begin + crow.size();
-  pc->rows = (uint32_t*)(pc->first + first.size());
-  GRE_CUDA(cudaMemcpyAsync(pc->row, crow.data(), sizeof(uint64_t) * crow.size(), cudaMemcpyHostToDevice, g->stream));
-  GRE_CUDA(cudaMemcpyAsync(pc->begin, cbeg.data(), sizeof(uint64_t) * cbeg.size(), cudaMemcpyHostToDevice, g->stream));
-  GRE_CUDA(cudaMemcpyAsync(pc->first, first.data(), sizeof(uint64_t) * first.size(), cudaMemcpyHostToDevice, g->stream));
-  GRE_CUDA(cudaMemcpyAsync(pc->rows, lrows.data(), sizeof(uint32_t) * lrows.size(), cudaMemcpyHostToDevice, g->stream));
-  GRE_CUDA(cudaStreamSynchronize(g->stream));
+}
+
+// Chunked rows: partial sums in chunk order, four loads in flight.
+template <int C>
+__global__ void __launch_bounds__(256) k_ppr_chunk_finish(const __grid_constant__ PprStep P) {
+  const uint32_t lane = lane_id();
+  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  constexpr int V = C / 32;
+  const uint32_t seed0 = V * lane < P.kk ? P.seeds[V * lane] : 0xffffffffu;
+  const uint32_t seed1 = V == 2 && V * lane + 1 < P.kk ? P.seeds[V * lane + 1] : 0xffffffffu;
+  for (uint64_t i = warp; i < P.chunks.nrows; i += nwarps) {
+    const uint32_t v = P.chunks.rows[i];
+    const uint32_t od = P.outdeg[v];
+    PprVec<C> acc;
+    uint64_t c = P.chunks.first[i];
+    const uint64_t end = P.chunks.first[i + 1];
+    for (; c + 4 <= end; c += 4) {
+      PprVec<C> x[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[j] = PprVec<C>::load(P.partial + (c + j) * C);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc.add(x[j]);
+    }
+    for (; c < end; ++c) acc.add(PprVec<C>::load(P.partial + c * C));
+    ppr_finish<C>(P, v, od, acc, seed0, seed1);
+  }
+}
+
+// The restart mass in both buffers of contributions (zeroed before).
+template <int C>
+__global__ void k_ppr_seed(uint32_t kk, const uint32_t* __restrict__ seeds, const uint32_t* __restrict__ outdeg, double tele,
+                           double* __restrict__ c0, double* __restrict__ c1) {
+  for (uint32_t j = threadIdx.x; j < kk; j += blockDim.x) {
+    const uint32_t s = seeds[j];
+    const uint32_t od = outdeg[s];
+    const double c = od ? tele / (double)od : 0.0;
+    c0[(uint64_t)s * C + j] = c;
+    c1[(uint64_t)s * C + j] = c;
+  }
+}
+
+// A seed whose row has no in-arcs (or all seeds, before any superstep) keeps its restart mass as its
+// value: no superstep wrote it.
+template <int C>
+__global__ void k_ppr_seed_values(uint32_t kk, const uint32_t* __restrict__ seeds, const uint64_t* __restrict__ roff, bool all,
+                                  double tele, double* __restrict__ x) {
+  for (uint32_t j = threadIdx.x; j < kk; j += blockDim.x) {
+    const uint32_t s = seeds[j];
+    if (all || roff[s + 1] == roff[s]) x[(uint64_t)s * C + j] = tele;
+  }
+}
+
+// out[j * n + u] = x[row of u][j] for the slice's kk vectors, u in the caller's order: 32 rows at a
+// time through shared memory, so that both sides move whole lines.
+template <int C>
+__global__ void __launch_bounds__(256) k_ppr_out(uint64_t n, uint32_t kk, const double* __restrict__ x,
+                                                 const uint32_t* __restrict__ iperm, double* __restrict__ out) {
+  __shared__ double tile[32][C + 1];
+  const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+  for (uint64_t u0 = blockIdx.x * 32ull; u0 < n; u0 += gridDim.x * 32ull) {
+    for (uint32_t r = w; r < 32; r += 8) {
+      if (u0 + r >= n) break;
+      const uint64_t v = iperm ? __ldg(iperm + u0 + r) : u0 + r;
+#pragma unroll
+      for (int j = 0; j < C / 32; ++j) tile[r][lane + 32 * j] = __ldg(x + v * C + lane + 32 * j);
+    }
+    __syncthreads();
+    if (u0 + lane < n)
+      for (uint32_t j = w; j < kk; j += 8) out[(uint64_t)j * n + u0 + lane] = tile[lane][j];
+    __syncthreads();
+  }
+}
+
+// One slice: kk <= C seeds (device), the results to out (kk rows of n in the caller's order).
+template <int C>
+static int ppr_slice(gre_graph g, PprStep P, uint32_t iters, double* c0, double* c1, double* out) {
+  const uint64_t n = g->n;
+  static int per_sm = 0;
+  if (!per_sm) {
+    int b = 0;
+    GRE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_ppr_step<C>, 256, 0));
+    per_sm = b > 0 ? b : 1;
+  }
+  GRE_CUDA(cudaMemsetAsync(c0, 0, sizeof(double) * n * C, g->stream));
+  GRE_CUDA(cudaMemsetAsync(c1, 0, sizeof(double) * n * C, g->stream));
+  k_ppr_seed<C><<<1, C, 0, g->stream>>>(P.kk, P.seeds, g->outdeg, P.tele, c0, c1);
+  const uint64_t warps = P.chunks.nchunks + (P.nrows - P.nshort) + (P.nshort + kPprBatch - 1) / kPprBatch;
+  for (uint32_t it = 0; it < iters; ++it) {
+    P.cur = c0;
+    P.next = c1;
+    P.last = it + 1 == iters;
+    k_ppr_step<C><<<grid_for(warps * 32, 256, per_sm), 256, 0, g->stream>>>(P);
+    if (P.chunks.nrows) k_ppr_chunk_finish<C><<<grid_for(P.chunks.nrows * 32, 256, 8), 256, 0, g->stream>>>(P);
+    std::swap(c0, c1);
+  }
+  k_ppr_seed_values<C><<<1, C, 0, g->stream>>>(P.kk, P.seeds, g->roff, iters == 0, P.tele, c0);
+  k_ppr_out<C><<<grid_for(n * 8, 256, 16), 256, 0, g->stream>>>(n, P.kk, c0, g->iperm, out);
+  GRE_LAUNCH_CHECK();
   return GRE_SUCCESS;
 }
 
@@ -526,12 +605,12 @@ int gre_ppr(gre_graph g, const uint32_t* seeds, uint32_t k, double d, uint32_t i
   GRE_CHECK(map_ids(g, &hs, "gre_ppr"));
   GRE_CHECK(ensure_bins(g, true));
   const double tele = 1.0 - d;
-  double *dfinal, *dout;
+  double* dfinal;
   GRE_CHECK(prepare_output(g, out, (uint64_t)k * n, WS_OUTBUF, &dfinal));
-  GRE_CHECK(perm_out_begin(g, dfinal, k, 8, (void**)&dout));
   RunTimer timer(g);
   if (!batched) {
-    double *c0, *c1, *partial;
+    double *dout, *c0, *c1, *partial;
+    GRE_CHECK(perm_out_begin(g, dfinal, k, 8, (void**)&dout));
     GRE_CHECK(ws_array(g, WS_A, n, &c0));
     GRE_CHECK(ws_array(g, WS_B, n, &c1));
     GRE_CHECK(ws_array(g, WS_C, g->bins_in.n_partials + 1, &partial));
@@ -546,60 +625,46 @@ int gre_ppr(gre_graph g, const uint32_t* seeds, uint32_t k, double d, uint32_t i
         std::swap(cur, nxt);
       }
     }
+    GRE_CHECK(perm_out_end(g, dout, dfinal, k, 8));
     if (st) st->algo_bytes = (uint64_t)k * iters * pr_bytes_per_iter(n, g->m);
   } else {
-    PprChunks pc;
-    GRE_CHECK(ppr_chunks(g, &pc));
-    double *x, *c0, *c1, *partial;
+    GRE_CHECK(ensure_chunk_table(g, g->ppr_chunks, kPprChunk));
+    double *c0, *c1, *partial;
     uint32_t* dseeds;
-    GRE_CHECK(ws_array(g, WS_A, n * kCols, &x));
-    GRE_CHECK(ws_array(g, WS_B, n * kCols, &c0));
-    GRE_CHECK(ws_array(g, WS_C, n * kCols, &c1));
-    GRE_CHECK(ws_array(g, WS_D, (pc.nchunks + 1) * kCols, &partial));
-    GRE_CHECK(ws_array(g, WS_E, kCols, &dseeds));
+    PprStep P{};
+    const int cols = k > 32 ? 64 : 32;
+    GRE_CHECK(ws_array(g, WS_A, n * cols, &c0));
+    GRE_CHECK(ws_array(g, WS_B, n * cols, &c1));
+    GRE_CHECK(ws_array(g, WS_D, (g->ppr_chunks.nchunks + 1) * cols, &partial));
+    GRE_CHECK(ws_array(g, WS_E, k, &dseeds));
+    GRE_CUDA(cudaMemcpyAsync(dseeds, hs.data(), sizeof(uint32_t) * k, cudaMemcpyHostToDevice, g->stream));
     const DegreeBins& B = g->bins_in;
-    uint64_t short_rows = 0;
-    for (int b = 0; b < DegreeBins::NB; ++b) short_rows += B.count[b];  // rows longer than kPprChunk are skipped
-    std::unique_ptr<Recorded> rec;
-    uint32_t rec_kk = 0;
-    for (uint32_t j0 = 0; j0 < k; j0 += kCols) {
-      const uint32_t kk = (k - j0) < (uint32_t)kCols ? (k - j0) : (uint32_t)kCols;
-      GRE_CUDA(cudaMemcpyAsync(dseeds, hs.data() + j0, sizeof(uint32_t) * kk, cudaMemcpyHostToDevice, g->stream));
-      k_ppr_init<<<grid_for(n * kCols, 256), 256, 0, g->stream>>>(n, kk, dseeds, g->outdeg, tele, x, c0, c1);
-      k_ppr_seed<<<1, 128, 0, g->stream>>>(kk, dseeds, g->outdeg, tele, x, c0, c1);
-      auto superstep = [&](double* a, double* b) -> int {
-        PprRow R{g->roff, g->rcol, a};
-        PprFinish F{x, b, g->outdeg, dseeds, kk, tele, d};
-        if (short_rows) k_ppr_rows<<<grid_for(short_rows * 32, 256, 8), 256, 0, g->stream>>>(B.rows, short_rows, R, F);
-        if (pc.nrows) {
-          k_ppr_chunks<<<grid_for(pc.nchunks * 32, 256, 8), 256, 0, g->stream>>>(pc.rows, pc.row, pc.begin, pc.nchunks, R, partial);
-          k_ppr_chunk_finish<<<grid_for(pc.nrows * 32, 256, 8), 256, 0, g->stream>>>(pc.rows, pc.nrows, pc.first, partial, F);
-        }
-        GRE_LAUNCH_CHECK();
-        return GRE_SUCCESS;
-      };
-      // two supersteps (the buffers swap back) recorded once per block width, then replayed
-      if (!rec || rec_kk != kk) {
-        rec.reset(new Recorded());
-        rec_kk = kk;
-        GRE_CHECK(rec->record(g->stream, [&]() {
-          int e = superstep(c0, c1);
-          if (!e) e = superstep(c1, c0);
-          return e;
-        }));
-      }
-      uint32_t it = 0;
-      for (; it + 2 <= iters; it += 2) GRE_CHECK(rec->replay(g->stream));
-      if (it < iters) GRE_CHECK(superstep(c0, c1));
-      k_ppr_transpose<<<grid_for((uint64_t)kk * n, 256), 256, 0, g->stream>>>(n, kk, x, dout + (uint64_t)j0 * n);
-      GRE_LAUNCH_CHECK();
+    P.roff = g->roff;
+    P.rcol = g->rcol;
+    P.outdeg = g->outdeg;
+    P.partial = partial;
+    P.rows = B.rows;
+    P.chunks = g->ppr_chunks;
+    P.tele = tele;
+    P.d = d;
+    for (int b = 0; b < DegreeBins::NB; ++b) {
+      P.nrows += (uint32_t)B.count[b];
+      if (b < 5 && ((uint64_t)B.sched.lane_arcs << b) <= kPprShort) P.nshort += (uint32_t)B.count[b];
+    }
+    for (uint32_t j0 = 0; j0 < k;) {
+      // 64 columns a slice; a rest of at most 32 in a slice of 32
+      const uint32_t width = k - j0 > 32 ? 64 : 32;
+      P.kk = std::min<uint32_t>(width, k - j0);
+      P.seeds = dseeds + j0;
+      double* o = dfinal + (uint64_t)j0 * n;
+      GRE_CHECK(width == 64 ? ppr_slice<64>(g, P, iters, c0, c1, o) : ppr_slice<32>(g, P, iters, c0, c1, o));
+      j0 += P.kk;
     }
     if (st) {
-      const uint64_t passes = (k + kCols - 1) / kCols;
-      st->algo_bytes = passes * iters * (8 * (n + 1) + 4 * g->m + (uint64_t)kCols * (8 * g->m + 24 * n));
+      const uint64_t passes = (k + 63) / 64;
+      st->algo_bytes = iters * (passes * (8 * (n + 1) + 4 * g->m) + (uint64_t)k * (8 * g->m + 16 * n));
     }
   }
-  GRE_CHECK(perm_out_end(g, dout, dfinal, k, 8));
   GRE_CHECK(finish_output(g, out, dfinal, (uint64_t)k * n));
   GRE_CHECK(timer.stop(st));
   if (st) {

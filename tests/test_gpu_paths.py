@@ -195,3 +195,25 @@ def test_sssp_shapes(monkeypatch, n, directed, delta, binned, wide):
     d, _ = G.sssp(g, srcs)
     for i, s in enumerate(srcs):
         np.testing.assert_array_equal(d[i * n:(i + 1) * n], sssp_ref(n, off, col, w, s))
+
+
+@pytest.mark.parametrize("iters", [0, 1, 2, 5])
+@pytest.mark.parametrize("k", [1, 31, 32, 33, 64, 65, 96, 97, 130])
+@pytest.mark.parametrize("reorder", [False, True])
+def test_ppr_slices(k, iters, reorder):
+    """Slices of 64 and 32 vectors, full and ragged, rows shorter and longer than a warp's width and
+    than a chunk; seeds twice, without in-arcs and without out-arcs."""
+    degrees = [0, 1, 7, 8, 9, 31, 32, 33, 40, 64, 65, 1023, 1024, 1025, 2100, 0, 3] * 3
+    n = 333
+    off, col = rows_graph(degrees, n, k)
+    g = G.Graph.from_csr(n, off, col)
+    if reorder:
+        g.reorder()
+    seeds = np.random.default_rng(k).integers(0, n, k).astype(np.uint32)
+    seeds[: min(3, k)] = [0, 332, 14][: min(3, k)]
+    base = np.zeros((n, k))
+    base[seeds, np.arange(k)] = 0.15
+    ref = pagerank_ref(n, off, col, iters, base).T
+    out, _ = G.ppr(g, seeds, 0.85, iters)
+    # sums of at most 2100 positive terms below 1, a division and a product a superstep
+    assert np.max(np.abs(out.reshape(k, n) - ref)) <= (iters + 1) * 2100 * 2.3e-16
