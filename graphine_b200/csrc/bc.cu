@@ -211,49 +211,9 @@ static int bc_single(gre_graph g, const std::vector<uint32_t>& hs, double* dbc, 
 // ---------------------------------------------------------------------------------------------
 // batched: 64 sources per word
 // ---------------------------------------------------------------------------------------------
-__global__ void k_bcm_seed(const uint32_t* __restrict__ srcs, uint32_t k, unsigned long long* __restrict__ seen,
-                           unsigned long long* __restrict__ f0, double* __restrict__ sigma) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  for (uint32_t j = 0; j < k; ++j) {
-    const uint32_t s = srcs[j];
-    seen[s] |= 1ull << j;
-    f0[s] |= 1ull << j;
-    sigma[(uint64_t)s * 64 + j] = 1.0;
-  }
-}
-
-// F_next[v] = (OR over in-neighbours u of F_d[u]) & ~seen[v]; early exit when all unseen found
-__global__ void __launch_bounds__(256) k_bcm_forward(uint64_t n, unsigned long long full, const uint64_t* __restrict__ roff,
-                                                     const uint32_t* __restrict__ rcol, const unsigned long long* __restrict__ fd,
-                                                     unsigned long long* __restrict__ fnext, unsigned long long* __restrict__ seen,
-                                                     unsigned long long* __restrict__ counters) {
-  unsigned long long found = 0, scanned = 0;
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
-    const unsigned long long s = seen[v];
-    const unsigned long long want = full & ~s;
-    unsigned long long nb = 0;
-    if (want) {
-      unsigned long long acc = 0;
-      const uint64_t a1 = roff[v + 1];
-      for (uint64_t a = roff[v]; a < a1; ++a) {
-        acc |= fd[__ldg(rcol + a)];
-        ++scanned;
-        if ((acc & want) == want) break;
-      }
-      nb = acc & want;
-      if (nb) seen[v] = s | nb;
-    }
-    fnext[v] = nb;
-    found += nb != 0;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    found += __shfl_xor_sync(0xffffffffu, found, o);
-    scanned += __shfl_xor_sync(0xffffffffu, scanned, o);
-  }
-  if ((threadIdx.x & 31u) == 0) {
-    if (found) atomicAdd(counters, found);
-    if (scanned) atomicAdd(counters + 1, scanned);
-  }
+// sigma of the sources, in the columns of theirs
+__global__ void k_bcm_seed(const uint32_t* __restrict__ srcs, uint32_t k, double* __restrict__ sigma) {
+  if (threadIdx.x < k) sigma[(uint64_t)srcs[threadIdx.x] * 64 + threadIdx.x] = 1.0;
 }
 
 // list of vertices with a non-zero frontier word
@@ -415,83 +375,30 @@ __global__ void k_bcm_accumulate(uint64_t n, const uint32_t* __restrict__ srcs, 
   }
 }
 
-static int fpool_levels(gre_graph g, uint64_t levels) {
-  if (g->bc_fpool_levels >= levels) return GRE_SUCCESS;
-  uint64_t want = std::max<uint64_t>(levels, std::max<uint64_t>(32, 2 * g->bc_fpool_levels));
-  uint64_t* p = nullptr;
-  GRE_CUDA(cudaMalloc(&p, sizeof(uint64_t) * g->n * want));
-  if (g->bc_fpool) {
-    GRE_CUDA(cudaMemcpyAsync(p, g->bc_fpool, sizeof(uint64_t) * g->n * g->bc_fpool_levels, cudaMemcpyDeviceToDevice, g->stream));
-    GRE_CUDA(cudaStreamSynchronize(g->stream));
-    cudaFree(g->bc_fpool);
-  }
-  g->bc_fpool = p;
-  g->bc_fpool_levels = want;
-  return GRE_SUCCESS;
-}
-
 static int bc_batched(gre_graph g, const std::vector<uint32_t>& hs, double* dbc, gre_stats* st) {
   const uint64_t n = g->n;
   const ChunkTable& T = g->bc_chunks;
   double *sigma, *dep, *partial;
   uint32_t *list, *srcs;
-  unsigned long long *seen, *cnt, *acc;
+  unsigned long long* cnt;
+  MsBfs word;
   GRE_CHECK(ws_array(g, WS_BC1, n * 64, &sigma));
   GRE_CHECK(ws_array(g, WS_BC2, n * 64, &dep));
   GRE_CHECK(ws_array(g, WS_BC3, n, &list));
-  GRE_CHECK(ws_array(g, WS_BC4, n, &seen));
   GRE_CHECK(ws_array(g, WS_BC5, (T.nchunks + 1) * 64, &partial));
   GRE_CHECK(ws_array(g, WS_BC6, 8, &cnt));
-  GRE_CHECK(ensure_bins(g, true));
-  GRE_CHECK(ws_array(g, WS_BC0, n, &acc));
-  GRE_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long) * n, g->stream));
   GRE_CHECK(ws_array(g, WS_BC7, 64, &srcs));
-  GRE_CHECK(fpool_levels(g, 32));
+  GRE_CHECK(word.prepare(g, true));
   uint64_t arcs = 0, bytes = 0;
   const int sms = num_sms();
   for (size_t j0 = 0; j0 < hs.size(); j0 += 64) {
     const uint32_t k = (uint32_t)std::min<size_t>(64, hs.size() - j0);
-    const unsigned long long full = k == 64 ? ~0ull : ((1ull << k) - 1ull);
     GRE_CUDA(cudaMemcpyAsync(srcs, hs.data() + j0, sizeof(uint32_t) * k, cudaMemcpyHostToDevice, g->stream));
     GRE_CUDA(cudaMemsetAsync(sigma, 0, sizeof(double) * n * 64, g->stream));
     GRE_CUDA(cudaMemsetAsync(dep, 0, sizeof(double) * n * 64, g->stream));
-    GRE_CUDA(cudaMemsetAsync(seen, 0, sizeof(unsigned long long) * n, g->stream));
-    GRE_CUDA(cudaMemsetAsync(g->bc_fpool, 0, sizeof(unsigned long long) * n, g->stream));
-    k_bcm_seed<<<1, 32, 0, g->stream>>>(srcs, k, seen, (unsigned long long*)g->bc_fpool, sigma);
-    // forward: frontier words of every level
-    uint64_t nl = 1;  // levels stored: F_0 .. F_{nl-1}
-    unsigned long long live = full;  // sources whose frontier is not empty
-    while (true) {
-      GRE_CHECK(fpool_levels(g, nl + 1));
-      unsigned long long* fd = (unsigned long long*)g->bc_fpool + (nl - 1) * n;
-      unsigned long long* fn = (unsigned long long*)g->bc_fpool + nl * n;
-      // push from a sparse frontier, pull otherwise (same frontier words either way)
-      GRE_CUDA(cudaMemsetAsync(cnt, 0, 64, g->stream));
-      ms::k_frontier_list<<<grid_for(n, 256, 8), 256, 0, g->stream>>>(n, fd, g->off, list, (unsigned int*)(cnt + 2), cnt + 3);
-      unsigned long long h[6];
-      GRE_CUDA(cudaMemcpyAsync(h, cnt, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, g->stream));
-      GRE_CUDA(cudaStreamSynchronize(g->stream));
-      const bool push = h[3] * 14 < g->m;
-      if (push)
-        ms::k_push<<<grid_for((h[2] & 0xffffffffull) * 32, 256, 8), 256, 0, g->stream>>>(list, (unsigned int*)(cnt + 2), g->off,
-                                                                                          g->col, fd, seen, acc);
-      else
-        GRE_CHECK(ms::pull(g->bins_in, live, g->roff, g->rcol, fd, seen, acc, cnt + 4, g->stream));
-      ms::k_commit<<<grid_for(n, 256, 8), 256, 0, g->stream>>>(n, acc, seen, fn, nullptr, 0, cnt, cnt + 5);
-      GRE_LAUNCH_CHECK();
-      GRE_CUDA(cudaMemcpyAsync(h, cnt, sizeof h, cudaMemcpyDeviceToHost, g->stream));
-      GRE_CUDA(cudaStreamSynchronize(g->stream));
-      if (push) {
-        arcs += h[3];
-        bytes += 16 * (h[2] & 0xffffffffull) + 12 * h[3] + 32 * n;
-      } else {
-        arcs += h[4];
-        bytes += 24 * n + 12 * h[4];
-      }
-      if (h[0] == 0) break;
-      live = h[5];
-      ++nl;
-    }
+    GRE_CHECK(word.run(srcs, k, false));
+    const uint64_t nl = word.levels + 1;  // F_0 .. F_{nl-1}
+    k_bcm_seed<<<1, 64, 0, g->stream>>>(srcs, k, sigma);
     unsigned long long* F = (unsigned long long*)g->bc_fpool;
     auto level_pass = [&](bool fwd, uint64_t d) -> int {
       BcM B{g->roff, g->rcol, fwd ? F + (d - 1) * n : F + (d + 1) * n, F + d * n, sigma, dep};
@@ -527,8 +434,8 @@ static int bc_batched(gre_graph g, const std::vector<uint32_t>& hs, double* dbc,
     if (st) st->supersteps += (uint32_t)(2 * nl);
   }
   if (st) {
-    st->arcs_traversed += arcs;
-    st->algo_bytes += bytes;
+    st->arcs_traversed += arcs + word.scanned;
+    st->algo_bytes += bytes + word.bytes;
   }
   return GRE_SUCCESS;
 }

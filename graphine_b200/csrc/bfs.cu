@@ -16,9 +16,7 @@
 //    thread that scans its in-arcs for a parent in the frontier bitmap and stops at the first; a
 //    warp covers 32 consecutive vertices, so the next-frontier word is one __ballot_sync and needs
 //    no atomics.
-//  * gre_msbfs: 64 sources per uint64 word (multi-source BFS, Then et al. 2014): seen/frontier
-//    words per vertex; a level is one pull over in-arcs OR-ing neighbour frontier words, so the
-//    topology is read once per level for all 64 sources.
+//  * gre_msbfs: 64 sources per uint64 word, the level loop in msbfs.cu.
 //
 // Byte model, top-down level: 16 F (queue + offsets) + 8 A (column + visited probe) + 8 N;
 // bottom-up level: 16 U (offsets + level of unvisited) + 4.125 A (column + frontier bit) + 4 N
@@ -33,14 +31,6 @@
 #include "msbfs.cuh"
 
 namespace gre {
-
-// persist.cu
-bool msbfs_persistent_available(uint64_t n);
-size_t msbfs_ctl_bytes();
-int msbfs_word_persistent(gre_graph g, unsigned long long full, unsigned long long* seen, unsigned long long* fa,
-                          unsigned long long* fb, unsigned long long* acc, uint32_t* list0, uint32_t* list1, int32_t* levels,
-                          void* ctl_mem, unsigned long long* found_per_level, uint32_t* levels_out, uint64_t* scanned,
-                          uint64_t* bytes, std::vector<unsigned long long>* found);
 
 template <class T>
 static int ws_array(gre_graph g, int slot, uint64_t count, T** p) {
@@ -211,93 +201,6 @@ __global__ void k_bits_to_queue(uint64_t n, const uint32_t* __restrict__ bits, u
   }
 }
 
-// Undirected edges with a reached endpoint: sum over reached v of outdeg(v) / 2 (symmetric).
-// sum of the degrees of reached vertices over `rows` level arrays of n entries each
-__global__ void k_reached_degree(uint64_t n, uint64_t rows, const int32_t* __restrict__ level, const uint32_t* __restrict__ deg,
-                                 unsigned long long* __restrict__ out) {
-  unsigned long long s = 0;
-  const uint64_t total = n * rows;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x)
-    if (level[i] >= 0) s += deg[i % n];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31u) == 0 && s) atomicAdd(out, s);
-}
-
-int count_reached_edges(gre_graph g, const int32_t* level, uint64_t* edges, uint64_t rows) {
-  unsigned long long* c;
-  GRE_CHECK(ws_array(g, WS_COUNTERS, 4, &c));
-  GRE_CUDA(cudaMemsetAsync(c, 0, 8, g->stream));
-  k_reached_degree<<<grid_for(g->n * rows, 256), 256, 0, g->stream>>>(g->n, rows, level, g->outdeg, c);
-  unsigned long long h = 0;
-  GRE_CUDA(cudaMemcpyAsync(&h, c, 8, cudaMemcpyDeviceToHost, g->stream));
-  GRE_CUDA(cudaStreamSynchronize(g->stream));
-  *edges = g->symmetric() ? h / 2 : h;
-  return GRE_SUCCESS;
-}
-
-// ---------------------------------------------------------------------------------------------
-// multi-source BFS, 64 sources per word
-// ---------------------------------------------------------------------------------------------
-__global__ void k_ms_seed(const uint32_t* __restrict__ srcs, uint32_t k, uint64_t n, unsigned long long* __restrict__ seen,
-                          unsigned long long* __restrict__ front, int32_t* __restrict__ levels) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  for (uint32_t j = 0; j < k; ++j) {
-    const uint32_t s = srcs[j];
-    seen[s] |= 1ull << j;
-    front[s] |= 1ull << j;
-    levels[(uint64_t)j * n + s] = 0;
-  }
-}
-
-// One level: for every vertex with unseen sources, OR the frontier words of its in-neighbours.
-// Thread per vertex; stops early once every unseen source has been found.
-__global__ void __launch_bounds__(256) k_ms_pull(uint64_t n, uint32_t k, unsigned long long full, const uint64_t* __restrict__ roff,
-                                                 const uint32_t* __restrict__ rcol, const unsigned long long* __restrict__ front,
-                                                 unsigned long long* __restrict__ next, unsigned long long* __restrict__ seen,
-                                                 int32_t* __restrict__ levels, int32_t next_level,
-                                                 unsigned long long* __restrict__ counters) {
-  unsigned long long found = 0, scanned = 0;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < n; base += stride) {
-    const uint64_t v = base + (threadIdx.x & 31u);
-    unsigned long long nb = 0;
-    if (v < n) {
-      const unsigned long long s = seen[v];
-      const unsigned long long want = full & ~s;
-      if (want) {
-        unsigned long long acc = 0;
-        const uint64_t a1 = roff[v + 1];
-        for (uint64_t a = roff[v]; a < a1; ++a) {
-          acc |= front[__ldg(rcol + a)];
-          ++scanned;
-          if ((acc & want) == want) break;
-        }
-        nb = acc & want;
-      }
-      next[v] = nb;
-      if (nb) seen[v] = s | nb;
-    }
-    // levels: all lanes walk the union of their new bits so the writes of one bit coalesce
-    unsigned int lo = __reduce_or_sync(0xffffffffu, (unsigned int)(nb & 0xffffffffull));
-    unsigned int hi = __reduce_or_sync(0xffffffffu, (unsigned int)(nb >> 32));
-    unsigned long long any = ((unsigned long long)hi << 32) | lo;
-    while (any) {
-      const int j = __ffsll(any) - 1;
-      any &= any - 1;
-      if ((nb >> j) & 1ull) levels[(uint64_t)j * n + v] = next_level;
-    }
-    found += __popcll(nb);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    found += __shfl_xor_sync(0xffffffffu, found, o);
-    scanned += __shfl_xor_sync(0xffffffffu, scanned, o);
-  }
-  if ((threadIdx.x & 31u) == 0) {
-    if (found) atomicAdd(counters, found);
-    if (scanned) atomicAdd(counters + 1, scanned);
-  }
-}
-
 }  // namespace gre
 
 using namespace gre;
@@ -361,97 +264,37 @@ int gre_msbfs(gre_graph g, const uint32_t* srcs, uint32_t nsrc, int32_t* levels,
   std::vector<uint32_t> hs(nsrc);
   if (nsrc) GRE_CUDA(cudaMemcpy(hs.data(), srcs, sizeof(uint32_t) * nsrc, cudaMemcpyDefault));
   GRE_CHECK(map_ids(g, &hs, "gre_msbfs"));
-  int32_t *dfinal, *dl;
-  unsigned long long *seen, *fa, *fb, *cnt;
+  int32_t* dl;
   uint32_t* dsrc;
-  GRE_CHECK(prepare_output(g, levels, (uint64_t)nsrc * n, WS_OUTBUF, &dfinal));
-  GRE_CHECK(perm_out_begin(g, dfinal, nsrc, 4, (void**)&dl));
-  GRE_CHECK(ws_array(g, WS_A, n, &seen));
-  GRE_CHECK(ws_array(g, WS_B, n, &fa));
-  GRE_CHECK(ws_array(g, WS_C, n, &fb));
-  unsigned long long* acc;
-  uint32_t *flist, *flist2 = nullptr;
-  unsigned char* ctl = nullptr;
-  GRE_CHECK(ws_array(g, WS_D, 64, &dsrc));
-  GRE_CHECK(ws_array(g, WS_E, n, &acc));
-  GRE_CHECK(ws_array(g, WS_F, n, &flist));
-  GRE_CHECK(ws_array(g, WS_COUNTERS, 8, &cnt));
-  GRE_CHECK(ensure_bins(g, true));
-  const bool persist = msbfs_persistent_available(n);
-  if (persist) {  // the level loop as one cooperative launch per word (persist.cu)
-    GRE_CHECK(ws_array(g, WS_G, n, &flist2));
-    GRE_CHECK(ws_array(g, WS_H, msbfs_ctl_bytes(), &ctl));
-  }
+  unsigned long long* reached;
+  GRE_CHECK(prepare_output(g, levels, (uint64_t)nsrc * n, WS_OUTBUF, &dl));
+  GRE_CHECK(ws_array(g, WS_I, nsrc, &dsrc));
+  GRE_CHECK(ws_array(g, WS_COUNTERS, 8, &reached));
   RunTimer timer(g);
-  GRE_CUDA(cudaMemsetAsync(dl, 0xff, sizeof(int32_t) * nsrc * n, g->stream));
-  GRE_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long) * n, g->stream));
-  uint64_t scanned = 0, bytes = 0;
   uint32_t max_levels = 0;
-  for (uint32_t j0 = 0; j0 < nsrc; j0 += 64) {
-    const uint32_t k = std::min<uint32_t>(64, nsrc - j0);
-    const unsigned long long full = k == 64 ? ~0ull : ((1ull << k) - 1ull);
-    GRE_CUDA(cudaMemcpyAsync(dsrc, hs.data() + j0, sizeof(uint32_t) * k, cudaMemcpyHostToDevice, g->stream));
-    GRE_CUDA(cudaMemsetAsync(seen, 0, sizeof(unsigned long long) * n, g->stream));
-    GRE_CUDA(cudaMemsetAsync(fa, 0, sizeof(unsigned long long) * n, g->stream));
-    int32_t* lv = dl + (uint64_t)j0 * n;
-    k_ms_seed<<<1, 32, 0, g->stream>>>(dsrc, k, n, seen, fa, lv);
-    if (persist) {
-      uint32_t nl = 0;
-      std::vector<unsigned long long> found;
-      GRE_CHECK(msbfs_word_persistent(g, full, seen, fa, fb, acc, flist, flist2, lv, ctl,
-                                      (unsigned long long*)(ctl + msbfs_ctl_bytes()) - GRE_MAX_RECORDED_SUPERSTEPS, &nl,
-                                      &scanned, &bytes, nsrc <= 64 ? &found : nullptr));
-      for (unsigned long long f : found) stats_record(st, f);
-      max_levels = std::max<uint32_t>(max_levels, nl);
-      continue;
+  MsBfs word;
+  unsigned long long arcs = 0;
+  if (nsrc) {
+    GRE_CHECK(word.prepare(g, false));
+    GRE_CUDA(cudaMemsetAsync(reached, 0, sizeof *reached, g->stream));
+    GRE_CUDA(cudaMemcpyAsync(dsrc, hs.data(), sizeof(uint32_t) * nsrc, cudaMemcpyHostToDevice, g->stream));
+    for (uint32_t j0 = 0; j0 < nsrc; j0 += 64) {
+      const uint32_t k = std::min<uint32_t>(64, nsrc - j0);
+      GRE_CHECK(word.run(dsrc + j0, k, st && nsrc <= 64));
+      GRE_CHECK(word.write_levels(k, dl + (uint64_t)j0 * n, reached));
+      max_levels = std::max(max_levels, word.levels);
     }
-    unsigned long long* front = fa;
-    unsigned long long* next = fb;
-    unsigned long long live = full;  // sources whose frontier is not empty
-    for (int32_t d = 0;; ++d) {
-      // direction: push when the frontier's arcs are few (Beamer's rule against all arcs)
-      GRE_CUDA(cudaMemsetAsync(cnt, 0, 64, g->stream));
-      ms::k_frontier_list<<<grid_for(n, 256, 8), 256, 0, g->stream>>>(n, front, g->off, flist, (unsigned int*)(cnt + 2), cnt + 3);
-      unsigned long long h[6];
-      GRE_CUDA(cudaMemcpyAsync(h, cnt, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, g->stream));
-      GRE_CUDA(cudaStreamSynchronize(g->stream));
-      const bool push = h[3] * 14 < g->m;
-      if (push)
-        ms::k_push<<<grid_for((h[2] & 0xffffffffull) * 32, 256, 8), 256, 0, g->stream>>>(flist, (unsigned int*)(cnt + 2), g->off,
-                                                                                          g->col, front, seen, acc);
-      else
-        GRE_CHECK(ms::pull(g->bins_in, live, g->roff, g->rcol, front, seen, acc, cnt + 4, g->stream));
-      ms::k_commit<<<grid_for(n, 256, 8), 256, 0, g->stream>>>(n, acc, seen, next, lv, d + 1, cnt, cnt + 5);
-      GRE_LAUNCH_CHECK();
-      GRE_CUDA(cudaMemcpyAsync(h, cnt, sizeof h, cudaMemcpyDeviceToHost, g->stream));
-      GRE_CUDA(cudaStreamSynchronize(g->stream));
-      const unsigned long long found_bits = h[1];
-      live = h[5];
-      if (push) {
-        scanned += h[3];
-        bytes += 16 * (h[2] & 0xffffffffull) + 12 * h[3] + 32 * n;
-      } else {
-        scanned += h[4];
-        bytes += 24 * n + 12 * h[4];
-      }
-      std::swap(front, next);
-      if (nsrc <= 64) stats_record(st, found_bits);
-      if (found_bits == 0) {
-        max_levels = std::max<uint32_t>(max_levels, (uint32_t)d);
-        break;
-      }
-    }
+    GRE_CUDA(cudaMemcpyAsync(&arcs, reached, sizeof arcs, cudaMemcpyDeviceToHost, g->stream));
+    GRE_CUDA(cudaStreamSynchronize(g->stream));
   }
-  uint64_t edges = 0;
-  GRE_CHECK(count_reached_edges(g, dl, &edges, nsrc));  // all sources in one pass
-  GRE_CHECK(perm_out_end(g, dl, dfinal, nsrc, 4));
-  GRE_CHECK(finish_output(g, levels, dfinal, (uint64_t)nsrc * n));
+  GRE_CHECK(finish_output(g, levels, dl, (uint64_t)nsrc * n));
   GRE_CHECK(timer.stop(st));
   if (st) {
+    for (unsigned long long f : word.found) stats_record(st, f);
     st->supersteps = max_levels;
-    st->arcs_traversed = scanned;
-    st->traversed_edges = edges;
-    st->algo_bytes = bytes;
+    st->arcs_traversed = word.scanned;
+    st->traversed_edges = g->symmetric() ? arcs / 2 : arcs;
+    st->algo_bytes = word.bytes;
   }
   return GRE_SUCCESS;
 }

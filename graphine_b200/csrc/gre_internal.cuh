@@ -348,8 +348,6 @@ int ensure_chunk_table(gre_graph g, ChunkTable& T, uint64_t ch);
 void free_chunk_table(ChunkTable& T);
 // CSC slot -> CSR arc map; built once per graph.
 int ensure_rarc(gre_graph g);
-// Undirected edge count with both endpoints in a reached set (Graph500 TEPS numerator).
-int count_reached_edges(gre_graph g, const int32_t* level, uint64_t* edges, uint64_t rows = 1);
 // SSSP bucket width: 3/8 of the mean uint32 weight (GRE_SSSP_DELTA overrides; 0 = no buckets).
 int sssp_delta(gre_graph g, uint32_t* delta);
 // Heads a partitioned relaxation owns itself (sssp.cu offer forms): heads in [lo, lo + len) are

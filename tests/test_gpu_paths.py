@@ -217,3 +217,99 @@ def test_ppr_slices(k, iters, reorder):
     out, _ = G.ppr(g, seeds, 0.85, iters)
     # sums of at most 2100 positive terms below 1, a division and a product a superstep
     assert np.max(np.abs(out.reshape(k, n) - ref)) <= (iters + 1) * 2100 * 2.3e-16
+
+
+def bc_ref(n, off, col, srcs):
+    """Brandes in float64 with the framework's directions: levels over the out-arcs, path counts and
+    dependencies both pulled over the in-arcs (as the reference's plugins do)."""
+    u = np.repeat(np.arange(n), np.diff(off.astype(np.int64)))
+    bc = np.zeros(n)
+    for s in srcs:
+        lev = bfs_ref(n, off, col, [s])
+        sigma, dep = np.zeros(n), np.zeros(n)
+        sigma[s] = 1.0
+        top = lev.max()
+        for d in range(1, top + 1):
+            on = (lev[u] == d - 1) & (lev[col] == d)
+            sigma += np.bincount(col[on], weights=sigma[u[on]], minlength=n)
+        for d in range(top - 1, -1, -1):
+            on = (lev[u] == d + 1) & (lev[col] == d)
+            dep += np.bincount(col[on], weights=(1 + dep[u[on]]) / sigma[u[on]], minlength=n) * np.where(lev == d, sigma, 0)
+        dep[s] = 0
+        bc += dep
+    return bc
+
+
+def deep_graph(path, hub, extra, directed, seed):
+    """A path that ends in a vertex with `hub` arcs to (and, some of them, from) leaves with random arcs
+    between them, then a second path; `extra` vertices without arcs; in any id order.  Returns the
+    vertices in that sequence too."""
+    rng = np.random.default_rng(seed)
+    n = path + 1 + hub + path + extra
+    ids = rng.permutation(n)
+    leaves = np.arange(path + 1, path + 1 + hub)
+    u = [np.arange(path), np.full(hub, path), rng.choice(leaves, hub // 2, False), rng.choice(leaves, 3 * hub), np.arange(path + hub, 2 * path + hub)]
+    v = [np.arange(1, path + 1), leaves, np.full(hub // 2, path), rng.choice(leaves, 3 * hub), np.arange(path + hub + 1, 2 * path + hub + 1)]
+    u, v = ids[np.concatenate(u)], ids[np.concatenate(v)]
+    if not directed:
+        u, v = np.concatenate([u, v]), np.concatenate([v, u])
+    keys = np.unique(u.astype(np.int64) * n + v)
+    keys = keys[keys // n != keys % n]
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(keys // n, minlength=n))
+    return n, off, (keys % n).astype(np.uint32), ids
+
+
+# (path, leaves, vertices without arcs): around the head and the tail pieces of a long row, levels
+# within one group of bit planes, two and three, and within and beyond the first pool of levels
+DEEP = [(1, 3, 0), (3, 512, 1), (14, 513, 2), (15, 1025, 0), (40, 2500, 7), (150, 700, 300), (2100, 90, 0)]
+
+
+def word_sources(n, ids, k, seed):
+    srcs = np.random.default_rng(seed).integers(0, n, k).astype(np.uint32)
+    first = [ids[0], ids[n // 2], ids[0]]  # the first path's end, one of the leaves; one twice
+    srcs[: min(3, k)] = first[: min(3, k)]
+    return srcs
+
+
+@pytest.mark.parametrize("directed,reorder", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("k", [1, 2, 63, 64, 65])
+@pytest.mark.parametrize("shape", DEEP)
+def test_word_bfs_shapes(shape, directed, reorder, k):
+    """The 64-source level loop: more levels than the first planes hold, rows that go on as tails,
+    sources without in-arcs, without out-arcs and twice."""
+    n, off, col, ids = deep_graph(*shape, directed, k)
+    g = G.Graph.from_csr(n, off, col, symmetric=not directed)
+    if reorder:
+        g.reorder()
+    srcs = word_sources(n, ids, k, n + k)
+    lv, st = G.msbfs(g, srcs)
+    lv = lv.reshape(k, n)
+    deg = np.diff(off.astype(np.int64))
+    arcs = sum(deg[row >= 0].sum() for row in lv)
+    check = range(k) if shape[0] < 100 else (0, k // 2, k - 1)
+    for i in check:
+        np.testing.assert_array_equal(lv[i], bfs_ref(n, off, col, [int(srcs[i])]))
+    assert st.traversed_edges == (arcs if directed else arcs // 2)
+    assert st.supersteps == lv.max()
+
+
+@pytest.mark.parametrize("directed,reorder", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("k", [1, 3, 65])
+@pytest.mark.parametrize("shape", DEEP)
+def test_batched_betweenness_shapes(shape, directed, reorder, k):
+    """Batched betweenness where the levels outgrow the pool, rows are longer and shorter than a chunk and
+    sources coincide: equal to one source at a time, and to Brandes in float64."""
+    n, off, col, ids = deep_graph(*shape, directed, k)
+    g = G.Graph.from_csr(n, off, col, symmetric=not directed)
+    if reorder:
+        g.reorder()
+    srcs = word_sources(n, ids, k, n + k)
+    got, _ = G.bc(g, srcs, batched=True)
+    np.testing.assert_array_equal(got, G.bc(g, srcs, batched=True)[0])
+    if shape[0] < 100 or k == 1:
+        np.testing.assert_array_equal(got, G.bc(g, srcs, batched=False)[0])
+    if k <= 3 and shape[0] < 1000:
+        # positive terms only, so that every sum, product and division costs at most half an ulp of what it
+        # adds to; no more than n sums and two roundings a level follow one another, on either side
+        np.testing.assert_allclose(got, bc_ref(n, off, col, srcs), rtol=2 * 3 * n * 1.2e-16, atol=0)
