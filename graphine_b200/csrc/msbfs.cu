@@ -48,6 +48,7 @@ struct MsSlot {  // the frontier of one level
 struct MsCtl {
   GridBar bar;
   MsSlot slot[3];  // level d: slot d % 3; the next one is filled, the one after cleared
+  u64 frontiers;     // vertices of all levels
   u64 push_levels, push_list, push_arcs, pull_levels, pull_scanned;
   unsigned int levels, d, queued, done;
 };
@@ -377,6 +378,7 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_msbfs(const __grid_constant__
     const bool push = st.mf * 14 < R.m;
     if (first && !resumed) {
       c->pull_scanned += st.scanned;
+      c->frontiers += st.nf;
       if (d > 0 && d - 1 < R.nrec) R.rec[d - 1] = st.bits;
       MsSlot* sz = &c->slot[(d + 2) % 3];  // last read a level ago
       sz->nf = sz->bits = sz->mf = sz->scanned = sz->live = 0;
@@ -592,6 +594,7 @@ int MsBfs::run(const uint32_t* dsrcs, uint32_t k, bool record) {
     GRE_CUDA(cudaMemsetAsync(&ctl->bar, 0, sizeof(GridBar), g->stream));
   } while (true);
   levels = h.levels;
+  frontier_vertices = h.frontiers;
   scanned += h.push_arcs + h.pull_scanned;
   bytes += 16 * h.push_list + 12 * h.push_arcs + 32 * n * h.push_levels + 24 * n * h.pull_levels + 12 * h.pull_scanned;
   if (record) {

@@ -14,6 +14,7 @@ struct MsBfs {
   gre_graph g = nullptr;
   unsigned long long* seen = nullptr;  // n words
   uint32_t levels = 0;                 // the deepest level with a vertex (last word)
+  uint64_t frontier_vertices = 0;      // of all levels (last word)
   uint64_t scanned = 0, bytes = 0;     // running totals over the words
   std::vector<unsigned long long> found;  // (vertex, source) pairs of levels 1, 2, ..., the empty one included
 
