@@ -372,6 +372,7 @@ __global__ void k_ppr1_init(uint64_t n, uint32_t seed, const uint32_t* __restric
 // weighted PageRank and its adjoint
 // ---------------------------------------------------------------------------------------------
 struct GatherWeighted {  // sum_a p[a] * x[col[a]]
+  static constexpr bool kDeep = true;
   const uint32_t* __restrict__ col;
   const double* __restrict__ p;
   const double* __restrict__ x;
@@ -396,7 +397,10 @@ struct FinishAffine {
   const double* __restrict__ base;  // null: constant base_c
   double base_c, scale, d;
   double* __restrict__ maxdiff;
+  const double* __restrict__ before;  // null, or the largest change at the last check: nothing is left to do
+  double tol;
   unsigned long long largest = 0;
+  __device__ __forceinline__ bool stopped() const { return before && *before <= tol; }
   __device__ __forceinline__ void operator()(uint32_t v, double sum) {
     const double b = base ? scale * base[v] : base_c;
     const double val = b + d * sum;
@@ -428,117 +432,116 @@ __global__ void k_affine_init(uint64_t n, const double* __restrict__ base, doubl
   }
 }
 
-// p[a] = w[a] / s[row(a)] over the CSR, and pw[slot] = rw[slot] / s[rcol[slot]] over the CSC
-struct VisitNormalise {
+// Visits of every arc through the row schedule: a warp a row left a hub to one warp (RMAT-20: 1050 us to
+// normalise, 1320 for the weight gradient).
+struct VisitNormalise {  // p[a] = w[a] / s[row]
   const double* __restrict__ w;
   const double* __restrict__ s;
   double* __restrict__ p;
+  __device__ __forceinline__ double operator()(uint32_t u, uint64_t a) const {
+    p[a] = __ldg(w + a) / __ldg(s + u);
+    return 0.0;
+  }
+};
+struct VisitGradW {  // gw[a] = d * r[u] / s[u] * (lambda[col[a]] - pl[u]), f[u] = d * r[u] / s[u]
+  const uint32_t* __restrict__ col;
+  const double* __restrict__ f;
+  const double* __restrict__ lambda;
+  const double* __restrict__ pl;
+  double* __restrict__ gw;
+  __device__ __forceinline__ double operator()(uint32_t u, uint64_t a) const {
+    gw[a] = __ldg(f + u) * (__ldg(lambda + __ldg(col + a)) - __ldg(pl + u));
+    return 0.0;
+  }
+};
+struct VisitEnd {
+  __device__ __forceinline__ void operator()(uint32_t, double) const {}
 };
 
+__global__ void k_grad_factor(uint64_t n, const double* __restrict__ r, const double* __restrict__ s, double d, double* __restrict__ f) {
+  for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x) f[u] = d * r[u] / s[u];
+}
+
+// pw[slot] = rw[slot] / s[rcol[slot]] over the CSC
 __global__ void k_csc_normalise(uint64_t m, const uint32_t* __restrict__ rcol, const double* __restrict__ rw,
                                 const double* __restrict__ s, double* __restrict__ pw) {
   for (uint64_t a = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; a < m; a += (uint64_t)gridDim.x * blockDim.x)
     pw[a] = rw[a] / s[rcol[a]];
-}
-__global__ void k_csr_normalise(uint64_t n, const uint64_t* __restrict__ off, const double* __restrict__ w,
-                                const double* __restrict__ s, double* __restrict__ p) {
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint64_t u = warp; u < n; u += nwarps) {
-    const double su = s[u];
-    for (uint64_t a = off[u] + lane; a < off[u + 1]; a += 32) p[a] = w[a] / su;
-  }
-}
-
-// grad_w[a] = d * r[u] / s[u] * (lambda[col[a]] - pl[u]) for every arc of row u
-__global__ void k_grad_w(uint64_t n, const uint64_t* __restrict__ off, const uint32_t* __restrict__ col, const double* __restrict__ r,
-                         const double* __restrict__ s, const double* __restrict__ lambda, const double* __restrict__ pl, double d,
-                         double* __restrict__ gw) {
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint64_t u = warp; u < n; u += nwarps) {
-    const uint64_t a0 = off[u], a1 = off[u + 1];
-    if (a0 == a1) continue;
-    const double f = d * r[u] / s[u];
-    const double plu = pl[u];
-    for (uint64_t a = a0 + lane; a < a1; a += 32) gw[a] = f * (lambda[col[a]] - plu);
-  }
 }
 
 __global__ void k_scale(uint64_t n, const double* __restrict__ x, double f, double* __restrict__ y) {
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) y[v] = f * x[v];
 }
 
-// Row sums s, CSR-normalised p and CSC-normalised pw of the FP64 weights (kept in workspace).
+// Row sums s of the FP64 weights and the normalised ones (in workspace): by CSC slot (pw) for the
+// forward solve, by CSR arc (p) for the adjoint.
 struct WeightedPrep {
   double* s;
   double* p;
   double* pw;
 };
-static int weighted_prep(gre_graph g, WeightedPrep* wp) {
+static int weighted_prep(gre_graph g, bool adjoint, WeightedPrep* wp) {
   if (!g->w64 || !g->rw64) {
     set_error("weighted PageRank needs FP64 arc weights (gre_graph_set_weights_f64)");
     return GRE_INVALID_ARG;
   }
   GRE_CHECK(ensure_bins(g, false));
   GRE_CHECK(ws_array(g, WS_I, g->n, &wp->s));
-  GRE_CHECK(ws_array(g, WS_J, g->m, &wp->p));
-  GRE_CHECK(ws_array(g, WS_K, g->m, &wp->pw));
   double* partial;
   GRE_CHECK(ws_array(g, WS_H, g->bins_out.n_partials + 1, &partial));
   GRE_CUDA(cudaMemsetAsync(wp->s, 0, sizeof(double) * g->n, g->stream));
   GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, GatherW{g->w64}, FinishStore{wp->s}, partial, g->stream));
-  k_csr_normalise<<<grid_for(g->n * 32, 256), 256, 0, g->stream>>>(g->n, g->off, g->w64, wp->s, wp->p);
-  k_csc_normalise<<<grid_for(g->m, 256), 256, 0, g->stream>>>(g->m, g->rcol, g->rw64, wp->s, wp->pw);
+  if (adjoint) {
+    GRE_CHECK(ws_array(g, WS_J, g->m, &wp->p));
+    GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, VisitNormalise{g->w64, wp->s, wp->p}, VisitEnd{}, partial, g->stream));
+  } else {
+    GRE_CHECK(ws_array(g, WS_K, g->m, &wp->pw));
+    k_csc_normalise<<<grid_for(g->m, 256), 256, 0, g->stream>>>(g->m, g->rcol, g->rw64, wp->s, wp->pw);
+  }
   GRE_LAUNCH_CHECK();
   return GRE_SUCCESS;
 }
 
 // Jacobi iteration y = base + d * (A x) with A given by (bins, off, col, p), to tolerance.
+//
+// The largest change is looked at after every fourth iteration.  The host launches kAhead iterations
+// and then reads their changes; a kernel whose last looked-at change was small enough returns at
+// once, so the result is that of the first such look whatever was launched behind it (a host read every
+// four iterations cost 5 us an iteration, RMAT-20: 113).
 static int affine_solve(gre_graph g, const DegreeBins& B, const uint64_t* off, const uint32_t* col, const double* p,
                         const double* base, double scale, double base_c, double d, double tol, uint32_t max_iters,
                         double* xa, double* xb, double** result, uint32_t* iters_done, gre_stats* st) {
+  constexpr uint32_t kCheck = 4, kAhead = 32;  // even: the buffers are back in place
   double* partial;
-  double* maxdiff;
+  double* maxdiff;  // of the iterations launched together
   GRE_CHECK(ws_array(g, WS_H, B.n_partials + 1, &partial));
-  GRE_CHECK(ws_array(g, WS_COUNTERS, 2, &maxdiff));
+  GRE_CHECK(ws_array(g, WS_COUNTERS, kAhead, &maxdiff));
   k_affine_init<<<grid_for(g->n, 256), 256, 0, g->stream>>>(g->n, base, base_c, scale, xa, xb);
-  // one iteration x -> y; maxdiff holds that iteration's largest change (reset first)
-  auto iteration = [&](double* x, double* y) -> int {
-    GRE_CUDA(cudaMemsetAsync(maxdiff, 0, sizeof(double), g->stream));
-    // rows without arcs keep base (set by init in both buffers)
-    return rows::reduce_rows(B, off, GatherWeighted{col, p, x}, FinishAffine{y, x, base, base_c, scale, d, maxdiff}, partial,
-                             g->stream);
-  };
-  // convergence is read every check_every iterations (an even number: the buffers are back in
-  // place), so that block is recorded once as a CUDA graph and replayed until it converges
-  const uint32_t check_every = 4;
-  Recorded rec;
-  GRE_CHECK(rec.record(g->stream, [&]() {
-    int e = 0;
-    for (uint32_t i = 0; i < check_every && !e; ++i) e = (i & 1) ? iteration(xb, xa) : iteration(xa, xb);
-    return e;
-  }));
-  double* x = xa;
-  double* y = xb;
+  GRE_LAUNCH_CHECK();
+  double *x = xa, *y = xb;
   uint32_t it = 0;
-  while (it < max_iters) {
-    if (it + check_every <= max_iters && x == xa) {
-      GRE_CHECK(rec.replay(g->stream));
-      it += check_every;
-    } else {
-      GRE_CHECK(iteration(x, y));
-      std::swap(x, y);
-      ++it;
+  for (bool small = false; !small && it < max_iters;) {
+    const uint32_t k = std::min(kAhead, max_iters - it);
+    GRE_CUDA(cudaMemsetAsync(maxdiff, 0, sizeof(double) * k, g->stream));
+    double *from = x, *to = y;
+    for (uint32_t i = 0; i < k; ++i) {
+      // rows without arcs keep base (set by init in both buffers)
+      const double* before = i >= kCheck ? maxdiff + i / kCheck * kCheck - 1 : nullptr;
+      GRE_CHECK(rows::reduce_rows(B, off, GatherWeighted{col, p, from},
+                                  FinishAffine{to, from, base, base_c, scale, d, maxdiff + i, before, tol}, partial, g->stream));
+      std::swap(from, to);
     }
-    if (it % check_every == 0 || it == max_iters) {
-      double h = 0;
-      GRE_CUDA(cudaMemcpyAsync(&h, maxdiff, sizeof h, cudaMemcpyDeviceToHost, g->stream));
-      GRE_CUDA(cudaStreamSynchronize(g->stream));
-      if (h <= tol) break;
-    }
+    double h[kAhead];
+    GRE_CUDA(cudaMemcpyAsync(h, maxdiff, sizeof(double) * k, cudaMemcpyDeviceToHost, g->stream));
+    GRE_CUDA(cudaStreamSynchronize(g->stream));
+    uint32_t ran = k;
+    for (uint32_t i = kCheck; i <= k && !small; i += kCheck)
+      if (h[i - 1] <= tol) {
+        small = true;
+        ran = i;
+      }
+    it += ran;
+    if (ran & 1) std::swap(x, y);
   }
   *result = x;
   *iters_done = it;
@@ -682,8 +685,8 @@ int gre_pagerank_weighted(gre_graph g, double d, const double* pers, double tol,
   stats_reset(st);
   const uint64_t n = g->n;
   GRE_CHECK(ensure_bins(g, true));
-  WeightedPrep wp;
-  GRE_CHECK(weighted_prep(g, &wp));
+  WeightedPrep wp{};
+  GRE_CHECK(weighted_prep(g, false, &wp));
   const double* dpers;
   double *dr, *xa, *xb, *res;
   GRE_CHECK(stage_input(g, pers, n, WS_G, &dpers));
@@ -715,8 +718,8 @@ int gre_pagerank_adjoint(gre_graph g, double d, const double* r, const double* c
   stats_reset(st);
   const uint64_t n = g->n, m = g->m;
   GRE_CHECK(ensure_bins(g, true));
-  WeightedPrep wp;
-  GRE_CHECK(weighted_prep(g, &wp));
+  WeightedPrep wp{};
+  GRE_CHECK(weighted_prep(g, true, &wp));
   const double *dr, *dc;
   double *xa, *xb, *res, *pl, *dgw, *dlam = nullptr, *dgp = nullptr;
   GRE_CHECK(stage_input(g, r, n, WS_F, &dr));
@@ -741,7 +744,9 @@ int gre_pagerank_adjoint(gre_graph g, double d, const double* r, const double* c
   GRE_CHECK(ws_array(g, WS_H, g->bins_out.n_partials + 1, &partial));
   GRE_CUDA(cudaMemsetAsync(pl, 0, sizeof(double) * n, g->stream));
   GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, GatherWeighted{g->col, wp.p, res}, FinishStore{pl}, partial, g->stream));
-  k_grad_w<<<grid_for(n * 32, 256), 256, 0, g->stream>>>(n, g->off, g->col, dr, wp.s, res, pl, d, dgw);
+double* f = res == xa ? xb : xa;
+  k_grad_factor<<<grid_for(n, 256), 256, 0, g->stream>>>(n, dr, wp.s, d, f);
+  GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, VisitGradW{g->col, f, res, pl, dgw}, VisitEnd{}, partial, g->stream));
   GRE_LAUNCH_CHECK();
   if (g->perm) GRE_CHECK(arcs_to_caller(g, dgw, dgw_final, 8));
   dgw = dgw_final;

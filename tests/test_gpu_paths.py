@@ -313,3 +313,54 @@ def test_batched_betweenness_shapes(shape, directed, reorder, k):
         # positive terms only, so that every sum, product and division costs at most half an ulp of what it
         # adds to; no more than n sums and two roundings a level follow one another, on either side
         np.testing.assert_allclose(got, bc_ref(n, off, col, srcs), rtol=2 * 3 * n * 1.2e-16, atol=0)
+
+
+@pytest.mark.parametrize("schedule", ["", "2,32,64,0", "2,32,64,100", "8,512,65536,0"])
+@pytest.mark.parametrize("tol,limits", [(0.0, [0, 1, 3, 4, 6, 31, 32, 33, 70]), (1e-3, [5, 28, 200]), (1e-14, [400])])
+def test_weighted_solve_stops_where_it_converges(monkeypatch, schedule, tol, limits):
+    """The solve looks at every fourth iteration's change: ranks and the number of iterations equal a plain
+    loop's for limits around the launches' groups, and the gradients those of the formulas, over rows at the
+    limits of every bin."""
+    if schedule:
+        monkeypatch.setenv("GRE_ROW_SCHEDULE", schedule)
+    n, d = 400, 0.85
+    off, col = rows_graph(EDGES * 3, n, 5)
+    rng = np.random.default_rng(6)
+    w, c = np.exp(rng.standard_normal(len(col))), rng.standard_normal(n)
+    src = np.repeat(np.arange(n), np.diff(off.astype(np.int64)))
+    s = np.bincount(src, weights=w, minlength=n)
+    p = w / s[src]
+    g = G.Graph.from_csr(n, off, col)
+    g.set_weights_f64(w)
+
+    def solve(base, to, frm, limit):
+        x, it = base.copy(), 0
+        while it < limit:
+            y = base + d * np.bincount(to, weights=p * x[frm], minlength=n)
+            change = np.abs(y - x).max()
+            x, it = y, it + 1
+            if it % 4 == 0 and change <= tol:
+                break
+        return x, it
+
+    for limit in limits:
+        ref, it = solve(np.full(n, 1 - d), col, src, limit)
+        r, st, _ = G.pagerank_weighted(g, d, tol=tol, max_iters=limit)
+        # sums of at most 1025 positive terms below the result, a product and a sum an iteration
+        bound = 1100 * 2.3e-16 / (1 - d)
+
+        def same_end(got, ref, largest):
+            # a tolerance below the roundings themselves is met when they settle, not at a given iteration
+            assert got == ref if not 0 < tol < bound * largest else got % 4 == 0 and got < limit
+
+        same_end(st.supersteps, it, ref.max())
+        np.testing.assert_allclose(r, ref, rtol=bound, atol=0)
+        lam, gp, gw, st, _ = G.pagerank_adjoint(g, ref, c, d, tol=tol, max_iters=limit)
+        ref_lam, it = solve(c, src, col, limit)
+        scale = np.abs(c).max() / (1 - d)  # of every partial sum
+        same_end(st.supersteps, it, scale)
+        pl = np.bincount(src, weights=p * ref_lam[col], minlength=n)
+        np.testing.assert_allclose(lam, ref_lam, rtol=0, atol=bound * scale)
+        np.testing.assert_allclose(gp, (1 - d) * ref_lam, rtol=0, atol=bound * scale)
+        f = (d * ref / np.where(s > 0, s, 1))[src]
+        np.testing.assert_allclose(gw, f * (ref_lam[col] - pl[src]), rtol=0, atol=4 * bound * scale * f.max())
