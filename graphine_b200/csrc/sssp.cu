@@ -515,7 +515,14 @@ struct AddU64 {
 // Bucket width of the near-far split.  Default: 3/8 of the mean arc weight (RMAT-26, weights in
 // [1, 255], heavy passes pulled: delta 24 / 32 / 40 / 48 / 64 / 96 / 128 gave 23.3 / 20.6 / 20.4
 // / 19.9 / 20.4 / 22.2 / 25.0 ms); 0 relaxes every improved vertex at once (Bellman-Ford frontier).
+// On a smaller graph a pass is a chain of round trips whatever its arcs, and arcs relaxed again cost less
+// than a bucket more: 3/4 of the mean below 2^22 arcs, twice the mean below 2^20.  Four sources, weights in
+// [1, 255], at 3/8, 3/4 and 2 of the mean: 26K arcs 1381 / 1076 / 1019 us, 135K 1827 / 1483 / 1353, 670K (directed)
+// 2409 / 1993 / 1852, 1.9M 2356 / 2280 / 2407, 2.4M 3150 / 2761 / 3163, 9.7M 4520 / 4493 / 4783, 34M
+// 5490 / 5823 / 6752.  (No buckets at all is faster still on these graphs up to 2^20 arcs, 1651 us at 670K, but
+// nothing bounds what it relaxes again.)
 // The GRE_SSSP_DELTA environment variable overrides it.
+constexpr uint64_t kWideBucketArcs = 1ull << 20, kNarrowBucketArcs = 1ull << 22;
 int sssp_delta(gre_graph g, uint32_t* delta) {
   if (const char* e = getenv("GRE_SSSP_DELTA")) {
     *delta = (uint32_t)strtoul(e, nullptr, 10);
@@ -534,7 +541,7 @@ int sssp_delta(gre_graph g, uint32_t* delta) {
     GRE_CUDA(cudaStreamSynchronize(g->stream));
     g->w32_mean = g->m ? (double)sum / (double)g->m : 1.0;
   }
-  const double d = g->w32_mean * 0.375;
+  const double d = g->w32_mean * (g->m < kWideBucketArcs ? 2.0 : g->m < kNarrowBucketArcs ? 0.75 : 0.375);
   *delta = d < 1.0 ? 1u : d > 1e9 ? 1000000000u : (uint32_t)d;
   return GRE_SUCCESS;
 }
