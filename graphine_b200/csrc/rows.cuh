@@ -43,6 +43,11 @@ __device__ __forceinline__ auto row_skipped(const G& g, uint32_t v, int) -> decl
 template <class G>
 __device__ __forceinline__ bool row_skipped(const G&, uint32_t, long) { return false; }
 
+// Programmatic dependent launch: the next launch of the row kernel may start its blocks once all of this
+// one's have started; they wait for its end (and so for all before it) ahead of their first load.
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Sum of gat(v, a) over a = a0 + lig, a0 + lig + L, ... < a1.  Four arcs per pass so that each
 // lane has four independent (column, gathered value) load chains in flight: the loop is bound
 // by memory latency, not bandwidth, when a lane waits on one chain at a time.  Eight where the gather
@@ -163,6 +168,8 @@ template <class Gather, class Finish>
 __global__ void __launch_bounds__(kCta) k_rows_all(const __grid_constant__ RowPlan P, const uint64_t* __restrict__ off, Gather gat,
                                                    Finish fin, double* __restrict__ partial) {
   __shared__ double smem[kCta / 32];
+  launch_next();
+  wait_previous();
   if (launch_stopped(fin, 0)) return;
   uint32_t s = 0;
   while (blockIdx.x >= P.block[s + 1]) ++s;
@@ -231,7 +238,17 @@ int reduce_rows(const DegreeBins& B, const uint64_t* off, Gather gat, Finish fin
   const bool windows = B.seg_nchunks != 0;  // the rows above cta_min, window by window
   const RowPlan P = plan_rows(B, windows);
   if (!P.block[8]) return GRE_SUCCESS;
-  k_rows_all<<<P.block[8], kCta, 0, s>>>(P, off, gat, fin, partial);
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(P.block[8]);
+  cfg.blockDim = dim3(kCta);
+  cfg.stream = s;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  GRE_CUDA(cudaLaunchKernelEx(&cfg, k_rows_all<Gather, Finish>, P, off, gat, fin, partial));
+  launch_count_add(1);
   if (windows)
     k_rows_chunk_finish<<<grid_for(B.seg_nrows, 128, 4), 128, 0, s>>>(B.seg_rows, B.seg_nrows, B.seg_first, partial, fin);
   else if (B.count[7])
