@@ -285,6 +285,30 @@ int device_ingest_parts(const char* prefix, uint32_t nparts, uint32_t flags, int
 
 void launch_count_add(long long k);
 
+// Launch with programmatic stream serialization: once all blocks of the kernel before it in the stream have
+// called launch_next (or ended), this one's may start.  They call wait_previous, all of them, ahead of
+// anything that depends on the stream's earlier work: it returns when that kernel has ended and, as that
+// one waited in its turn, all before it.
+template <class... P, class... A>
+int launch_early(cudaStream_t s, unsigned int grid, unsigned int block, void (*kernel)(P...), A... args) {
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = s;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  GRE_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+  launch_count_add(1);
+  return GRE_SUCCESS;
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 inline void stats_reset(gre_stats* st) {
   if (!st) return;
   st->supersteps = 0;

@@ -29,6 +29,7 @@ struct GatherContrib {
   const double* __restrict__ contrib;
   // contrib is read-only during a superstep (the next values go to the other buffer)
   __device__ __forceinline__ double operator()(uint32_t, uint64_t a) const { return __ldg(contrib + __ldg(rcol + a)); }
+  __device__ __forceinline__ void warm(uint64_t a) const { asm volatile("" ::"r"(__ldg(rcol + a))); }
 };
 
 struct FinishPR {
@@ -377,6 +378,7 @@ struct GatherWeighted {  // sum_a p[a] * x[col[a]]
   const double* __restrict__ p;
   const double* __restrict__ x;
   __device__ __forceinline__ double operator()(uint32_t, uint64_t a) const { return __ldg(p + a) * x[__ldg(col + a)]; }
+  __device__ __forceinline__ void warm(uint64_t a) const { asm volatile("" ::"r"(__ldg(col + a))); }
 };
 struct GatherW {  // sum_a w[a]
   const double* __restrict__ w;
