@@ -174,10 +174,16 @@ __global__ void k_uf_flatten(uint64_t n, uint32_t* parent, uint32_t* __restrict_
 }
 
 // Relabelled graphs: least[r] = smallest caller id in the tree of root r (parent[v] = root of v on
-// the way; least starts as a copy of perm).  A warp's lanes in the tree of its first lane send one atomic, and an id that is not
-// smaller than the one already there sends none: the giant tree's word would serialise them.
+// the way; least starts as a copy of perm).  A warp keeps the smallest id of the tree of its first lane
+// from step to step and hands it on when that tree changes: nearly all warps meet the giant tree's
+// word, which serves one request a clock, reads too (looked at every step: RMAT-22 42 us, so 23).
+__device__ __forceinline__ void uf_lower(uint32_t* least, uint32_t r, uint32_t id) {
+  if (id < __ldcg(least + r)) atomicMin(least + r, id);
+}
 __global__ void k_uf_least(uint64_t n, uint32_t* parent, const uint32_t* __restrict__ perm, uint32_t* least) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const bool lead = (threadIdx.x & 31u) == 0;
+  uint32_t tree = 0xffffffffu, low = 0xffffffffu;  // the warp's
   for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < n; base += stride) {
     const uint64_t v = base + (threadIdx.x & 31u);
     uint32_t r = 0xffffffffu, id = 0xffffffffu;
@@ -187,11 +193,16 @@ __global__ void k_uf_least(uint64_t n, uint32_t* parent, const uint32_t* __restr
       id = __ldg(perm + v);
     }
     const uint32_t first = __shfl_sync(0xffffffffu, r, 0);  // lane 0 holds a vertex
-    const uint32_t low = __reduce_min_sync(0xffffffffu, r == first ? id : 0xffffffffu);
-    const bool lead = (threadIdx.x & 31u) == 0;
-    if (lead) id = low;
-    if (v < n && (lead || r != first) && id < __ldcg(least + r)) atomicMin(least + r, id);
+    if (first != tree) {
+      if (lead && tree != 0xffffffffu) uf_lower(least, tree, low);
+      tree = first;
+      low = 0xffffffffu;
+    }
+    const uint32_t step = __reduce_min_sync(0xffffffffu, r == first ? id : 0xffffffffu);
+    low = step < low ? step : low;
+    if (v < n && r != first) uf_lower(least, r, id);
   }
+  if (lead && tree != 0xffffffffu) uf_lower(least, tree, low);
 }
 __global__ void k_uf_label(uint64_t n, const uint32_t* __restrict__ iperm, const uint32_t* __restrict__ parent,
                            const uint32_t* __restrict__ least, uint32_t* __restrict__ label) {
