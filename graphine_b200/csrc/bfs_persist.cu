@@ -34,6 +34,16 @@ namespace gre {
 
 constexpr int kBfsThreads = 512;
 
+// Back from bottom-up to top-down below n/18 frontier vertices; not yet, for two levels, when the vertices
+// not found so far hold less than 1/32 of the arcs: with so little left to look at a bottom-up step is
+// 4-5 us, the way back (queue from the bits, one barrier more, a top-down step) 10-16 us, and most searches
+// end there (RMAT-22, a frontier of 65473: 15.8 us).  RMAT-22, 16 sources 2610 -> 2540 us; eight over 20000 vertices
+// 537 -> 484, over 200000 748 -> 680, over 1.5M 964 -> 906.  At RMAT-25 the bits themselves are 4 MB a step:
+// 7490 -> 7640 us for eight, so graphs above 2^23 vertices go back at once.
+constexpr uint64_t kFewLeft = 32;
+constexpr uint32_t kLate = 2;
+constexpr uint64_t kLateVertices = 1ull << 23;
+
 struct BfsSlot {  // the frontier of one level
   unsigned long long nf, mf;      // vertices, their out-arcs
   unsigned long long scanned;     // arcs looked at by the bottom-up step that found it
@@ -290,7 +300,7 @@ __global__ void __launch_bounds__(kBfsThreads, 2) k_bfs_persist(const __grid_con
   long long mu = (long long)R.m;
   unsigned long long visited = 0;
   bool bu = false;
-  uint32_t d = 0;
+  uint32_t d = 0, late = 0;
   for (;; ++d) {
     BfsSlot* s = &c->slot[d % 3];
     BfsSlot* sn = &c->slot[(d + 1) % 3];
@@ -318,10 +328,11 @@ __global__ void __launch_bounds__(kBfsThreads, 2) k_bfs_persist(const __grid_con
     uint2* queue = (d & 1) ? R.q1 : R.q0;
     if (!bu && (double)mf > (double)mu / 15.0 && nf > 64) {
       bu = true;
-    } else if (bu && nf < R.n / 18) {
+    } else if (bu && nf < R.n / 18 && (R.n > kLateVertices || mu > (long long)(R.m / kFewLeft) || ++late > kLate)) {
       bits_to_items(R, cur, other, queue, &s->nitems, st, gwarp, nwarps);
       if (!grid_barrier(&c->bar, target, R.wait_ns, [&] { st.nitems = __ldcg(&s->nitems); })) return;
       bu = false;
+      late = 0;
     }
     if (bu) {
       if (first) c->bytes += 16 * (R.n - visited) + R.n / 8;
