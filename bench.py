@@ -269,8 +269,17 @@ def reference_configs(workdir: str) -> dict:
 REF_THREADS = 12  # the reference engine's fixed worker pool (Engine.hpp:211), plus its master thread
 
 
+def reference_built():
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle as O
+    return O.reference_available()
+
+
 def run_reference_arm(args, rank, world):
     if rank != 0:
+        return 0
+    if not reference_built():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference engine's binaries (oracle/_ref) are not built here"}))
         return 0
     t0 = time.perf_counter()
     with tempfile.TemporaryDirectory() as td:
@@ -690,7 +699,7 @@ def run_ours(args, rank, world, local_rank):
         extra["configs"] = configs_block(G, local_rank)
         extra["same_scale_as_reference"] = same_scale_block(G, local_rank, args)
     cpu = None
-    if world == 1 and not args.no_cpu_baseline:
+    if world == 1 and not args.no_cpu_baseline and reference_built():
         with tempfile.TemporaryDirectory() as td:
             res, info = reference_suite(args.ref_scale, 1, td)
         e, s = res[0]
