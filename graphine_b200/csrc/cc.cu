@@ -173,14 +173,17 @@ __global__ void k_uf_flatten(uint64_t n, uint32_t* parent, uint32_t* __restrict_
     label[v] = uf_find(parent, (uint32_t)v);
 }
 
-// Relabelled graphs: least[r] = smallest caller id in the tree of root r (parent[v] = root of v on
-// the way; least starts as a copy of perm).  A warp keeps the smallest id of the tree of its first lane
+// Relabelled graphs: least[r] = smallest caller id in the tree of root r (least starts as a copy of perm)
+// and label[caller id of v] = root of v.  The root is written to the label, not to parent[v]: another
+// thread's uf_find that passes through v may store an inner vertex to parent[v] after it, and on deep trees did.
+// A warp keeps the smallest id of the tree of its first lane
 // from step to step and hands it on when that tree changes: nearly all warps meet the giant tree's
 // word, which serves one request a clock, reads too (looked at every step: RMAT-22 42 us, so 23).
 __device__ __forceinline__ void uf_lower(uint32_t* least, uint32_t r, uint32_t id) {
   if (id < __ldcg(least + r)) atomicMin(least + r, id);
 }
-__global__ void k_uf_least(uint64_t n, uint32_t* parent, const uint32_t* __restrict__ perm, uint32_t* least) {
+__global__ void k_uf_least(uint64_t n, uint32_t* parent, const uint32_t* __restrict__ perm, uint32_t* least,
+                           uint32_t* __restrict__ label) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const bool lead = (threadIdx.x & 31u) == 0;
   uint32_t tree = 0xffffffffu, low = 0xffffffffu;  // the warp's
@@ -189,8 +192,8 @@ __global__ void k_uf_least(uint64_t n, uint32_t* parent, const uint32_t* __restr
     uint32_t r = 0xffffffffu, id = 0xffffffffu;
     if (v < n) {
       r = uf_find(parent, (uint32_t)v);
-      parent[v] = r;
       id = __ldg(perm + v);
+      label[id] = r;
     }
     const uint32_t first = __shfl_sync(0xffffffffu, r, 0);  // lane 0 holds a vertex
     if (first != tree) {
@@ -204,10 +207,9 @@ __global__ void k_uf_least(uint64_t n, uint32_t* parent, const uint32_t* __restr
   }
   if (lead && tree != 0xffffffffu) uf_lower(least, tree, low);
 }
-__global__ void k_uf_label(uint64_t n, const uint32_t* __restrict__ iperm, const uint32_t* __restrict__ parent,
-                           const uint32_t* __restrict__ least, uint32_t* __restrict__ label) {
+__global__ void k_uf_label(uint64_t n, const uint32_t* __restrict__ least, uint32_t* __restrict__ label) {
   for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x)
-    label[u] = __ldg(least + __ldg(parent + __ldg(iperm + u)));
+    label[u] = __ldg(least + label[u]);
 }
 
 uint32_t uf_most_frequent(std::vector<uint32_t>& hs, uint32_t ns) {
@@ -276,8 +278,8 @@ int gre_cc(gre_graph g, uint32_t* label, gre_stats* st) {
   }
   if (g->perm) {
     GRE_CUDA(cudaMemcpyAsync(least, g->perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, g->stream));
-    k_uf_least<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent, g->perm, least);
-    k_uf_label<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->iperm, parent, least, dlabel);
+    k_uf_least<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent, g->perm, least, dlabel);
+    k_uf_label<<<grid_for(n, 256), 256, 0, g->stream>>>(n, least, dlabel);
   } else {
     k_uf_flatten<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent, dlabel);
   }

@@ -1,0 +1,76 @@
+"""Graphs of large diameter (paths, grids, combs, trees): union-find trees that are deep when the labels are
+taken.  Every component is known from the construction, so the label is its smallest id."""
+import numpy as np
+import pytest
+
+from graphine_b200 import gre as G
+
+pytestmark = pytest.mark.gpu
+
+
+def path(n):
+    return n, np.arange(n - 1), np.arange(1, n)
+
+
+def grid(side):
+    i = np.arange(side * side)
+    right, down = i[i % side != side - 1], i[i < side * (side - 1)]
+    return side * side, np.concatenate([right, down]), np.concatenate([right + 1, down + side])
+
+
+def comb(spine, tooth):
+    s = np.arange(spine)
+    t = spine + s[:, None] * tooth + np.arange(tooth)
+    u = np.concatenate([s[:-1], s, t[:, :-1].ravel()])
+    return spine * (tooth + 1), u, np.concatenate([s[1:], t[:, 0], t[:, 1:].ravel()])
+
+
+def tree(n, window, rng):
+    """Every vertex hangs under one of the `window` before it (0: under any)."""
+    i = np.arange(1, n)
+    back = rng.integers(0, window, n - 1) if window else (rng.random(n - 1) * i).astype(np.int64)
+    return n, np.maximum(0, i - 1 - back), i
+
+
+def pieces(size, rng):
+    """Components of each shape, `size` vertices each, and some small ones: arcs and component of each vertex."""
+    side = int(size**0.5)
+    parts = [path(size), grid(side), comb(side, side - 1), tree(size, 0, rng), tree(size, 8, rng)]
+    parts += [path(1 + i % 7) for i in range(50)]
+    base = np.cumsum([0] + [p[0] for p in parts])
+    u = np.concatenate([p[1] + b for p, b in zip(parts, base)])
+    v = np.concatenate([p[2] + b for p, b in zip(parts, base)])
+    return int(base[-1]), u, v, np.repeat(np.arange(len(parts)), np.diff(base))
+
+
+def deep_forest(size, ids, directed, seed):
+    rng = np.random.default_rng(seed)
+    n, u, v, comp = pieces(size, rng)
+    order = np.arange(n) if ids == "rising" else np.arange(n)[::-1] if ids == "falling" else rng.permutation(n)
+    u, v = order[u], order[v]
+    if directed:
+        turn = rng.random(len(u)) < 0.5  # weakly connected: the direction says nothing
+        u, v = np.where(turn, v, u), np.where(turn, u, v)
+    else:
+        u, v = np.concatenate([u, v]), np.concatenate([v, u])
+    at = np.argsort(u, kind="stable")
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(u, minlength=n))
+    low = np.full(comp.max() + 1, n)
+    np.minimum.at(low, comp, order)
+    want = np.empty(n, np.uint32)
+    want[order] = low[comp]
+    return n, off, v[at].astype(np.uint32), want
+
+
+@pytest.mark.parametrize("reorder", [False, True])
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("ids", ["rising", "falling", "mixed"])
+@pytest.mark.parametrize("size", [900, 200000])
+def test_components_of_deep_graphs(size, ids, directed, reorder):
+    n, off, col, want = deep_forest(size, ids, directed, size)
+    g = G.Graph.from_csr(n, off, col, symmetric=not directed)
+    if reorder:
+        g.reorder()
+    for _ in range(20):  # the threads meet differently every time
+        np.testing.assert_array_equal(G.cc(g)[0], want)
