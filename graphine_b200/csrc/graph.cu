@@ -415,7 +415,9 @@ int finish_graph(gre_graph g) {
   return GRE_SUCCESS;
 }
 
-// Drops everything derived from the CSR (degrees, CSC, arc maps, bins, chunk tables).
+// Drops everything derived from the CSR or indexed by its ids (degrees, CSC, arc maps, bins, chunk tables, the
+// frontier words of the betweenness: those of a vertex without in-arcs are zero because no search writes them,
+// and after a relabelling another vertex has that place).
 static void drop_derived(gre_graph g) {
   g->sssp_split.release();
   const bool alias = (g->roff == g->off);
@@ -439,6 +441,9 @@ static void drop_derived(gre_graph g) {
   free_bins(g->bins_sssp);
   free_chunk_table(g->bc_chunks);
   free_chunk_table(g->ppr_chunks);
+  cudaFree(g->bc_fpool);
+  g->bc_fpool = nullptr;
+  g->bc_fpool_levels = 0;
 }
 
 // Relabel by decreasing degree: new row i = old row perm[i], neighbour ids mapped through

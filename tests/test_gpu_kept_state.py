@@ -1,0 +1,42 @@
+"""State that a graph keeps from one call to the next, where something changes in between."""
+import numpy as np
+import pytest
+
+from graphine_b200 import gre as G
+
+pytestmark = pytest.mark.gpu
+
+
+def dense_part(n, directed, seed):
+    """Random arcs within every second third of the ids (two levels reach all of it, found by pulling), the other
+    vertices without arcs or, on a directed graph, with out-arcs only."""
+    rng = np.random.default_rng(seed)
+    on = np.flatnonzero(np.arange(n) // 3 % 2)
+    u, v = rng.choice(on, 12 * n), rng.choice(on, 12 * n)
+    if directed:
+        off_ids = np.setdiff1d(np.arange(n), on)
+        u, v = np.concatenate([u, off_ids]), np.concatenate([v, rng.choice(on, len(off_ids))])
+    else:
+        u, v = np.concatenate([u, v]), np.concatenate([v, u])
+    keys = np.unique(u.astype(np.int64) * n + v)
+    keys = keys[keys // n != keys % n]
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(keys // n, minlength=n))
+    return off, (keys % n).astype(np.uint32), on
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("n", [100, 5000])
+def test_batched_betweenness_after_relabelling(n, directed):
+    """The frontier words kept for the batched betweenness are those of the ids that searched last."""
+    off, col, on = dense_part(n, directed, n)
+    srcs = np.random.default_rng(1).choice(on, 70).astype(np.uint32)
+    g = G.Graph.from_csr(n, off, col, symmetric=not directed)
+    before, _ = G.bc(g, srcs, batched=True)
+    np.testing.assert_array_equal(before, G.bc(g, srcs, batched=False)[0])
+    g.reorder()
+    after, _ = G.bc(g, srcs, batched=True)
+    np.testing.assert_array_equal(after, G.bc(g, srcs, batched=False)[0])
+    fresh = G.Graph.from_csr(n, off, col, symmetric=not directed)
+    fresh.reorder()
+    np.testing.assert_array_equal(after, G.bc(fresh, srcs, batched=True)[0])
