@@ -123,18 +123,21 @@ __global__ void k_uf_compress_skip(uint64_t n, uint32_t* parent, const uint64_t*
   }
 }
 
-// parent[v] = root of v, and the roots of an evenly spaced sample of vertices
-__global__ void k_uf_compress(uint64_t n, uint32_t* parent, uint64_t stride, uint32_t* __restrict__ sample, uint32_t nsample) {
+// root[v] = root of v, and the roots of an evenly spaced sample of vertices.  parent[v] is set to it too, but
+// a find that passes through v may leave an inner vertex there after that: only root[] is to be relied on.
+__global__ void k_uf_compress(uint64_t n, uint32_t* parent, uint32_t* __restrict__ root, uint64_t stride,
+                              uint32_t* __restrict__ sample, uint32_t nsample) {
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t r = uf_find(parent, (uint32_t)v);
     parent[v] = r;
+    root[v] = r;
     if (v % stride == 0 && v / stride < nsample) sample[v / stride] = r;
   }
 }
 
 // skip bit of every vertex already in the largest component c; counts[0] += arcs sampled,
 // counts[1] += arcs the second pass still visits (byte model)
-__global__ void k_uf_skipbits(uint64_t n, const uint32_t* __restrict__ parent, const uint64_t* __restrict__ off, uint32_t c,
+__global__ void k_uf_skipbits(uint64_t n, const uint32_t* __restrict__ root, const uint64_t* __restrict__ off, uint32_t c,
                               uint32_t k, uint32_t* __restrict__ skip, unsigned long long* __restrict__ counts) {
   const uint64_t nwords = (n + 31) >> 5;
   unsigned long long sampled = 0, rest = 0;
@@ -143,7 +146,7 @@ __global__ void k_uf_skipbits(uint64_t n, const uint32_t* __restrict__ parent, c
     for (uint32_t b = 0; b < 32 && (w << 5) + b < n; ++b) {
       const uint64_t v = (w << 5) + b;
       const uint64_t d = off[v + 1] - off[v];
-      const bool in_c = parent[v] == c;
+      const bool in_c = root[v] == c;
       bits |= (uint32_t)in_c << b;
       sampled += d < k ? d : k;
       if (!in_c && d > k) rest += d - k;

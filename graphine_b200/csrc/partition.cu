@@ -545,12 +545,13 @@ __global__ void k_pcc_count_remote(uint64_t arcs, const uint32_t* __restrict__ c
   if ((threadIdx.x & 31u) == 0 && c) atomicAdd(out, c);
 }
 
-// after phase 1 (parent[i] = root of i): every slot's label is its root's key, every root's
-// component label too
-__global__ void k_pcc_labels(uint64_t L, const uint32_t* __restrict__ parent, const uint32_t* __restrict__ key,
-                             uint32_t* __restrict__ lab, uint32_t* __restrict__ rootlab) {
+// after phase 1 (root[i] = root of i): every slot hangs under its root and its label is the root's key,
+// every root's component label too
+__global__ void k_pcc_labels(uint64_t L, const uint32_t* __restrict__ root, const uint32_t* __restrict__ key,
+                             uint32_t* __restrict__ parent, uint32_t* __restrict__ lab, uint32_t* __restrict__ rootlab) {
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < L; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t r = parent[i];
+    const uint32_t r = root[i];
+    parent[i] = r;
     lab[i] = key[r];
     if (r == i) rootlab[i] = key[i];
   }
@@ -1272,18 +1273,19 @@ int gre_part_cc(gre_part p, uint32_t* label, gre_exchange_fn xchg, void* ctx, gr
   // phase 1: union-find over the arcs inside this rank (Afforest on a symmetric graph, as gre_cc:
   // the first arcs of every row, then the rows outside the largest local component)
   uint64_t visited = 0;
+  uint32_t* roots = lab_all;  // free until the first exchange
   k_uf_init<<<grid_for(L, 256), 256, 0, s->stream>>>(L, parent);
   if (sym) {
     k_pcc_sample<<<grid_for(L, 256), 256, 0, s->stream>>>(L, s->roff, s->rcol, kSampled, lo, parent, key);
     const uint64_t stride = L > kSample ? L / kSample : 1;
     const uint32_t ns = (uint32_t)std::min<uint64_t>(kSample, (L + stride - 1) / stride);
-    k_uf_compress<<<grid_for(L, 256), 256, 0, s->stream>>>(L, parent, stride, sample, ns);
+    k_uf_compress<<<grid_for(L, 256), 256, 0, s->stream>>>(L, parent, roots, stride, sample, ns);
     std::vector<uint32_t> hs(kSample, 0);
     GRE_CUDA(cudaMemcpyAsync(hs.data(), sample, sizeof(uint32_t) * ns, cudaMemcpyDeviceToHost, s->stream));
     GRE_CUDA(cudaStreamSynchronize(s->stream));
     const uint32_t big = uf_most_frequent(hs, ns);
     GRE_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), s->stream));
-    k_uf_skipbits<<<grid_for((L + 31) >> 5, 256), 256, 0, s->stream>>>(L, parent, s->roff, big, kSampled, skip, counts);
+    k_uf_skipbits<<<grid_for((L + 31) >> 5, 256), 256, 0, s->stream>>>(L, roots, s->roff, big, kSampled, skip, counts);
     HookLocal rest{s->rcol, parent, key, lo, (uint32_t)L, skip, s->roff, kSampled};
     GRE_CHECK(rows::reduce_rows(s->bins_in, s->roff, rest, NoFinishPart{}, partial, s->stream));
     unsigned long long h[2] = {0, 0};
@@ -1297,8 +1299,8 @@ int gre_part_cc(gre_part p, uint32_t* label, gre_exchange_fn xchg, void* ctx, gr
                                 s->stream));
     visited = p->arcs_in + p->arcs_out;
   }
-  k_uf_compress<<<grid_for(L, 256), 256, 0, s->stream>>>(L, parent, L + 1, nullptr, 0);
-  k_pcc_labels<<<grid_for(L, 256), 256, 0, s->stream>>>(L, parent, key, lab, rootlab);
+  k_uf_compress<<<grid_for(L, 256), 256, 0, s->stream>>>(L, parent, roots, L + 1, nullptr, 0);
+  k_pcc_labels<<<grid_for(L, 256), 256, 0, s->stream>>>(L, roots, key, parent, lab, rootlab);
   GRE_LAUNCH_CHECK();
   uint64_t bytes = 8 * (L + 1) + 12 * visited + 16 * L;
   // phase 2: the local components' labels meet over the cut arcs, a round per all-gather of the

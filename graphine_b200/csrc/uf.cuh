@@ -43,8 +43,9 @@ __device__ __forceinline__ void uf_union(uint32_t* parent, const uint32_t* __res
 
 // kernels defined in cc.cu
 __global__ void k_uf_init(uint64_t n, uint32_t* __restrict__ parent);
-__global__ void k_uf_compress(uint64_t n, uint32_t* parent, uint64_t stride, uint32_t* __restrict__ sample, uint32_t nsample);
-__global__ void k_uf_skipbits(uint64_t n, const uint32_t* __restrict__ parent, const uint64_t* __restrict__ off, uint32_t c,
+__global__ void k_uf_compress(uint64_t n, uint32_t* parent, uint32_t* __restrict__ root, uint64_t stride,
+                              uint32_t* __restrict__ sample, uint32_t nsample);
+__global__ void k_uf_skipbits(uint64_t n, const uint32_t* __restrict__ root, const uint64_t* __restrict__ off, uint32_t c,
                               uint32_t k, uint32_t* __restrict__ skip, unsigned long long* __restrict__ counts);
 
 // The most frequent root among `ns` sampled roots (Afforest's guess of the largest component).

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from graphine_b200 import gre as G
+from graphine_b200 import partition as PT
 
 pytestmark = pytest.mark.gpu
 
@@ -74,3 +75,21 @@ def test_components_of_deep_graphs(size, ids, directed, reorder):
         g.reorder()
     for _ in range(20):  # the threads meet differently every time
         np.testing.assert_array_equal(G.cc(g)[0], want)
+
+
+# (mixed ids over several parts cut every path everywhere: a round for each cut that a label has to cross)
+@pytest.mark.parametrize("directed,reorder", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("parts,size,ids", [(1, 900, "falling"), (1, 40000, "rising"), (1, 40000, "mixed"), (2, 900, "falling"),
+                                            (2, 40000, "rising"), (3, 900, "mixed"), (3, 40000, "rising")])
+def test_partitioned_components_of_deep_graphs(size, ids, directed, reorder, parts):
+    n, off, col, want = deep_forest(size, ids, directed, size)
+    g = G.Graph.from_csr(n, off, col, symmetric=not directed)
+    if reorder:
+        g.reorder()
+
+    def job(part, exchange):
+        return [part.cc(exchange)[0] for _ in range(10 if parts == 1 else 2)]
+
+    for labels in PT.run_local(g, parts, job):
+        for got in labels:
+            np.testing.assert_array_equal(got, want)
