@@ -35,11 +35,11 @@ struct HookArcs {
   const uint32_t* __restrict__ col;
   uint32_t* parent;
   // Afforest's second pass: rows flagged in `skip` are left out and the first `sampled` arcs of
-  // the others were already united (null: every arc)
-  const uint32_t* __restrict__ skip = nullptr;
+  // the others were already united (null: every arc).  Plain loads: the launch before writes the flags
+  const uint32_t* skip = nullptr;
   const uint64_t* __restrict__ off = nullptr;
   uint32_t sampled = 0;
-  __device__ __forceinline__ bool skips(uint32_t u) const { return skip && ((__ldg(skip + (u >> 5)) >> (u & 31u)) & 1u); }
+  __device__ __forceinline__ bool skips(uint32_t u) const { return skip && ((skip[u >> 5] >> (u & 31u)) & 1u); }
   __device__ __forceinline__ double operator()(uint32_t u, uint64_t a) const {
     if (skip && a < __ldg(off + u) + sampled) return 0.0;
     uf_union(parent, nullptr, u, __ldg(col + a));

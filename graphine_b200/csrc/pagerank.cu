@@ -25,10 +25,12 @@ namespace gre {
 // plain PageRank
 // ---------------------------------------------------------------------------------------------
 struct GatherContrib {
+  // eight blocks an SM: left alone, plain loads take 40 registers and six blocks (PageRank-20, default schedule: RMAT-18
+  // 403 -> 436 us, RMAT-20 1663 -> 1889, RMAT-22 7498 -> 8191, RMAT-24 33.5 -> 35.3 ms; directed RMAT-16 alone 167 -> 146)
+  static constexpr int kBlocks = 8;
   const uint32_t* __restrict__ rcol;
-  const double* __restrict__ contrib;
-  // contrib is read-only during a superstep (the next values go to the other buffer)
-  __device__ __forceinline__ double operator()(uint32_t, uint64_t a) const { return __ldg(contrib + __ldg(rcol + a)); }
+  const double* contrib;  // plain loads: the launch before may still write it when this one starts (launch_early)
+  __device__ __forceinline__ double operator()(uint32_t, uint64_t a) const { return contrib[__ldg(rcol + a)]; }
   __device__ __forceinline__ void warm(uint64_t a) const { asm volatile("" ::"r"(__ldg(rcol + a))); }
 };
 
@@ -376,7 +378,7 @@ struct GatherWeighted {  // sum_a p[a] * x[col[a]]
   static constexpr bool kDeep = true;
   const uint32_t* __restrict__ col;
   const double* __restrict__ p;
-  const double* __restrict__ x;
+  const double* x;  // the launch before may still write it (launch_early)
   __device__ __forceinline__ double operator()(uint32_t, uint64_t a) const { return __ldg(p + a) * x[__ldg(col + a)]; }
   __device__ __forceinline__ void warm(uint64_t a) const { asm volatile("" ::"r"(__ldg(col + a))); }
 };
@@ -395,11 +397,11 @@ struct FinishStore {
 // and bounded the superstep (RMAT-20, 1M rows: 0.90 -> 0.41 ms an iteration).
 struct FinishAffine {
   double* __restrict__ y;
-  const double* __restrict__ xprev;
+  const double* xprev;               // this and `before`: the launch before may still write them
   const double* __restrict__ base;  // null: constant base_c
   double base_c, scale, d;
   double* __restrict__ maxdiff;
-  const double* __restrict__ before;  // null, or the largest change at the last check: nothing is left to do
+  const double* before;  // null, or the largest change at the last check: nothing is left to do
   double tol;
   unsigned long long largest = 0;
   __device__ __forceinline__ bool stopped() const { return before && *before <= tol; }
@@ -438,21 +440,21 @@ __global__ void k_affine_init(uint64_t n, const double* __restrict__ base, doubl
 // normalise, 1320 for the weight gradient).
 struct VisitNormalise {  // p[a] = w[a] / s[row]
   const double* __restrict__ w;
-  const double* __restrict__ s;
+  const double* s;  // the launch before may still write it
   double* __restrict__ p;
   __device__ __forceinline__ double operator()(uint32_t u, uint64_t a) const {
-    p[a] = __ldg(w + a) / __ldg(s + u);
+    p[a] = __ldg(w + a) / s[u];
     return 0.0;
   }
 };
 struct VisitGradW {  // gw[a] = d * r[u] / s[u] * (lambda[col[a]] - pl[u]), f[u] = d * r[u] / s[u]
   const uint32_t* __restrict__ col;
-  const double* __restrict__ f;
+  const double* f;  // the launch before writes it; lambda and pl were complete when that one started
   const double* __restrict__ lambda;
   const double* __restrict__ pl;
   double* __restrict__ gw;
   __device__ __forceinline__ double operator()(uint32_t u, uint64_t a) const {
-    gw[a] = __ldg(f + u) * (__ldg(lambda + __ldg(col + a)) - __ldg(pl + u));
+    gw[a] = f[u] * (__ldg(lambda + __ldg(col + a)) - __ldg(pl + u));
     return 0.0;
   }
 };

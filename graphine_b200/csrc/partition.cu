@@ -251,9 +251,10 @@ __global__ void k_part_out(uint64_t total, const uint32_t* __restrict__ xmap, co
 }
 
 struct PartGather {
+  static constexpr int kBlocks = 8;  // as GatherContrib
   const uint32_t* __restrict__ col;
-  const double* __restrict__ contrib;  // all P * L slots
-  __device__ __forceinline__ double operator()(uint32_t, uint64_t a) const { return __ldg(contrib + __ldg(col + a)); }
+  const double* contrib;  // all P * L slots; plain loads: what the exchange launched last may still write it (launch_early)
+  __device__ __forceinline__ double operator()(uint32_t, uint64_t a) const { return contrib[__ldg(col + a)]; }
 };
 
 // pr = tele + d * sum; the power iteration refreshes the owner's contribution pr / outdeg
@@ -503,13 +504,13 @@ struct HookLocal {
   const uint32_t* __restrict__ key;  // caller id of each slot
   uint32_t lo, L;
   // Afforest's second pass (symmetric graphs): rows flagged in `skip` are left out and the first
-  // `sampled` arcs of the others were already seen (null: every arc)
-  const uint32_t* __restrict__ skip = nullptr;
+  // `sampled` arcs of the others were already seen (null: every arc).  Plain loads: the launch before writes the flags
+  const uint32_t* skip = nullptr;
   const uint64_t* __restrict__ off = nullptr;
   uint32_t sampled = 0;
   __device__ __forceinline__ double operator()(uint32_t u, uint64_t a) const {
     if (skip) {
-      if ((__ldg(skip + (u >> 5)) >> (u & 31u)) & 1u) return 0.0;
+      if ((skip[u >> 5] >> (u & 31u)) & 1u) return 0.0;
       if (a < __ldg(off + u) + sampled) return 0.0;
     }
     const uint32_t x = __ldg(col + a) - lo;  // wraps past L for remote slots

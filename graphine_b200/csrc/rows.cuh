@@ -14,6 +14,7 @@
 //           __device__ bool skips(uint32_t row) const   (optional) rows left out: no arcs, sum 0
 //           __device__ void warm(uint64_t arc) const   (optional) loads of the arc that no launch changes
 //           static constexpr bool kDeep   (optional) true: eight arcs a lane in flight
+//           static constexpr int kBlocks   (optional) blocks an SM that the kernel's registers must allow
 //   Finish: __device__ void operator()(uint32_t row, double sum)
 //           __device__ void end()   (optional) after the block's last row, by all its threads
 //           __device__ bool stopped() const   (optional) true: the launch does nothing
@@ -39,6 +40,10 @@ template <class G>
 constexpr auto deep_gather(int) -> decltype(G::kDeep) { return G::kDeep; }
 template <class G>
 constexpr bool deep_gather(long) { return false; }
+template <class G>
+constexpr auto gather_blocks(int) -> decltype(G::kBlocks) { return G::kBlocks; }
+template <class G>
+constexpr int gather_blocks(long) { return 0; }  // the compiler chooses
 template <class G>
 __device__ __forceinline__ auto row_skipped(const G& g, uint32_t v, int) -> decltype(g.skips(v)) { return g.skips(v); }
 template <class G>
@@ -73,7 +78,9 @@ struct Ready {
 // lane has four independent (column, gathered value) load chains in flight: the loop is bound
 // by memory latency, not bandwidth, when a lane waits on one chain at a time.  Eight where the gather
 // asks for it: with a stream of FP64 weights beside the columns (RMAT-20, an iteration) 118 -> 113 us; the plain
-// PageRank, at 70-80% of what L1 and L2 give to gathers, lost 1% at RMAT-22.
+// PageRank, at 70-80% of what L1 and L2 give to gathers, lost 1% at RMAT-22.  The two or three arcs left are in
+// flight together as well (PageRank-20 at RMAT-22, default schedule: 7695 us one by one, 7498 so; 96 iterations of the weighted
+// solve at RMAT-20 10.91 -> 10.53 ms, RMAT-16 1163 -> 1050 us).
 template <int L, class Gather>
 __device__ __forceinline__ double strided_sum(Gather& gat, uint32_t v, uint64_t a0, uint64_t a1, uint32_t lig) {
   double acc = 0.0;
@@ -93,7 +100,13 @@ __device__ __forceinline__ double strided_sum(Gather& gat, uint32_t v, uint64_t 
     acc += x2;
     acc += x3;
   }
-  for (; a < a1; a += L) acc += gat(v, a);
+  if (a + L < a1) {
+    const double x0 = gat(v, a), x1 = gat(v, a + L);
+    acc += x0;
+    acc += x1;
+    a += 2 * (uint64_t)L;
+  }
+  if (a < a1) acc += gat(v, a);
   return acc;
 }
 
@@ -187,7 +200,7 @@ inline RowPlan plan_rows(const DegreeBins& B, bool windows, int seg_blocks = kSe
 // directed 820 -> 314 us, RMAT-24 36.1 -> 31.9 ms; weighted solves at RMAT-20 147 -> 60 ms).  The sums are
 // those of a launch per bin: a row's association order depends on its bin alone.
 template <class Gather, class Finish>
-__global__ void __launch_bounds__(kCta) k_rows_all(const __grid_constant__ RowPlan P, const uint64_t* __restrict__ off, Gather gat,
+__global__ void __launch_bounds__(kCta, gather_blocks<Gather>(0)) k_rows_all(const __grid_constant__ RowPlan P, const uint64_t* __restrict__ off, Gather gat,
                                                    Finish fin, double* __restrict__ partial) {
   __shared__ double smem[kCta / 32];
   launch_next();

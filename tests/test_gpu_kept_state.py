@@ -40,3 +40,32 @@ def test_batched_betweenness_after_relabelling(n, directed):
     fresh = G.Graph.from_csr(n, off, col, symmetric=not directed)
     fresh.reorder()
     np.testing.assert_array_equal(after, G.bc(fresh, srcs, batched=True)[0])
+
+
+@pytest.mark.parametrize("n", [200, 3000, 40000])
+def test_supersteps_that_start_early_read_the_last_values(n):
+    """A superstep's blocks are on the chip before the one before has ended, and their caches may hold the buffer's
+    older values: long runs of short supersteps give the same bits every time, and the ranks of a float64 loop."""
+    rng = np.random.default_rng(n)
+    u, v = rng.integers(0, n, 8 * n), (rng.integers(0, n, 8 * n) * rng.random(8 * n)).astype(np.int64)
+    order = np.argsort(u, kind="stable")
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(u, minlength=n))
+    col, deg = v[order].astype(np.uint32), np.maximum(np.bincount(u, minlength=n), 1)
+    g = G.Graph.from_csr(n, off, col)
+    iters, d = 120, 0.85
+    x = np.full(n, 1 - d)
+    for _ in range(iters):
+        x = (1 - d) + d * np.bincount(col, weights=(x / deg)[u[order]], minlength=n)
+    first, _ = G.pagerank(g, G.PR_ITER, d, iters)
+    # sums of positive terms, a product, a quotient and a sum a superstep; errors shrink by d from one to the next
+    longest = np.bincount(col, minlength=n).max()
+    np.testing.assert_allclose(first, x, rtol=2 * (longest + 3) * 1.2e-16 / (1 - d), atol=0)
+    for _ in range(30):
+        np.testing.assert_array_equal(G.pagerank(g, G.PR_ITER, d, iters)[0], first)
+    w = np.ones(len(col))
+    g.set_weights_f64(w)
+    weighted, _, _ = G.pagerank_weighted(g, d, tol=0.0, max_iters=iters)
+    np.testing.assert_allclose(weighted, x, rtol=2 * (longest + 3) * 1.2e-16 / (1 - d), atol=0)
+    for _ in range(30):
+        np.testing.assert_array_equal(G.pagerank_weighted(g, d, tol=0.0, max_iters=iters)[0], weighted)
