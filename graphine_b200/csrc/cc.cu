@@ -53,21 +53,40 @@ struct HookArcs {
 // start (ids fall along it, so no cycle), written with plain stores; most of the second arcs then
 // find both ends in one tree.  RMAT-22: 252 us with unions for both
 // arcs, 64 us (29 + 35) so; the whole call 1310 -> 240 us with it and the links by stored id.
+// On a graph without hubs (`joined` given: a bit per vertex) only a parent whose own first arc goes up is taken: rising
+// ids along a path or a tree would hang every vertex under the one before, and the unions that follow walk
+// those chains (10^6 vertices, rising ids, the call with chains / so: path 499 / 236 us, random tree 1172 / 231, comb
+// 379 / 136, grid 614 / 293; ids at random: the same).
 __global__ void k_uf_first(uint64_t n, const uint64_t* __restrict__ off, const uint32_t* __restrict__ col,
-                           uint32_t* __restrict__ parent) {
-  for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t a0 = off[u];
-    const uint32_t v = a0 < off[u + 1] ? __ldg(col + a0) : (uint32_t)u;
-    parent[u] = v < u ? v : (uint32_t)u;
+                           uint32_t* __restrict__ parent, uint32_t* __restrict__ joined) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < n; base += stride) {
+    const uint64_t u = base + (threadIdx.x & 31u);
+    bool in = false;
+    if (u < n) {
+      const uint64_t a0 = off[u];
+      const uint32_t v = a0 < off[u + 1] ? __ldg(col + a0) : (uint32_t)u;
+      in = v < u;
+      if (in && joined) {
+        const uint64_t b0 = off[v];
+        in = b0 == off[v + 1] || __ldg(col + b0) >= v;
+      }
+      parent[u] = in ? v : (uint32_t)u;
+    }
+    if (joined) {
+      const uint32_t word = __ballot_sync(0xffffffffu, in);
+      if ((threadIdx.x & 31u) == 0) joined[base >> 5] = word;
+    }
   }
 }
 __global__ void k_uf_sample(uint64_t n, const uint64_t* __restrict__ off, const uint32_t* __restrict__ col, uint32_t k,
-                            uint32_t* parent) {
+                            uint32_t* parent, const uint32_t* __restrict__ joined) {
   for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t a0 = off[u], a1 = off[u + 1];
     for (uint64_t a = a0; a < a1 && a < a0 + k; ++a) {
       const uint32_t v = __ldg(col + a);
-      if (a > a0 || v > u) uf_union(parent, nullptr, (uint32_t)u, v);
+      if (a == a0 && (joined ? (__ldg(joined + (u >> 5)) >> (u & 31u)) & 1u : v < u)) continue;
+      uf_union(parent, nullptr, (uint32_t)u, v);
     }
   }
 }
@@ -253,6 +272,7 @@ int gre_cc(gre_graph g, uint32_t* label, gre_stats* st) {
     least = (uint32_t*)p;
   }
   constexpr uint32_t kSampled = 2;
+  constexpr uint64_t kHubArcs = 256;  // largest degree of a graph with hubs
   uint32_t *skip = nullptr, *best = nullptr;
   unsigned long long* counts = nullptr;
   if (g->symmetric()) {
@@ -269,8 +289,9 @@ int gre_cc(gre_graph g, uint32_t* label, gre_stats* st) {
     // in both rows, so an edge between the largest component and another vertex is seen from
     // the other side.
     GRE_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), g->stream));
-    k_uf_first<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->off, g->col, parent);
-    k_uf_sample<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->off, g->col, kSampled, parent);
+    uint32_t* joined = g->max_outdeg < kHubArcs ? skip : nullptr;  // the skip flags' words are free until the compression
+    k_uf_first<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->off, g->col, parent, joined);
+    k_uf_sample<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->off, g->col, kSampled, parent, joined);
     k_uf_mode<<<1, kSample, 0, g->stream>>>(n, n > kSample ? n / kSample : 1, parent, best);
     k_uf_compress_skip<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent, g->off, best, kSampled, skip, counts);
     HookArcs rest{g->col, parent, skip, g->off, kSampled};

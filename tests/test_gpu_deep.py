@@ -33,20 +33,24 @@ def tree(n, window, rng):
     return n, np.maximum(0, i - 1 - back), i
 
 
-def pieces(size, rng):
-    """Components of each shape, `size` vertices each, and some small ones: arcs and component of each vertex."""
+def star(n):
+    return n, np.zeros(n - 1, int), np.arange(1, n)
+
+
+def pieces(size, hub, rng):
+    """Components of each shape, `size` vertices each, some small ones and a star: arcs and component of each vertex."""
     side = int(size**0.5)
     parts = [path(size), grid(side), comb(side, side - 1), tree(size, 0, rng), tree(size, 8, rng)]
-    parts += [path(1 + i % 7) for i in range(50)]
+    parts += [path(1 + i % 7) for i in range(50)] + [star(1 + hub)]
     base = np.cumsum([0] + [p[0] for p in parts])
     u = np.concatenate([p[1] + b for p, b in zip(parts, base)])
     v = np.concatenate([p[2] + b for p, b in zip(parts, base)])
     return int(base[-1]), u, v, np.repeat(np.arange(len(parts)), np.diff(base))
 
 
-def deep_forest(size, ids, directed, seed):
+def deep_forest(size, ids, directed, seed, hub=0):
     rng = np.random.default_rng(seed)
-    n, u, v, comp = pieces(size, rng)
+    n, u, v, comp = pieces(size, hub, rng)
     order = np.arange(n) if ids == "rising" else np.arange(n)[::-1] if ids == "falling" else rng.permutation(n)
     u, v = order[u], order[v]
     if directed:
@@ -74,6 +78,19 @@ def test_components_of_deep_graphs(size, ids, directed, reorder):
     if reorder:
         g.reorder()
     for _ in range(20):  # the threads meet differently every time
+        np.testing.assert_array_equal(G.cc(g)[0], want)
+
+
+@pytest.mark.parametrize("directed,reorder", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("size", [900, 70000])
+@pytest.mark.parametrize("hub", [255, 256, 5000])
+def test_components_of_deep_graphs_beside_a_hub(hub, size, directed, reorder):
+    """On either side of the degree from which first arcs are taken as they are."""
+    n, off, col, want = deep_forest(size, "rising", directed, hub, hub)
+    g = G.Graph.from_csr(n, off, col, symmetric=not directed)
+    if reorder:
+        g.reorder()
+    for _ in range(5):
         np.testing.assert_array_equal(G.cc(g)[0], want)
 
 
