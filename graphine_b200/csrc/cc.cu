@@ -273,6 +273,9 @@ int gre_cc(gre_graph g, uint32_t* label, gre_stats* st) {
   }
   constexpr uint32_t kSampled = 2;
   constexpr uint64_t kHubArcs = 256;  // largest degree of a graph with hubs
+  // Blocks of a bin an SM: one wave strides over the rows, so that those of small ids are linked and flattened before the
+  // rest start (directed grid of 10^6 vertices, 16 / 8 blocks: rising ids 234 / 173 us; ids at random 244 / 284)
+  constexpr int kWave = 8;
   uint32_t *skip = nullptr, *best = nullptr;
   unsigned long long* counts = nullptr;
   if (g->symmetric()) {
@@ -295,10 +298,17 @@ int gre_cc(gre_graph g, uint32_t* label, gre_stats* st) {
     k_uf_mode<<<1, kSample, 0, g->stream>>>(n, n > kSample ? n / kSample : 1, parent, best);
     k_uf_compress_skip<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent, g->off, best, kSampled, skip, counts);
     HookArcs rest{g->col, parent, skip, g->off, kSampled};
-    GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, rest, NoFinish{}, partial, g->stream));
+    GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, rest, NoFinish{}, partial, g->stream, kWave));
   } else {
     k_uf_init<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent);
-    GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, HookArcs{g->col, parent}, NoFinish{}, partial, g->stream));
+    const HookArcs arcs{g->col, parent};
+    // Hubs that do not have the smallest ids: their CTAs link the loose vertices of half the graph and the root
+    // changes under all of them, unless the short rows went first.  One launch / bin by bin: RMAT-16, 0.95M
+    // arcs 306 / 135 us, RMAT-18, 1.5M 545 / 230; about equal at 0.25M (97 / 92) and 4M (290 / 292); RMAT-20 at 6M 434 / 604,
+    // and a relabelled graph's hubs are the roots (RMAT-18: 128 / 275), as is a tree's parent (random tree: 81 / 520).
+    const bool apart = !g->perm && g->max_outdeg >= kHubArcs && g->m >= (1ull << 18) && g->m < (1ull << 22);
+    if (apart) GRE_CHECK(rows::visit_rows_apart(g->bins_out, g->off, arcs, NoFinish{}, partial, g->stream, kWave));
+    else GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, arcs, NoFinish{}, partial, g->stream, kWave));
   }
   if (g->perm) {
     GRE_CUDA(cudaMemcpyAsync(least, g->perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, g->stream));

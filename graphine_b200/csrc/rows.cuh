@@ -273,9 +273,10 @@ __global__ void k_rows_chunk_finish(const uint32_t* __restrict__ rows, uint64_t 
 
 // Launch the reductions of every non-empty row.  `partial` holds bins.n_partials doubles.
 template <class Gather, class Finish>
-int reduce_rows(const DegreeBins& B, const uint64_t* off, Gather gat, Finish fin, double* partial, cudaStream_t s) {
+int reduce_rows(const DegreeBins& B, const uint64_t* off, Gather gat, Finish fin, double* partial, cudaStream_t s,
+                int seg_blocks = kSegBlocks) {
   const bool windows = B.seg_nchunks != 0;  // the rows above cta_min, window by window
-  const RowPlan P = plan_rows(B, windows);
+  const RowPlan P = plan_rows(B, windows, seg_blocks);
   if (!P.block[8]) return GRE_SUCCESS;
   GRE_CHECK(launch_early(s, P.block[8], kCta, k_rows_all<Gather, Finish>, P, off, gat, fin, partial));
   if (windows)
@@ -283,6 +284,21 @@ int reduce_rows(const DegreeBins& B, const uint64_t* off, Gather gat, Finish fin
   else if (B.count[7])
     k_rows_chunk_finish<<<grid_for(B.count[7], 128, 4), 128, 0, s>>>(B.rows + B.start[7], B.count[7], B.hub_chunk_first, partial, fin);
   GRE_LAUNCH_CHECK();
+  return GRE_SUCCESS;
+}
+
+// Visits of every arc whose sums nobody reads: the bins one after the other, short rows first.
+template <class Gather, class Finish>
+int visit_rows_apart(const DegreeBins& B, const uint64_t* off, Gather gat, Finish fin, double* partial, cudaStream_t s,
+                     int seg_blocks) {
+  const RowPlan all = plan_rows(B, B.seg_nchunks != 0, seg_blocks);
+  for (int k = 7; k >= 0; --k) {
+    const uint32_t blocks = all.block[k + 1] - all.block[k];
+    if (!blocks) continue;
+    RowPlan P = all;
+    for (int i = 0; i <= 8; ++i) P.block[i] = i > k ? blocks : 0;
+    GRE_CHECK(launch_early(s, blocks, kCta, k_rows_all<Gather, Finish>, P, off, gat, fin, partial));
+  }
   return GRE_SUCCESS;
 }
 

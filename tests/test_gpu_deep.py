@@ -110,3 +110,31 @@ def test_partitioned_components_of_deep_graphs(size, ids, directed, reorder, par
     for labels in PT.run_local(g, parts, job):
         for got in labels:
             np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("arcs", [(1 << 18) - 1, 1 << 18, 600000, (1 << 22) - 1, 1 << 22])
+def test_components_of_directed_hubs(arcs):
+    """On either side of the sizes between which a directed graph's bins are visited one after the other: two halves,
+    each with a hub of large id, rows of every bin, and vertices that no arc meets."""
+    rng = np.random.default_rng(arcs)
+    n = arcs // 4
+    half = n // 2
+    u = np.concatenate([np.repeat([half - 1, n - 1], arcs // 8), (rng.random(arcs - 2 * (arcs // 8)) ** 4 * half).astype(np.int64)])
+    v = rng.integers(0, half - 20, arcs)
+    top = (u >= half) | ((u < half - 1) & (rng.random(arcs) < 0.5))
+    u, v = np.where(top & (u < half), u + half, u), np.where(top, v + half, v)
+    at = np.argsort(u, kind="stable")
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(u, minlength=n))
+    g = G.Graph.from_csr(n, off, v[at].astype(np.uint32))
+    want = np.arange(n)
+    while True:  # weak components: labels both ways, and along the labels
+        low = want.copy()
+        np.minimum.at(low, v, want[u])
+        np.minimum.at(low, u, low[v])
+        low = low[low]
+        if (low == want).all():
+            break
+        want = low
+    for _ in range(5):
+        np.testing.assert_array_equal(G.cc(g)[0], want.astype(np.uint32))
