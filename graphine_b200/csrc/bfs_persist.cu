@@ -272,11 +272,12 @@ __global__ void __launch_bounds__(kBfsThreads, 2) k_bfs_persist(const __grid_con
   for (uint64_t v = gtid; v < R.n; v += nthreads) R.level[v] = -1;
   for (uint64_t w = gtid; w < R.nwords; w += nthreads) R.vis0[w] = ~R.arc_bits[w];
   if (!grid_barrier(&c->bar, target, R.wait_ns)) return;
-  if (blockIdx.x == 0) {  // the roots, each once
+  // the roots, each once, over all blocks (one block took 10 ms for two million while the others waited)
+  if ((uint64_t)blockIdx.x * kBfsThreads < R.nroots) {
     unsigned long long nf = 0, mf = 0;
     BfsAppend append(st.items, &c->slot[0].nitems, R.q0);
-    for (uint32_t base = 0; base < R.nroots; base += kBfsThreads) {
-      const uint32_t i = base + threadIdx.x;
+    for (uint64_t base = (uint64_t)blockIdx.x * kBfsThreads; base < R.nroots; base += nthreads) {
+      const uint64_t i = base + threadIdx.x;
       uint32_t rv[1] = {0}, nit[1] = {0};
       if (i < R.nroots) {
         const uint32_t r = rv[0] = R.roots ? R.roots[i] : R.root;

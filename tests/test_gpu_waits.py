@@ -1,0 +1,67 @@
+"""The level loops' bounded waits, and several handles at work at once."""
+import threading
+
+import numpy as np
+import pytest
+
+from graphine_b200 import gre as G
+
+pytestmark = pytest.mark.gpu
+
+
+def rmat(scale, seed, directed=False, reorder=False):
+    n, off, col = G.rmat_host(scale, 16, seed, not directed)
+    g = G.Graph.from_csr(n, off, col, symmetric=not directed)
+    if reorder:
+        g.reorder()
+    g.set_weights_hash(5)
+    return g, G.sample_sources(off, 64, 1)
+
+
+@pytest.mark.parametrize("threads", [2, 4])
+def test_handles_of_several_threads(threads):
+    """Every handle has its stream, and every level loop asks for all SMs at once: calls from several host threads
+    give what each gives alone."""
+    jobs = []
+    for t in range(threads):
+        g, srcs = rmat(13 + t % 3, 40 + t, reorder=t % 2 == 1)
+        jobs.append((g, srcs, [
+            lambda g=g, s=srcs: G.bfs(g, s[:4])[0],
+            lambda g=g, s=srcs: G.sssp(g, s[:2])[0],
+            lambda g=g, s=srcs: G.msbfs(g, s)[0],
+            lambda g=g, s=srcs: G.bfs_multiroot(g, s[:3])[0],
+            lambda g=g, s=srcs: G.bc(g, s, batched=True)[0],
+            lambda g=g: G.pagerank(g, G.PR_ITER, 0.85, 10)[0],
+            lambda g=g: G.cc(g)[0],
+        ]))
+    want = [[call() for call in calls] for _, _, calls in jobs]
+    errors, start = [], threading.Barrier(threads)
+
+    def work(t):
+        try:
+            start.wait()
+            for turn in range(8):
+                for i in range(len(jobs[t][2])):
+                    k = (i + t + turn) % len(jobs[t][2])
+                    np.testing.assert_array_equal(jobs[t][2][k](), want[t][k])
+        except BaseException as e:  # noqa: BLE001
+            errors.append(e)
+
+    pool = [threading.Thread(target=work, args=(t,)) for t in range(threads)]
+    for p in pool:
+        p.start()
+    for p in pool:
+        p.join()
+    if errors:
+        raise errors[0]
+
+
+def test_many_roots_within_the_wait_budget(monkeypatch):
+    """Two million roots, most of them twice: taking them is no longer than a level (budget 2 ms, default 2000)."""
+    n = 1 << 21
+    off = np.minimum(np.arange(n + 1), n - 1).astype(np.uint64)  # a path along the ids, directed
+    g = G.Graph.from_csr(n, off, np.arange(1, n, dtype=np.uint32))
+    roots = np.concatenate([np.arange(1, n, 2), np.arange(n)[::-1]]).astype(np.uint32)
+    monkeypatch.setenv("GRE_GRID_WAIT_MS", "2")
+    level, _ = G.bfs_multiroot(g, roots)
+    np.testing.assert_array_equal(level, 0)
