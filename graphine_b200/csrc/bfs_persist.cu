@@ -226,6 +226,7 @@ __device__ __forceinline__ void bottom_up(const BfsRun& R, const uint32_t* cur, 
         const uint32_t n = __shfl_sync(0xffffffffu, len[j], src);
         bool hit = false;
         for (uint32_t i = 0; i < n && !hit; i += 64) {
+          if ((i & 0xffffu) == 0 && i && lane == 0) grid_beat(&R.ctl->bar);  // every 0.7 ms
           const uint32_t p = i + lane, q = p + 32;
           const uint32_t x = p < n ? __ldg(R.rcol + b + p) : 0u, y = q < n ? __ldg(R.rcol + b + q) : 0u;
           scanned += (p < n) + (q < n);

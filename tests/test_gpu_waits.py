@@ -65,3 +65,33 @@ def test_many_roots_within_the_wait_budget(monkeypatch):
     monkeypatch.setenv("GRE_GRID_WAIT_MS", "2")
     level, _ = G.bfs_multiroot(g, roots)
     np.testing.assert_array_equal(level, 0)
+
+
+def test_long_row_of_another_component_within_the_wait_budget(monkeypatch):
+    """A search that turns bottom-up looks at every row not reached, among them a star's: one warp is at it for some
+    40 ms, twice the budget, and says so."""
+    leaves, n1, ef = 4000000, 1 << 17, 32
+    rng = np.random.default_rng(3)
+    u, v = rng.integers(0, n1, n1 * ef), rng.integers(0, n1, n1 * ef)
+    n, hub = n1 + leaves + 1, n1
+    star = np.arange(hub + 1, n)
+    u, v = np.concatenate([u, v, np.full(leaves, hub), star]), np.concatenate([v, u, star, np.full(leaves, hub)])
+    at = np.argsort(u, kind="stable")
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(u, minlength=n))
+    col = v[at].astype(np.uint32)
+    g = G.Graph.from_csr(n, off, col, symmetric=True)
+    want, _ = G.bfs(g, [0])
+    front, level, d = np.array([0]), np.full(n, -1), 0
+    level[0] = 0
+    while len(front):
+        d += 1
+        on = np.zeros(n, bool)
+        on[front] = True
+        heads = v[on[u]]
+        front = np.unique(heads[level[heads] < 0])
+        level[front] = d
+    np.testing.assert_array_equal(want, level)
+    monkeypatch.setenv("GRE_GRID_WAIT_MS", "20")
+    for _ in range(3):
+        np.testing.assert_array_equal(G.bfs(g, [0])[0], level)
