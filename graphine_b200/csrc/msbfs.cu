@@ -36,7 +36,8 @@ using u64 = unsigned long long;
 
 constexpr int kMsThreads = 512;
 constexpr uint32_t kHead = 512, kTail = 512;  // multiples of 128
-constexpr uint32_t kPlanes = 4;               // bit planes of the first group: levels below 16
+constexpr uint32_t kPlanes = 4;               // bit planes of a group: levels below 16 need one, below 256 two, ...
+constexpr uint32_t kDeepGroups = 7;           // groups after the first (levels below 2^32)
 
 struct MsSlot {  // the frontier of one level
   u64 nf, bits, mf;  // vertices, (vertex, source) pairs, out-arcs of the vertices
@@ -68,7 +69,7 @@ struct MsRun {
   u64* front;   // frontier words of level d at (d & ring) * n
   uint32_t ring;
   u64* planes;  // null: none.  [n][4]: planes 0..3
-  u64* deep;    // planes 4.. in groups of [n][4]
+  u64* deep[kDeepGroups];  // planes 4..7, 8..11, ..: [n][4] each
   uint2* q0;
   uint2* q1;
   uint32_t limit;  // levels from this one on wait for more space
@@ -115,7 +116,7 @@ __device__ __forceinline__ uint64_t commit(const MsRun& R, u64* next, uint64_t v
     for (uint32_t x = level & (16u - 1u); x; x &= x - 1) R.planes[v * 4 + __ffs(x) - 1] |= nb;
     for (uint32_t x = level >> kPlanes; x; x &= x - 1) {
       const uint32_t b = __ffs(x) - 1;
-      R.deep[((b >> 2) * R.n + v) * 4 + (b & 3u)] |= nb;
+      R.deep[b / kPlanes][v * 4 + b % kPlanes] |= nb;
     }
   }
   const uint64_t deg = R.off[v + 1] - R.off[v];
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_msbfs(const __grid_constant__
     }
     resumed = false;
     if (st.bits == 0) break;
-    if (d + 1 >= R.limit) {  // the host makes room
+    if (d + 1 >= R.limit && !(R.planes && st.mf == 0)) {  // the host makes room (for planes: if anything can follow)
       if (first) {
         c->d = d;
         c->queued = queued;
@@ -450,10 +451,14 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_msbfs(const __grid_constant__
   }
 }
 
+struct MsDeep {
+  const u64* group[kDeepGroups];
+};
+
 // The planes of 32 vertices a warp, in the caller's order, as one row of 32 levels a source.
 template <bool DEEP>
 __global__ void __launch_bounds__(256) k_ms_levels(uint64_t n, uint32_t k, uint32_t nplanes, const u64* __restrict__ seen,
-                                                   const u64* __restrict__ planes, const u64* __restrict__ deep,
+                                                   const u64* __restrict__ planes, const __grid_constant__ MsDeep deep,
                                                    const uint32_t* __restrict__ iperm, const uint64_t* __restrict__ off,
                                                    int32_t* __restrict__ out, u64* __restrict__ reached) {
   u64 arcs = 0;
@@ -468,7 +473,7 @@ __global__ void __launch_bounds__(256) k_ms_levels(uint64_t n, uint32_t k, uint3
                    (uint32_t)((p23.y >> j) & 1ull) << 3;
       if constexpr (DEEP)
         for (uint32_t e = 0; e + kPlanes < nplanes; ++e)
-          x |= (uint32_t)((deep[((e >> 2) * n + v) * 4 + (e & 3u)] >> j) & 1ull) << (e + kPlanes);
+          x |= (uint32_t)((deep.group[e / kPlanes][v * 4 + e % kPlanes] >> j) & 1ull) << (e + kPlanes);
       out[(uint64_t)j * n + u] = (s >> j) & 1ull ? (int32_t)x : -1;
     }
   }
@@ -500,12 +505,6 @@ int pool_levels(gre_graph g, uint64_t levels) {
   g->bc_fpool = p;
   g->bc_fpool_levels = want;
   return GRE_SUCCESS;
-}
-
-uint32_t planes_for(uint64_t n) {  // levels are below n
-  uint32_t b = kPlanes;
-  while (b < 32 && (n >> b)) ++b;
-  return b;
 }
 
 }  // namespace
@@ -565,13 +564,13 @@ int MsBfs::run(const uint32_t* dsrcs, uint32_t k, bool record) {
   R.wait_ns = grid_wait_ns();
   R.ring = keep_ ? 0xffffffffu : 1u;
   R.limit = keep_ ? 0 : 1u << kPlanes;
-  deep_ = nullptr;
+  ngroups_ = 0;
   GRE_CUDA(cudaMemsetAsync(ctl, 0, sizeof(MsCtl), g->stream));
   MsCtl h;
   do {
     R.front = keep_ ? (u64*)g->bc_fpool : front_;
     if (keep_) R.limit = (uint32_t)std::min<uint64_t>(g->bc_fpool_levels, 0xffffffffu);
-    R.deep = deep_;
+    for (uint32_t e = 0; e < ngroups_; ++e) R.deep[e] = deep_[e];
     void* args[] = {&R};
     GRE_CUDA(cudaLaunchCooperativeKernel((const void*)k_msbfs, dim3(grid_), dim3(kMsThreads), args, 0, g->stream));
     launch_count_add(1);
@@ -586,10 +585,14 @@ int MsBfs::run(const uint32_t* dsrcs, uint32_t k, bool record) {
     if (keep_) {
       GRE_CHECK(pool_levels(g, g->bc_fpool_levels + 1));
     } else {
-      const uint64_t groups = (planes_for(n) - kPlanes + 3) / 4;
-      GRE_CHECK(ws_array(g, WS_G, groups * 4 * n, &deep_));
-      GRE_CUDA(cudaMemsetAsync(deep_, 0, sizeof(u64) * groups * 4 * n, g->stream));
-      R.limit = 0xffffffffu;
+      // a group more: all that levels up to n could need would be 192 bytes a vertex at 2^26 vertices
+      constexpr int slots[kDeepGroups] = {WS_G, WS_J, WS_K, WS_L, WS_M, WS_N, WS_PERM_IN};
+      u64** p = &deep_[ngroups_];
+      GRE_CHECK(ws_array(g, slots[ngroups_], kPlanes * n, p));
+      GRE_CUDA(cudaMemsetAsync(*p, 0, sizeof(u64) * kPlanes * n, g->stream));
+      ++ngroups_;
+      const uint32_t bits = kPlanes * (ngroups_ + 1);
+      R.limit = bits < 32 ? 1u << bits : 0xffffffffu;
     }
     GRE_CUDA(cudaMemsetAsync(&ctl->bar, 0, sizeof(GridBar), g->stream));
   } while (true);
@@ -610,7 +613,9 @@ int MsBfs::write_levels(uint32_t k, int32_t* out, unsigned long long* reached) {
   uint32_t nplanes = kPlanes;
   while (nplanes < 32 && (levels >> nplanes)) ++nplanes;
   auto kernel = nplanes > kPlanes ? k_ms_levels<true> : k_ms_levels<false>;
-  kernel<<<grid_for(n, 256, 8), 256, 0, g->stream>>>(n, k, nplanes, seen, planes_, deep_, g->iperm, g->off, out, reached);
+  MsDeep deep{};
+  for (uint32_t e = 0; e < ngroups_; ++e) deep.group[e] = deep_[e];
+  kernel<<<grid_for(n, 256, 8), 256, 0, g->stream>>>(n, k, nplanes, seen, planes_, deep, g->iperm, g->off, out, reached);
   GRE_LAUNCH_CHECK();
   return GRE_SUCCESS;
 }

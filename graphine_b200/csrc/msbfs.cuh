@@ -18,7 +18,7 @@ struct MsBfs {
   uint64_t scanned = 0, bytes = 0;     // running totals over the words
   std::vector<unsigned long long> found;  // (vertex, source) pairs of levels 1, 2, ..., the empty one included
 
-  // Workspaces (slots WS_A..WS_F, WS_H) and the launch shape.
+  // Workspaces (slots WS_A..WS_F, WS_H; deep searches WS_G, WS_J..WS_N) and the launch shape.
   int prepare(gre_graph graph, bool keep_levels);
   // The level loop from k <= 64 sources (internal ids, device); waited for.
   int run(const uint32_t* dsrcs, uint32_t k, bool record);
@@ -29,7 +29,9 @@ struct MsBfs {
  private:
   bool keep_ = false;
   uint2 *q0_ = nullptr, *q1_ = nullptr;
-  unsigned long long *acc_ = nullptr, *front_ = nullptr, *planes_ = nullptr, *deep_ = nullptr;
+  unsigned long long *acc_ = nullptr, *front_ = nullptr, *planes_ = nullptr;
+  unsigned long long* deep_[7] = {};  // further groups of planes, taken when a search gets that deep
+  uint32_t ngroups_ = 0;
   unsigned char* ctl_ = nullptr;
   int grid_ = 0;
 };

@@ -69,3 +69,23 @@ def test_supersteps_that_start_early_read_the_last_values(n):
     np.testing.assert_allclose(weighted, x, rtol=2 * (longest + 3) * 1.2e-16 / (1 - d), atol=0)
     for _ in range(30):
         np.testing.assert_array_equal(G.pagerank_weighted(g, d, tol=0.0, max_iters=iters)[0], weighted)
+
+
+@pytest.mark.parametrize("depth,groups", [(15, 0), (16, 1), (255, 1), (256, 2), (300, 2)])
+def test_word_bfs_takes_room_for_the_levels_it_meets(depth, groups):
+    """Levels as bit planes, 32 bytes a vertex for every four: a search takes those that its levels need."""
+    import torch
+
+    n = 1 << 20
+    off = np.minimum(np.arange(n + 1), depth).astype(np.uint64)  # a path of `depth` arcs, the rest without arcs
+    g = G.Graph.from_csr(n, off, np.arange(1, depth + 1, dtype=np.uint32))
+    out = torch.empty(2 * n, dtype=torch.int32, device="cuda")
+    G.msbfs(g, [depth, depth - 2], out=out)
+    free = torch.cuda.mem_get_info()[0]
+    G.msbfs(g, [0, 1], out=out)
+    taken = free - torch.cuda.mem_get_info()[0]
+    assert taken <= groups * (32 * n + (2 << 20)), f"{taken / n:.1f} bytes a vertex"
+    want = np.full((2, n), -1)
+    want[0, : depth + 1] = np.arange(depth + 1)
+    want[1, 1 : depth + 1] = np.arange(depth)
+    np.testing.assert_array_equal(out.cpu().numpy().reshape(2, n), want)
