@@ -245,7 +245,8 @@ struct __align__(16) BcEntry {
 
 // A level's part of the two lists of vertices.
 struct BcList {
-  uint32_t short0, long0;          // where it begins (known when the level before is complete)
+  uint64_t short0, long0;          // where it begins (known when the level before is complete); all levels together
+                                   // may hold up to 64 n vertices
   unsigned int nshort, nlong;
 };
 
