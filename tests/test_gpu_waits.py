@@ -95,3 +95,50 @@ def test_long_row_of_another_component_within_the_wait_budget(monkeypatch):
     monkeypatch.setenv("GRE_GRID_WAIT_MS", "20")
     for _ in range(3):
         np.testing.assert_array_equal(G.bfs(g, [0])[0], level)
+
+
+CALLS = {
+    "bfs": lambda g, s: G.bfs(g, s[:2]),
+    "bfs_multiroot": lambda g, s: G.bfs_multiroot(g, s[:9]),
+    "sssp": lambda g, s: G.sssp(g, s[:2]),
+    "msbfs": lambda g, s: G.msbfs(g, s),
+    "bc": lambda g, s: G.bc(g, s, batched=True),
+    "bc looped": lambda g, s: G.bc(g, s[:2], batched=False),
+}
+
+
+@pytest.mark.parametrize("reorder", [False, True])
+@pytest.mark.parametrize("call", CALLS)
+def test_a_wait_that_runs_out_leaves_the_handle_usable(monkeypatch, call, reorder):
+    """A budget of nothing: every wait gives up at once, the call ends with the status, and the next calls on the same
+    handle (that one, and those that share its scratch) give what they gave before."""
+    g, srcs = rmat(14, 32, reorder=reorder)
+    want = {name: f(g, srcs)[0] for name, f in CALLS.items()}
+    monkeypatch.setenv("GRE_GRID_WAIT_MS", "0")
+    for _ in range(2):
+        with pytest.raises(G.GreError) as e:
+            CALLS[call](g, srcs)
+        assert e.value.status == G.GRE_TIMEOUT
+        assert "grid barrier" in str(e.value)
+    monkeypatch.delenv("GRE_GRID_WAIT_MS")
+    for name in [call, *CALLS]:
+        np.testing.assert_array_equal(CALLS[name](g, srcs)[0], want[name])
+
+
+@pytest.mark.parametrize("directed,reorder", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("k", [1, 64])
+def test_counts_of_the_level_loops_are_those_of_the_levels(k, directed, reorder):
+    """Pairs found a level, supersteps and traversed edges of the 64-source BFS and of a search from several roots,
+    from the levels themselves."""
+    n, off, col = G.rmat_host(13, 16, 31, not directed)
+    g = G.Graph.from_csr(n, off, col, symmetric=not directed)
+    if reorder:
+        g.reorder()
+    srcs = G.sample_sources(off, k, 4)
+    deg = np.diff(off.astype(np.int64))
+    for levels, st in (G.msbfs(g, srcs), G.bfs_multiroot(g, srcs)):
+        rows = levels.reshape(-1, n)
+        # the level after the deepest is looked at too, and empty
+        assert list(st.active) == [int((rows == d).sum()) for d in range(1, rows.max() + 2)]
+        assert st.supersteps == rows.max()
+        assert st.traversed_edges == sum(deg[row >= 0].sum() for row in rows) // (1 if directed else 2)
