@@ -15,9 +15,9 @@
 // process under a key made from the degree distribution (arcs per power-of-two degree bucket,
 // log2 n, log2 m), so graphs of the same shape - the batches of a run, replicas - tune once.
 //
-// GRE_TUNE=0 in the environment turns the measurement off (the default schedule is used), and
-// graphs with fewer than 2^22 arcs always use a fixed one of short chains: their supersteps are
-// too short to time apart from launch overhead.  GRE_ROW_SCHEDULE=lane_arcs,cta_min,hub_chunk,seg_window
+// Graphs with fewer than 2^22 arcs are not measured: their supersteps are
+// too short to time apart from launch overhead.  From 2^16 arcs on they use a fixed schedule of short chains, below
+// that the default one.  GRE_TUNE=0 in the environment turns all of this off: every graph uses the default schedule.  GRE_ROW_SCHEDULE=lane_arcs,cta_min,hub_chunk,seg_window
 // imposes a schedule (tests use it to reach every kernel on small graphs).
 #include <cub/cub.cuh>
 
@@ -413,7 +413,7 @@ int ensure_bins(gre_graph g, bool in) {
   // 4096 314 us, 4 / 1024 231, 4 / 512 215, 8 / 512 196, 2 / 512 198, 4 / 256 214).  Larger graphs
   // lose by it (RMAT-24: 31.9 -> 34.6 ms); the smallest have no row that long and gain nothing
   // (RMAT-11, 45K arcs: 148 us either way; RMAT-12, 97K: 189 -> 148 us).
-  if (g->m >= kShortChainMinArcs && g->m < kTuneMinArcs) {
+  if (tuning_enabled() && g->m >= kShortChainMinArcs && g->m < kTuneMinArcs) {
     sched.lane_arcs = 8;
     sched.cta_min = 512;
   }

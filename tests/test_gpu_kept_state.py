@@ -89,3 +89,11 @@ def test_word_bfs_takes_room_for_the_levels_it_meets(depth, groups):
     want[0, : depth + 1] = np.arange(depth + 1)
     want[1, 1 : depth + 1] = np.arange(depth)
     np.testing.assert_array_equal(out.cpu().numpy().reshape(2, n), want)
+
+
+@pytest.mark.parametrize("scale,edgefactor,want", [(8, 4, (4, 4096)), (13, 16, (8, 512)), (16, 16, (8, 512))])
+def test_row_schedules_below_the_tuned_sizes(monkeypatch, scale, edgefactor, want):
+    """Short chains from 2^16 arcs on; with GRE_TUNE=0 the default schedule at every size."""
+    assert G.Graph.rmat(scale, edgefactor, 5, True).row_schedule()[:2] == want
+    monkeypatch.setenv("GRE_TUNE", "0")
+    assert G.Graph.rmat(scale, edgefactor, 5, True).row_schedule() == (4, 4096, 65536, 0)
