@@ -17,11 +17,12 @@
 //     kept; what is found goes to the other buffer.  Back to top-down, the queue is the difference
 //     of the two buffers.
 // Vertices without any arc count as visited from the start (RMAT: about half of all): their words
-// are skipped.  (Those with out-arcs only do not: they are nobody's parent until a search starts there.)  Levels go straight to the caller's order (perm), so nothing is reordered after.
+// are skipped.  (Those with out-arcs only are not marked: they are nobody's parent until a search
+// starts there.)  Levels go straight to the caller's order (perm), so nothing is reordered after.
 //
-// Measured against the host-driven loop: RMAT-22, 16 sources one after the other, 7240 -> 2870 us;
-// 32 graphs of 2^12..2^18 vertices in one union 517 -> 203 us; 4000 vertices 310 -> 104 us.  A
-// barrier is 1.5 us; most of a small level is the chain of dependent loads (queue, offsets, column,
+// Measured against the host-driven loop: RMAT-22, 16 sources one after the other, 7470 -> 2540 us;
+// 32 graphs of 2^12..2^18 vertices in one union 550 -> 204 us; 4000 vertices 294 -> 103 us; a grid of 1000 x 1000
+// 98 -> 14.4 ms.  A barrier is 1.5 us; most of a small level is the chain of dependent loads (queue, offsets, column,
 // bit, claim).
 #include <algorithm>
 #include <vector>
@@ -56,7 +57,6 @@ struct BfsCtl {
   unsigned long long arcs_td, arcs_bu, bytes, reached_arcs;
   unsigned int levels, pad;
 };
-size_t bfs_ctl_bytes() { return sizeof(BfsCtl); }
 
 struct BfsRun {
   uint64_t n, m, nwords;  // nwords: a multiple of 4

@@ -52,7 +52,7 @@ struct HookArcs {
 // first arc, where it leads to a smaller id, needs no union: it is the vertex's parent from the
 // start (ids fall along it, so no cycle), written with plain stores; most of the second arcs then
 // find both ends in one tree.  RMAT-22: 252 us with unions for both
-// arcs, 64 us (29 + 35) so; the whole call 1310 -> 240 us with it and the links by stored id.
+// arcs, 64 us (29 + 35) so; the whole call 1240 -> 215 us with it, the links by stored id and k_uf_least.
 // On a graph without hubs (`joined` given: a bit per vertex) only a parent whose own first arc goes up is taken: rising
 // ids along a path or a tree would hang every vertex under the one before, and the unions that follow walk
 // those chains (10^6 vertices, rising ids, the call with chains / so: path 499 / 236 us, random tree 1172 / 231, comb

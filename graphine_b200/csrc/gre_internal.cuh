@@ -334,7 +334,7 @@ int ensure_chunk_table(gre_graph g, ChunkTable& T, uint64_t ch);
 void free_chunk_table(ChunkTable& T);
 // CSC slot -> CSR arc map; built once per graph.
 int ensure_rarc(gre_graph g);
-// SSSP bucket width: 3/8 of the mean uint32 weight (GRE_SSSP_DELTA overrides; 0 = no buckets).
+// SSSP bucket width: 3/8 of the mean uint32 weight, more below 2^22 arcs (GRE_SSSP_DELTA overrides; 0 = no buckets).
 int sssp_delta(gre_graph g, uint32_t* delta);
 // Heads a partitioned relaxation owns itself (sssp.cu offer forms): heads in [lo, lo + len) are
 // relaxed in place, as in the one-GPU pass (dist[head - lo] lowered by atomic min, the head's bit

@@ -80,7 +80,7 @@ static int ws_array(gre_graph g, int slot, uint64_t count, T** p) {
 // at 43%, L2 at 46%, warps waiting for loads (ncu).  64 columns keep a quarter of the rows there (which
 // draw nine tenths of the arcs), one 16-byte load a lane and arc, eight arcs in flight; the columns' second
 // reading of the topology is 4 bytes an arc: 0.95 ms a slice and superstep, 17 TB/s of gathered rows,
-// L2 and L1 at 64% (RMAT-20, 128 vectors, 20 supersteps: 61.1 -> 41.5 ms; slices of 32 columns: 46.2).
+// L2 and L1 at 64% (RMAT-20, 128 vectors, 20 supersteps: 61.2 -> 42.7 ms; slices of 32 columns: 46.2).
 //
 // The columns are independent: a slice runs all its supersteps before the next.  The values
 // themselves are written by the last superstep only, in place of the next contributions.
@@ -748,7 +748,7 @@ int gre_pagerank_adjoint(gre_graph g, double d, const double* r, const double* c
   GRE_CHECK(ws_array(g, WS_H, g->bins_out.n_partials + 1, &partial));
   GRE_CUDA(cudaMemsetAsync(pl, 0, sizeof(double) * n, g->stream));
   GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, GatherWeighted{g->col, wp.p, res}, FinishStore{pl}, partial, g->stream));
-double* f = res == xa ? xb : xa;
+  double* f = res == xa ? xb : xa;
   k_grad_factor<<<grid_for(n, 256), 256, 0, g->stream>>>(n, dr, wp.s, d, f);
   GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, VisitGradW{g->col, f, res, pl, dgw}, VisitEnd{}, partial, g->stream));
   GRE_LAUNCH_CHECK();

@@ -520,7 +520,9 @@ struct AddU64 {
 // [1, 255], at 3/8, 3/4 and 2 of the mean: 26K arcs 1381 / 1076 / 1019 us, 135K 1827 / 1483 / 1353, 670K (directed)
 // 2409 / 1993 / 1852, 1.9M 2356 / 2280 / 2407, 2.4M 3150 / 2761 / 3163, 9.7M 4520 / 4493 / 4783, 34M
 // 5490 / 5823 / 6752.  (No buckets at all is faster still on these graphs up to 2^20 arcs, 1651 us at 670K, but
-// nothing bounds what it relaxes again.)
+// nothing bounds what it relaxes again.)  The partitioned path takes the same width: a pass there is host-driven, so fewer
+// buckets are worth more (two parts on one GPU, 3/8, 3/4 and 2 of the mean: 25K arcs 12.7 / 9.3 / 6.7 ms, 205K 12.6 / 9.2 / 5.9,
+// 884K 15.2 / 10.6 / 6.7, 2.6M 15.4 / 11.2 / 7.0, 3.7M 16.6 / 11.4 / 7.9).
 // The GRE_SSSP_DELTA environment variable overrides it.
 constexpr uint64_t kWideBucketArcs = 1ull << 20, kNarrowBucketArcs = 1ull << 22;
 int sssp_delta(gre_graph g, uint32_t* delta) {
