@@ -23,6 +23,7 @@
 // Byte model: 8(n+1) offsets + 12 per visited arc (column + two parent probes, mostly L2)
 // + 8n init/final labels (+ n/4 for the skip bits and their reads).
 #include <algorithm>
+#include <cstdlib>
 #include <vector>
 
 #include "gre_internal.cuh"
@@ -34,14 +35,14 @@ namespace gre {
 struct HookArcs {
   const uint32_t* __restrict__ col;
   uint32_t* parent;
-  // Afforest's second pass: rows flagged in `skip` are left out and the first `sampled` arcs of
-  // the others were already united (null: every arc).  Plain loads: the launch before writes the flags
+  // Afforest's second pass: rows flagged in `skip` (null: none) are left out and the first `sampled` arcs of
+  // the others were already united.  Plain loads: the launch before writes the flags
   const uint32_t* skip = nullptr;
   const uint64_t* __restrict__ off = nullptr;
   uint32_t sampled = 0;
   __device__ __forceinline__ bool skips(uint32_t u) const { return skip && ((skip[u >> 5] >> (u & 31u)) & 1u); }
   __device__ __forceinline__ double operator()(uint32_t u, uint64_t a) const {
-    if (skip && a < __ldg(off + u) + sampled) return 0.0;
+    if (sampled && a < __ldg(off + u) + sampled) return 0.0;
     uf_union(parent, nullptr, u, __ldg(col + a));
     return 0.0;
   }
@@ -79,13 +80,14 @@ __global__ void k_uf_first(uint64_t n, const uint64_t* __restrict__ off, const u
     }
   }
 }
+// The first k arcs of every row as unions; `all`: no first arc is a parent yet.
 __global__ void k_uf_sample(uint64_t n, const uint64_t* __restrict__ off, const uint32_t* __restrict__ col, uint32_t k,
-                            uint32_t* parent, const uint32_t* __restrict__ joined) {
+                            uint32_t* parent, const uint32_t* __restrict__ joined, bool all) {
   for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t a0 = off[u], a1 = off[u + 1];
     for (uint64_t a = a0; a < a1 && a < a0 + k; ++a) {
       const uint32_t v = __ldg(col + a);
-      if (a == a0 && (joined ? (__ldg(joined + (u >> 5)) >> (u & 31u)) & 1u : v < u)) continue;
+      if (a == a0 && !all && (joined ? (__ldg(joined + (u >> 5)) >> (u & 31u)) & 1u : v < u)) continue;
       uf_union(parent, nullptr, (uint32_t)u, v);
     }
   }
@@ -285,6 +287,27 @@ int gre_cc(gre_graph g, uint32_t* label, gre_stats* st) {
     counts = (unsigned long long*)p;
     best = (uint32_t*)(counts + 2);
   }
+  // Directed graphs: what is linked first decides how deep the trees get.  Us, one launch of all bins / the form chosen:
+  //  * few arcs, no hubs: short rows in the order of their ids, and what they have beyond four arcs after all of them.
+  //    10^6 vertices, trees with parents at most 10 ids back 476 / 141, relabelled 900 / 576, 50 back 314 / 139; grids and
+  //    paths the same; any id before 80 / 95, with ids at random 330 / 650; 2M
+  //    vertices of two random arcs 213 / 308;
+  //  * rows of about one length: four arcs a lane instead of the eight that suit a sum, since a lane's unions follow each
+  //    other, and bin by bin.  30000 vertices of 40 arcs 425 / 105, relabelled 401 / 137, 300000 of 8 216 / 111, 3000 of 40 115 /
+  //    66; 24000 arcs 48 / 60; 12M arcs 199 / 255;
+  //  * hubs that do not have the smallest ids: their CTAs link the loose vertices of half the graph and the root changes
+  //    under all of them, unless the short rows went first.  RMAT-16, 0.95M arcs 306 / 135, RMAT-18, 1.5M 545 / 230; about
+  //    equal at 0.25M (97 / 92) and 4M (290 / 292); RMAT-20 at 6M 434 / 604.  A relabelled graph's hubs are the roots
+  //    (RMAT-18: 128 / 275).
+  const bool directed = !g->symmetric(), hubs = g->max_outdeg >= kHubArcs, untuned = g->m < (1ull << 22);
+  const bool few = directed && !hubs && g->m < 4 * n && g->m < (1ull << 21);
+  const bool even = directed && !hubs && !few && g->m >= (1ull << 16) && untuned;
+  const bool loose = directed && hubs && !g->perm && g->m >= (1ull << 18) && untuned;
+  const DegreeBins* bins = &g->bins_out;
+  if (even && bins->sched.lane_arcs > RowSchedule().lane_arcs && !getenv("GRE_ROW_SCHEDULE")) {
+    if (!g->bins_cc.ready) GRE_CHECK(build_bins(g, g->bins_cc, g->off, g->col, RowSchedule()));
+    bins = &g->bins_cc;
+  }
   RunTimer timer(g);
   if (g->symmetric()) {
     // Afforest: unite the first arcs of every row, find the largest component from a sample,
@@ -294,21 +317,25 @@ int gre_cc(gre_graph g, uint32_t* label, gre_stats* st) {
     GRE_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), g->stream));
     uint32_t* joined = g->max_outdeg < kHubArcs ? skip : nullptr;  // the skip flags' words are free until the compression
     k_uf_first<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->off, g->col, parent, joined);
-    k_uf_sample<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->off, g->col, kSampled, parent, joined);
+    k_uf_sample<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->off, g->col, kSampled, parent, joined, false);
     k_uf_mode<<<1, kSample, 0, g->stream>>>(n, n > kSample ? n / kSample : 1, parent, best);
     k_uf_compress_skip<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent, g->off, best, kSampled, skip, counts);
     HookArcs rest{g->col, parent, skip, g->off, kSampled};
     GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, rest, NoFinish{}, partial, g->stream, kWave));
   } else {
     k_uf_init<<<grid_for(n, 256), 256, 0, g->stream>>>(n, parent);
-    const HookArcs arcs{g->col, parent};
-    // Hubs that do not have the smallest ids: their CTAs link the loose vertices of half the graph and the root
-    // changes under all of them, unless the short rows went first.  One launch / bin by bin: RMAT-16, 0.95M
-    // arcs 306 / 135 us, RMAT-18, 1.5M 545 / 230; about equal at 0.25M (97 / 92) and 4M (290 / 292); RMAT-20 at 6M 434 / 604,
-    // and a relabelled graph's hubs are the roots (RMAT-18: 128 / 275), as is a tree's parent (random tree: 81 / 520).
-    const bool apart = !g->perm && g->max_outdeg >= kHubArcs && g->m >= (1ull << 18) && g->m < (1ull << 22);
-    if (apart) GRE_CHECK(rows::visit_rows_apart(g->bins_out, g->off, arcs, NoFinish{}, partial, g->stream, kWave));
-    else GRE_CHECK(rows::reduce_rows(g->bins_out, g->off, arcs, NoFinish{}, partial, g->stream, kWave));
+    HookArcs arcs{g->col, parent};
+    if (few) {
+      constexpr uint32_t kFew = 4;
+      k_uf_sample<<<grid_for(n, 256), 256, 0, g->stream>>>(n, g->off, g->col, kFew, parent, nullptr, true);
+      arcs.off = g->off;
+      arcs.sampled = kFew;
+      if (g->max_outdeg > kFew) GRE_CHECK(rows::reduce_rows(*bins, g->off, arcs, NoFinish{}, partial, g->stream, kWave));
+    } else if (even || loose) {
+      GRE_CHECK(rows::visit_rows_apart(*bins, g->off, arcs, NoFinish{}, partial, g->stream, kWave));
+    } else {
+      GRE_CHECK(rows::reduce_rows(*bins, g->off, arcs, NoFinish{}, partial, g->stream, kWave));
+    }
   }
   if (g->perm) {
     GRE_CUDA(cudaMemcpyAsync(least, g->perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, g->stream));

@@ -296,6 +296,7 @@ void destroy_graph(gre_graph g) {
   free_bins(g->bins_in);
   free_bins(g->bins_out);
   free_bins(g->bins_sssp);
+  free_bins(g->bins_cc);
   free_chunk_table(g->bc_chunks);
   free_chunk_table(g->ppr_chunks);
   cudaFree(g->bc_fpool);
@@ -439,6 +440,7 @@ static void drop_derived(gre_graph g) {
   free_bins(g->bins_in);
   free_bins(g->bins_out);
   free_bins(g->bins_sssp);
+  free_bins(g->bins_cc);
   free_chunk_table(g->bc_chunks);
   free_chunk_table(g->ppr_chunks);
   cudaFree(g->bc_fpool);

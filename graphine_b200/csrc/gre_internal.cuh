@@ -162,6 +162,7 @@ struct gre_graph_s {
   // SSSP's binned passes, when the tuned schedule gives rows more than 8 arcs per lane or a warp
   // above 16384 arcs (sssp_bins): the pushes are latency-bound and want short chains per lane
   gre::DegreeBins bins_sssp;
+  gre::DegreeBins bins_cc;  // out-arc rows at the default schedule, for the components of directed graphs without hubs
   // Degree-ordered relabelling (GRE_GRAPH_REORDER / gre_graph_reorder): every internal array
   // uses internal ids; perm[i] is the caller's id of internal vertex i (the reference's
   // lvid2vid, DistributedGraph.hpp:57-59) and iperm its inverse.  Null when not relabelled.

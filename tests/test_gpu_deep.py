@@ -138,3 +138,41 @@ def test_components_of_directed_hubs(arcs):
         want = low
     for _ in range(5):
         np.testing.assert_array_equal(G.cc(g)[0], want.astype(np.uint32))
+
+
+def weak_labels(n, u, v):
+    want = np.arange(n)
+    while True:  # labels both ways, and along the labels
+        low = want.copy()
+        np.minimum.at(low, v, want[u])
+        np.minimum.at(low, u, low[v])
+        low = low[low]
+        if (low == want).all():
+            return want.astype(np.uint32)
+        want = low
+
+
+# arcs and vertices around the limits of the forms for rows of about one length: four arcs a vertex, 2^16, 2^21 and 2^22 arcs
+@pytest.mark.parametrize("n,arcs", [(3000, 11999), (3000, 12000), (5000, (1 << 16) - 1), (5000, 1 << 16), (16385, 1 << 16), (150000, 450000), (700000, (1 << 21) - 1), (700000, 1 << 21),
+                                    (200000, (1 << 22) - 1), (200000, 1 << 22)])
+def test_components_of_directed_graphs_without_hubs(n, arcs):
+    """Several parts that no arc joins, rows of about one length with some of none; the same graph before and after
+    it is relabelled, whose rows are binned anew."""
+    rng = np.random.default_rng(arcs)
+    part = np.sort(rng.integers(0, 7, n))
+    lo, hi = np.searchsorted(part, part), np.searchsorted(part, part, side="right")
+    u = rng.integers(0, n, arcs)
+    u -= (u % 11 == 0) & (u > 0)
+    v = lo[u] + (rng.random(arcs) * (hi - lo)[u]).astype(np.int64)
+    mix = rng.permutation(n)
+    u, v = mix[u], mix[v]
+    at = np.argsort(u, kind="stable")
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(u, minlength=n))
+    g = G.Graph.from_csr(n, off, v[at].astype(np.uint32))
+    want = weak_labels(n, u, v)
+    for _ in range(5):
+        np.testing.assert_array_equal(G.cc(g)[0], want)
+    g.reorder()
+    for _ in range(5):
+        np.testing.assert_array_equal(G.cc(g)[0], want)
