@@ -82,12 +82,21 @@ static int ws_array(gre_graph g, int slot, uint64_t count, T** p) {
 // reading of the topology is 4 bytes an arc: 0.95 ms a slice and superstep, 17 TB/s of gathered rows,
 // L2 and L1 at 64% (RMAT-20, 128 vectors, 20 supersteps: 61.2 -> 42.7 ms; slices of 32 columns: 46.2).
 //
-// The columns are independent: a slice runs all its supersteps before the next.  The values
-// themselves are written by the last superstep only, in place of the next contributions.
+// The columns are independent: a slice runs all its supersteps before the next, or, where a slice's warps leave
+// most of the GPU idle, several do side by side (3000 vertices of 16 arcs, 128 vectors, 20 supersteps: 788 us one after the
+// other, 196 side by side).  The values themselves are written by the last superstep only, in place of the
+// next contributions.
 // ---------------------------------------------------------------------------------------------
 constexpr uint64_t kPprChunk = 1024;
 constexpr int kPprBatch = 8;           // short rows a warp takes together
 constexpr uint32_t kPprShort = 32;     // arcs of a short row at most
+// Slices side by side: up to so many warps an SM together (counted with kPprBatch rows each), and two short rows a
+// warp, since there are more warps than work.  128 vectors, 20 supersteps, uniform rows of 16 arcs; 128-column rows of one slice /
+// slices of 64 in turn / side by side with 8, 4, 2, 1 rows a warp: 300 vertices 225 / 539 / 280, 231, 154, 149 us; 3000 252 / 788 /
+// 386, 282, 196, 198; 10000 411 / 802 / 443, 373, 346, 357; 40000 1233 / 1252 / 1066, 1011, 976, 1060.  Skewed rows, 20000 vertices
+// 7543 / 2015 / 1176, 1463, 1511, 1525.  At 100000 vertices two slices fill the GPU one by one: 2689 in turn, 2755 side by side.
+constexpr uint64_t kPprSideWarps = 128;
+constexpr int kPprSideBatch = 2;
 
 template <int C>
 struct PprVec;  // a lane's columns of a row: C/32 of them, side by side
@@ -130,9 +139,21 @@ struct PprStep {
   const uint32_t* __restrict__ rows;   // the bins' rows, short bins first
   uint32_t nrows, nshort;              // of which the first nshort have at most kPprShort arcs
   ChunkTable chunks;
-  uint32_t kk;
+  uint32_t kk;                         // columns of all slices side by side
+  uint64_t n;
   bool last;
   double tele, d;
+  // slice `i` of those side by side, each with buffers of its own
+  template <int C>
+  __device__ __forceinline__ PprStep slice(uint32_t i) const {
+    PprStep r = *this;
+    r.seeds += i * C;
+    r.kk = kk - i * C < C ? kk - i * C : C;
+    r.cur += i * n * C;
+    r.next += i * n * C;
+    r.partial += i * (chunks.nchunks + 1) * C;
+    return r;
+  }
 };
 
 // The place of the restart mass in a row: bit j of a lane's mask, its column j seeds vertex v.
@@ -191,12 +212,14 @@ __device__ __forceinline__ PprVec<C> ppr_sum(const PprStep& P, uint64_t a0, uint
 
 // One superstep but for the chunked rows' finish: first the chunks, then the rows from long to short
 // (the resident warps stride over them, each a share of every length).
-template <int C>
-__global__ void __launch_bounds__(256) k_ppr_step(const __grid_constant__ PprStep P) {
+// SIDE: slice blockIdx.y of several.
+template <int C, bool SIDE>
+__global__ void __launch_bounds__(256) k_ppr_step(const __grid_constant__ PprStep all) {
+  const PprStep P = SIDE ? all.slice<C>(blockIdx.y) : all;
   const uint32_t lane = lane_id();
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  constexpr int V = C / 32;
+  constexpr int V = C / 32, B = SIDE ? kPprSideBatch : kPprBatch;
   const uint32_t seed0 = V * lane < P.kk ? P.seeds[V * lane] : 0xffffffffu;
   const uint32_t seed1 = V == 2 && V * lane + 1 < P.kk ? P.seeds[V * lane + 1] : 0xffffffffu;
   uint64_t i = warp;
@@ -214,26 +237,26 @@ __global__ void __launch_bounds__(256) k_ppr_step(const __grid_constant__ PprSte
     ppr_finish<C>(P, v, od, ppr_sum<C>(P, a0, a1), seed0, seed1);
   }
   i -= nlong;
-  const uint64_t nbatches = ((uint64_t)P.nshort + kPprBatch - 1) / kPprBatch;
+  const uint64_t nbatches = ((uint64_t)P.nshort + B - 1) / B;
   for (; i < nbatches; i += nwarps) {
-    // lane j < kPprBatch: row j of the batch; then the columns of all of them
+    // lane j < B: row j of the batch; then the columns of all of them
     uint64_t a0 = 0;
     uint32_t v = 0, len = 0, od = 0;
-    const uint64_t at = i * kPprBatch + lane;
-    if (lane < kPprBatch && at < P.nshort) {
+    const uint64_t at = i * B + lane;
+    if (lane < B && at < P.nshort) {
       v = P.rows[P.nshort - 1 - at];
       a0 = P.roff[v];
       len = (uint32_t)(P.roff[v + 1] - a0);
       od = P.outdeg[v];
     }
-    uint32_t idx[kPprBatch];
+    uint32_t idx[B];
 #pragma unroll
-    for (int j = 0; j < kPprBatch; ++j) {
+    for (int j = 0; j < B; ++j) {
       const uint64_t b = __shfl_sync(0xffffffffu, a0, j);
       idx[j] = lane < __shfl_sync(0xffffffffu, len, j) ? __ldg(P.rcol + b + lane) : 0u;
     }
 #pragma unroll
-    for (int j = 0; j < kPprBatch; ++j) {
+    for (int j = 0; j < B; ++j) {
       const uint32_t n = __shfl_sync(0xffffffffu, len, j);
       PprVec<C> acc;
       ppr_gather(P.cur, idx[j], n, acc);
@@ -243,8 +266,9 @@ __global__ void __launch_bounds__(256) k_ppr_step(const __grid_constant__ PprSte
 }
 
 // Chunked rows: partial sums in chunk order, four loads in flight.
-template <int C>
-__global__ void __launch_bounds__(256) k_ppr_chunk_finish(const __grid_constant__ PprStep P) {
+template <int C, bool SIDE>
+__global__ void __launch_bounds__(256) k_ppr_chunk_finish(const __grid_constant__ PprStep all) {
+  const PprStep P = SIDE ? all.slice<C>(blockIdx.y) : all;
   const uint32_t lane = lane_id();
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -271,25 +295,26 @@ __global__ void __launch_bounds__(256) k_ppr_chunk_finish(const __grid_constant_
 
 // The restart mass in both buffers of contributions (zeroed before).
 template <int C>
-__global__ void k_ppr_seed(uint32_t kk, const uint32_t* __restrict__ seeds, const uint32_t* __restrict__ outdeg, double tele,
+__global__ void k_ppr_seed(uint64_t n, uint32_t kk, const uint32_t* __restrict__ seeds, const uint32_t* __restrict__ outdeg, double tele,
                            double* __restrict__ c0, double* __restrict__ c1) {
   for (uint32_t j = threadIdx.x; j < kk; j += blockDim.x) {
     const uint32_t s = seeds[j];
     const uint32_t od = outdeg[s];
     const double c = od ? tele / (double)od : 0.0;
-    c0[(uint64_t)s * C + j] = c;
-    c1[(uint64_t)s * C + j] = c;
+    const uint64_t at = (j / C * n + s) * C + j % C;
+    c0[at] = c;
+    c1[at] = c;
   }
 }
 
 // A seed whose row has no in-arcs (or all seeds, before any superstep) keeps its restart mass as its
 // value: no superstep wrote it.
 template <int C>
-__global__ void k_ppr_seed_values(uint32_t kk, const uint32_t* __restrict__ seeds, const uint64_t* __restrict__ roff, bool all,
+__global__ void k_ppr_seed_values(uint64_t n, uint32_t kk, const uint32_t* __restrict__ seeds, const uint64_t* __restrict__ roff, bool all,
                                   double tele, double* __restrict__ x) {
   for (uint32_t j = threadIdx.x; j < kk; j += blockDim.x) {
     const uint32_t s = seeds[j];
-    if (all || roff[s + 1] == roff[s]) x[(uint64_t)s * C + j] = tele;
+    if (all || roff[s + 1] == roff[s]) x[(j / C * n + s) * C + j % C] = tele;
   }
 }
 
@@ -300,6 +325,9 @@ __global__ void __launch_bounds__(256) k_ppr_out(uint64_t n, uint32_t kk, const 
                                                  const uint32_t* __restrict__ iperm, double* __restrict__ out) {
   __shared__ double tile[32][C + 1];
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+  x += blockIdx.y * n * C;  // slice blockIdx.y of those side by side
+  out += blockIdx.y * n * C;
+  kk = kk - blockIdx.y * C < C ? kk - blockIdx.y * C : C;
   for (uint64_t u0 = blockIdx.x * 32ull; u0 < n; u0 += gridDim.x * 32ull) {
     for (uint32_t r = w; r < 32; r += 8) {
       if (u0 + r >= n) break;
@@ -314,30 +342,36 @@ __global__ void __launch_bounds__(256) k_ppr_out(uint64_t n, uint32_t kk, const 
   }
 }
 
-// One slice: kk <= C seeds (device), the results to out (kk rows of n in the caller's order).
-template <int C>
-static int ppr_slice(gre_graph g, PprStep P, uint32_t iters, double* c0, double* c1, double* out) {
-  const uint64_t n = g->n;
+// Chunks, long rows and batches of short ones.
+static uint64_t ppr_warps(const PprStep& P, uint32_t batch) {
+  return P.chunks.nchunks + (P.nrows - P.nshort) + (P.nshort + batch - 1) / batch;
+}
+
+// One slice, or several side by side (SIDE): P.kk <= slices * C seeds (device), the results to out (kk rows of n in the
+// caller's order).
+template <int C, bool SIDE>
+static int ppr_slices(gre_graph g, PprStep P, uint32_t slices, uint32_t iters, double* c0, double* c1, double* out) {
+  const uint64_t n = g->n, warps = ppr_warps(P, SIDE ? kPprSideBatch : kPprBatch);
   static int per_sm = 0;
   if (!per_sm) {
     int b = 0;
-    GRE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_ppr_step<C>, 256, 0));
+    GRE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_ppr_step<C, SIDE>, 256, 0));
     per_sm = b > 0 ? b : 1;
   }
-  GRE_CUDA(cudaMemsetAsync(c0, 0, sizeof(double) * n * C, g->stream));
-  GRE_CUDA(cudaMemsetAsync(c1, 0, sizeof(double) * n * C, g->stream));
-  k_ppr_seed<C><<<1, C, 0, g->stream>>>(P.kk, P.seeds, g->outdeg, P.tele, c0, c1);
-  const uint64_t warps = P.chunks.nchunks + (P.nrows - P.nshort) + (P.nshort + kPprBatch - 1) / kPprBatch;
+  auto side = [&](int blocks) { return dim3(blocks, slices); };
+  GRE_CUDA(cudaMemsetAsync(c0, 0, sizeof(double) * n * C * slices, g->stream));
+  GRE_CUDA(cudaMemsetAsync(c1, 0, sizeof(double) * n * C * slices, g->stream));
+  k_ppr_seed<C><<<1, C, 0, g->stream>>>(n, P.kk, P.seeds, g->outdeg, P.tele, c0, c1);
   for (uint32_t it = 0; it < iters; ++it) {
     P.cur = c0;
     P.next = c1;
     P.last = it + 1 == iters;
-    k_ppr_step<C><<<grid_for(warps * 32, 256, per_sm), 256, 0, g->stream>>>(P);
-    if (P.chunks.nrows) k_ppr_chunk_finish<C><<<grid_for(P.chunks.nrows * 32, 256, 8), 256, 0, g->stream>>>(P);
+    k_ppr_step<C, SIDE><<<side(grid_for(warps * 32, 256, per_sm)), 256, 0, g->stream>>>(P);
+    if (P.chunks.nrows) k_ppr_chunk_finish<C, SIDE><<<side(grid_for(P.chunks.nrows * 32, 256, 8)), 256, 0, g->stream>>>(P);
     std::swap(c0, c1);
   }
-  k_ppr_seed_values<C><<<1, C, 0, g->stream>>>(P.kk, P.seeds, g->roff, iters == 0, P.tele, c0);
-  k_ppr_out<C><<<grid_for(n * 8, 256, 16), 256, 0, g->stream>>>(n, P.kk, c0, g->iperm, out);
+  k_ppr_seed_values<C><<<1, C, 0, g->stream>>>(n, P.kk, P.seeds, g->roff, iters == 0, P.tele, c0);
+  k_ppr_out<C><<<side(grid_for(n * 8, 256, 16)), 256, 0, g->stream>>>(n, P.kk, c0, g->iperm, out);
   GRE_LAUNCH_CHECK();
   return GRE_SUCCESS;
 }
@@ -639,17 +673,11 @@ int gre_ppr(gre_graph g, const uint32_t* seeds, uint32_t k, double d, uint32_t i
     double *c0, *c1, *partial;
     uint32_t* dseeds;
     PprStep P{};
-    const int cols = k > 32 ? 64 : 32;
-    GRE_CHECK(ws_array(g, WS_A, n * cols, &c0));
-    GRE_CHECK(ws_array(g, WS_B, n * cols, &c1));
-    GRE_CHECK(ws_array(g, WS_D, (g->ppr_chunks.nchunks + 1) * cols, &partial));
-    GRE_CHECK(ws_array(g, WS_E, k, &dseeds));
-    GRE_CUDA(cudaMemcpyAsync(dseeds, hs.data(), sizeof(uint32_t) * k, cudaMemcpyHostToDevice, g->stream));
     const DegreeBins& B = g->bins_in;
+    P.n = n;
     P.roff = g->roff;
     P.rcol = g->rcol;
     P.outdeg = g->outdeg;
-    P.partial = partial;
     P.rows = B.rows;
     P.chunks = g->ppr_chunks;
     P.tele = tele;
@@ -658,13 +686,30 @@ int gre_ppr(gre_graph g, const uint32_t* seeds, uint32_t k, double d, uint32_t i
       P.nrows += (uint32_t)B.count[b];
       if (b < 5 && ((uint64_t)B.sched.lane_arcs << b) <= kPprShort) P.nshort += (uint32_t)B.count[b];
     }
+    const uint64_t fit = kPprSideWarps * (uint64_t)num_sms() / std::max<uint64_t>(1, ppr_warps(P, kPprBatch));
+    const uint32_t slices = k <= 64 ? 1 : (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(fit, (k + 63) / 64));
+    const uint64_t cols = k > 32 ? 64ull * slices : 32;
+    GRE_CHECK(ws_array(g, WS_A, n * cols, &c0));
+    GRE_CHECK(ws_array(g, WS_B, n * cols, &c1));
+    GRE_CHECK(ws_array(g, WS_D, (g->ppr_chunks.nchunks + 1) * cols, &partial));
+    GRE_CHECK(ws_array(g, WS_E, k, &dseeds));
+    GRE_CUDA(cudaMemcpyAsync(dseeds, hs.data(), sizeof(uint32_t) * k, cudaMemcpyHostToDevice, g->stream));
+    P.partial = partial;
     for (uint32_t j0 = 0; j0 < k;) {
       // 64 columns a slice; a rest of at most 32 in a slice of 32
-      const uint32_t width = k - j0 > 32 ? 64 : 32;
-      P.kk = std::min<uint32_t>(width, k - j0);
+      const uint32_t left = k - j0;
       P.seeds = dseeds + j0;
       double* o = dfinal + (uint64_t)j0 * n;
-      GRE_CHECK(width == 64 ? ppr_slice<64>(g, P, iters, c0, c1, o) : ppr_slice<32>(g, P, iters, c0, c1, o));
+      if (slices > 1 && left > 64) {
+        P.kk = std::min<uint32_t>(64 * slices, left);
+        GRE_CHECK((ppr_slices<64, true>(g, P, (P.kk + 63) / 64, iters, c0, c1, o)));
+      } else if (left > 32) {
+        P.kk = std::min<uint32_t>(64, left);
+        GRE_CHECK((ppr_slices<64, false>(g, P, 1, iters, c0, c1, o)));
+      } else {
+        P.kk = left;
+        GRE_CHECK((ppr_slices<32, false>(g, P, 1, iters, c0, c1, o)));
+      }
       j0 += P.kk;
     }
     if (st) {

@@ -97,3 +97,23 @@ def test_row_schedules_below_the_tuned_sizes(monkeypatch, scale, edgefactor, wan
     assert G.Graph.rmat(scale, edgefactor, 5, True).row_schedule()[:2] == want
     monkeypatch.setenv("GRE_TUNE", "0")
     assert G.Graph.rmat(scale, edgefactor, 5, True).row_schedule() == (4, 4096, 65536, 0)
+
+
+@pytest.mark.parametrize("n", [50, 3000, 45000])
+@pytest.mark.parametrize("k", [65, 128, 193, 232, 300])
+def test_personalised_slices_side_by_side(n, k):
+    """Slices of 64 vectors run side by side on a small graph, as many as fit, then the rest: every vector has the
+    bits that it has in a call of its slice alone."""
+    rng = np.random.default_rng(n)
+    u, v = rng.integers(0, n, 9 * n), (rng.integers(0, n, 9 * n) * rng.random(9 * n) ** 4).astype(np.int64)
+    at = np.argsort(u, kind="stable")
+    off = np.zeros(n + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(u, minlength=n))
+    g = G.Graph.from_csr(n, off, v[at].astype(np.uint32))
+    if n == 3000:
+        g.reorder()
+    seeds = rng.integers(0, n, k).astype(np.uint32)
+    seeds[-1] = seeds[0]
+    out = G.ppr(g, seeds, 0.85, 3)[0].reshape(k, n)
+    for j in range(0, k, 64):
+        np.testing.assert_array_equal(out[j : j + 64].reshape(-1), G.ppr(g, seeds[j : j + 64], 0.85, 3)[0])
