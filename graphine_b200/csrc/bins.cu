@@ -15,9 +15,10 @@
 // process under a key made from the degree distribution (arcs per power-of-two degree bucket,
 // log2 n, log2 m), so graphs of the same shape - the batches of a run, replicas - tune once.
 //
-// Graphs with fewer than 2^22 arcs are not measured: their supersteps are
-// too short to time apart from launch overhead.  From 2^16 arcs on they use a fixed schedule of short chains, below
-// that the default one.  GRE_TUNE=0 in the environment turns all of this off: every graph uses the default schedule.  GRE_ROW_SCHEDULE=lane_arcs,cta_min,hub_chunk,seg_window
+// Graphs with fewer than 2^22 arcs are not measured: their supersteps are too short to time apart from
+// launch overhead.  From 2^16 arcs on they use a fixed schedule of short chains, below that the default one.
+// GRE_TUNE=0 in the environment turns all of this off: every graph uses the default schedule.
+// GRE_ROW_SCHEDULE=lane_arcs,cta_min,hub_chunk,seg_window
 // imposes a schedule (tests use it to reach every kernel on small graphs).
 #include <cub/cub.cuh>
 

@@ -289,7 +289,10 @@ void launch_count_add(long long k);
 // Launch with programmatic stream serialization: once all blocks of the kernel before it in the stream have
 // called launch_next (or ended), this one's may start.  They call wait_previous, all of them, ahead of
 // anything that depends on the stream's earlier work: it returns when that kernel has ended and, as that
-// one waited in its turn, all before it.
+// one waited in its turn, all before it.  What those wrote is visible to plain loads from then on.  __ldg, and
+// __restrict__ to const, which the compiler may turn into it, promise data that stays as it is while the kernel
+// lives: they are for arrays that were complete before the launch ahead of this one began (the graph's own), not for
+// what that launch writes.
 template <class... P, class... A>
 int launch_early(cudaStream_t s, unsigned int grid, unsigned int block, void (*kernel)(P...), A... args) {
   cudaLaunchAttribute early{};

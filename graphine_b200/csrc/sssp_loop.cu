@@ -20,8 +20,9 @@
 // (a heavy pass or a rise the next bucket's too, a rise the next far count) and clears the one after.
 //
 // Measured against the host-driven loop: RMAT-22, four sources, 16.9 -> 8.3 ms; RMAT-26 17.3 -> 12.2 ms
-// a source; 60000 vertices, directed, 2810 -> 446 us (630 at the same bucket width); a grid of 1000 x 1000 690 -> 73 ms.  A pass over a handful of vertices is 4 us (half of
-// it the barrier), one over a few thousand 8-18 us (five dependent round trips).
+// a source; 60000 vertices, directed, 2810 -> 446 us (630 at the same bucket width); a grid of 1000 x 1000
+// 690 -> 73 ms.  A pass over a handful of vertices is 4 us (half of it the barrier), one over a few thousand 8-18 us
+// (five dependent round trips).
 #include <algorithm>
 
 #include "sssp_loop.cuh"
